@@ -1127,6 +1127,94 @@ int engforce_finish(mdff_ctx* ctx) {
     return MDFF_OK;
 }
 
+// Plan and buffers of the FP64 path's tensor-core reciprocal space for the
+// vectors with ak != 0; off (the CUDA-core kernels run) when kz > 31, where the
+// seven digit levels of one tile no longer fit tensor memory, or when a tile's
+// tables do not fit shared memory.
+int plan_t7(mdff_ctx* ctx, const std::vector<double>& ak, size_t* part, size_t* fpart) {
+    const KGrid& kg = ctx->kg;
+    T7K& t = ctx->rs.t7;
+    const int n = ctx->n;
+    t.kx = kg.kmax[0]; t.ky = kg.kmax[1]; t.kz = kg.kmax[2]; t.nzl = kg.nzl;
+    t.N = ((2 * (t.kz + 1) + 15) / 16) * 16;
+    t.KZ = ((2 * (t.kz + 1) + 31) / 32) * 32;
+    if (t.N > tc7::NLEV_MAX || t.KZ > tc7::FK_MAX) return MDFF_OK;
+    const int nyn = 2 * t.ky + 1;
+    std::vector<int> cols, pairs, tr;
+    std::vector<char> has(kg.ncol, 0);
+    for (int col = 0; col < kg.ncol; ++col) {
+        for (int m = 0; m < kg.nzl; ++m) has[col] |= ak[(size_t)col * kg.nzl + m] != 0.0;
+        if (has[col]) cols.push_back(col);
+    }
+    for (int nx = 0; nx <= t.kx; ++nx)
+        for (int ny = 0; ny <= t.ky; ++ny)
+            if (has[nx * nyn + t.ky + ny] || has[nx * nyn + t.ky - ny]) { pairs.push_back(nx); pairs.push_back(ny); }
+    if (cols.empty()) return MDFF_OK;
+    t.ncol = (int)cols.size();
+    t.npair = (int)(pairs.size() / 2);
+    t.ntile = (t.npair + tc7::TP - 1) / tc7::TP;
+    t.pstride = t.ntile * tc7::TP;
+    for (int b = 0; b < t.ntile; ++b) {
+        int x0 = t.kx, x1 = 0, y0 = t.ky, y1 = 0;
+        for (int q = b * tc7::TP; q < std::min(t.npair, (b + 1) * tc7::TP); ++q) {
+            x0 = std::min(x0, pairs[2 * q]); x1 = std::max(x1, pairs[2 * q]);
+            y0 = std::min(y0, pairs[2 * q + 1]); y1 = std::max(y1, pairs[2 * q + 1]);
+        }
+        tr.insert(tr.end(), {x0, x1 - x0 + 1, y0, y1 - y0 + 1});
+        t.entmax = std::max(t.entmax, x1 - x0 + 1 + y1 - y0 + 1);
+    }
+    const size_t smax = 227 * 1024 - 2048;   // static shared memory aside
+    t.nin = tc7::Layout::depth(t.N, t.entmax, smax);
+    if (t.nin < 2) return MDFF_OK;
+    const tc7::Layout lay(t.N, t.entmax, t.nin);
+    t.smem = lay.smem_bytes();
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->p.device);
+    // atoms split so that the grid covers the SMs about once
+    t.nblk = (n + tc7::SA - 1) / tc7::SA;
+    t.npad = t.nblk * tc7::SA;
+    const int S = std::max(1, sms / t.ntile);
+    t.bps = std::min(std::max(1, (t.nblk + S - 1) / S), tc7::MAX_BLOCKS_PER_CTA);
+    t.nsplit = (t.nblk + t.bps - 1) / t.bps;
+    t.ntile_f = (n + 127) / 128;
+    t.ncb2 = (t.ncol + tc7::Cfg<2>::CB - 1) / tc7::Cfg<2>::CB;
+    t.ncb3 = (t.ncol + tc7::Cfg<3>::CB - 1) / tc7::Cfg<3>::CB;
+    t.grid2 = (int)std::min<long>((long)t.ntile_f * t.ncb2, sms);
+    t.grid3 = (int)std::min<long>((long)t.ntile_f * t.ncb3, sms);
+    const tc7::FLayout f2(t.KZ, tc7::Cfg<2>::CB), f3(t.KZ, tc7::Cfg<3>::CB);
+    t.smem_f2 = f2.smem_bytes();
+    t.smem_f3 = f3.smem_bytes();
+    auto slots = [&](int ncb, int grid) {   // most CTAs that share a tile
+        const long U = (long)t.ntile_f * ncb;
+        int m = 1;
+        for (int b = 0; b < t.ntile_f; ++b)
+            m = std::max(m, tc7::cta_of((long)b * ncb + ncb - 1, U, grid) - tc7::cta_of((long)b * ncb, U, grid) + 1);
+        return (size_t)m;
+    };
+    *part = (size_t)t.nsplit * 4 * t.N * t.pstride;
+    *fpart = (size_t)n * tc7::NQ * std::max(3 * slots(t.ncb2, t.grid2), 9 * slots(t.ncb3, t.grid3));
+    const int ent = t.kx + t.ky + 2;
+    TRY(dalloc(ctx, &t.pairs, pairs.size()));
+    TRY(dalloc(ctx, &t.trange, tr.size()));
+    TRY(dalloc(ctx, &t.cols, cols.size()));
+    TRY(dalloc(ctx, &t.xy, (size_t)t.nblk * ent * tc7::AP));
+    TRY(dalloc(ctx, &t.bimg, (size_t)t.nblk * lay.b_bytes()));
+    TRY(dalloc(ctx, &t.aimg, (size_t)t.ntile_f * f2.a_bytes));
+    TRY(dalloc(ctx, &t.prm, (size_t)t.npad));
+    TRY(dalloc(ctx, &t.bmax, (size_t)t.nblk));
+    TRY(dalloc(ctx, &t.fimg, std::max((size_t)t.ncb2 * f2.stage_bytes, (size_t)t.ncb3 * f3.stage_bytes)));
+    CK(cudaMemcpyAsync(t.pairs, pairs.data(), sizeof(int) * pairs.size(), cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaMemcpyAsync(t.trange, tr.data(), sizeof(int) * tr.size(), cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaMemcpyAsync(t.cols, cols.data(), sizeof(int) * cols.size(), cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaStreamSynchronize(ctx->st));   // the host vectors go out of scope
+    // one limit for every context of the process, whatever its sizes
+    CK(cudaFuncSetAttribute(tc7::k_sfac_t7, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax));
+    CK(cudaFuncSetAttribute(tc7::k_kfield_t7<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax));
+    CK(cudaFuncSetAttribute(tc7::k_kfield_t7<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax));
+    t.on = 1;
+    return MDFF_OK;
+}
+
 int set_units(mdff_ctx* ctx) {
     if (ctx->p.lreduced) ctx->u = {1.0, 1.0, 1.0, 1.0};
     else ctx->u = {0.00624150964712042, 8.61734229648141e-05, 98.2269514139276, 14.3996441494161};
@@ -3339,13 +3427,18 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
             CK(cudaMemcpyAsync(kg.mask, mk.data(), kg.nrect, cudaMemcpyHostToDevice, ctx->st));
             CK(cudaStreamSynchronize(ctx->st));
         }
-        size_t fp = 0;
-        size_t pc = std::max(tc_part, rec_scratch_doubles(n, kg, &fp, p.precision == MDFF_PREC_MIXED));
+        size_t fp = 0, pc = 0;
+        ctx->rs.t7 = T7K();
+        if (p.precision == MDFF_PREC_FP64) TRY(plan_t7(ctx, ak, &pc, &fp));
+        if (!ctx->rs.t7.on) {
+            pc = std::max(tc_part, rec_scratch_doubles(n, kg, &fp, p.precision == MDFF_PREC_MIXED));
+        }
         fp = std::max(fp, (size_t)2 * tcf::NQ * 9 * n);   // tensor-core field pass: NQ column parts x 2 column slots
         TRY(dalloc(ctx, &ctx->rs.part, pc));
         TRY(dalloc(ctx, &ctx->rs.fpart, fp));
         TRY(dalloc(ctx, &ctx->rs.aks, 2 * (size_t)kg.nrect));
         TRY(dalloc(ctx, &ctx->rs.aks_acc, 2 * (size_t)kg.nrect));
+        CK(cudaMemsetAsync(ctx->rs.aks, 0, sizeof(double) * 2 * kg.nrect, ctx->st));   // vectors no pass writes
         TRY(dalloc(ctx, &ctx->rs.fixed, 3 * (size_t)n));
         TRY(dalloc(ctx, &ctx->rs.tab, (size_t)n * 16));
         TRY(dalloc(ctx, &ctx->rs.aks2, (size_t)kg.ncol * (((kg.nzl + 15) / 16) * 16)));
@@ -3353,6 +3446,7 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
         ctx->rs.fpart_cap = fp;
     }
     int parts = std::max(16 * 1024, 12 * (int)(((size_t)n * 32 + 255) / 256));
+    if (p.lcoulomb) parts = std::max(parts, 7 * ctx->rs.t7.ntile * (ctx->rs.t7.kz + 1));
     TRY(dalloc(ctx, &ctx->part.buf, parts));
     ctx->part.capacity = parts;
     // neighbour lists

@@ -289,6 +289,28 @@ struct TcK {
     size_t smem_f2 = 0, smem_f3 = 0;
 };
 
+// FP64-grade tensor-core reciprocal space of the FP64 path (ewald_tc7.cuh).
+struct T7K {
+    int on = 0;
+    int kx = 0, ky = 0, kz = 0, nzl = 0;
+    int npair = 0, ncol = 0;      // (nx, +-ny) pairs of the structure factor, columns of the field
+    int N = 0, KZ = 0;            // structure-factor GEMM N, field K bytes per atom row
+    int ntile = 0, pstride = 0;   // 32-pair tiles, padded pair count
+    int nblk = 0, npad = 0, bps = 0, nsplit = 0;   // 16-atom blocks, blocks per split, splits
+    int nin = 0, entmax = 0;      // input pipeline depth, most table entries of a tile
+    int ntile_f = 0, ncb2 = 0, ncb3 = 0, grid2 = 0, grid3 = 0;   // 128-atom tiles, column blocks and CTAs (E / E + grad)
+    size_t smem = 0, smem_f2 = 0, smem_f3 = 0;
+    int* pairs = nullptr;         // [npair][2]: nx, ny >= 0
+    int* trange = nullptr;        // [ntile][4]: first X entry, count, first Y entry, count
+    int* cols = nullptr;          // [ncol] rectangle column index
+    double2* xy = nullptr;        // per position update: X/Y tables
+    uint8_t* bimg = nullptr;      //   structure-factor B images
+    uint8_t* aimg = nullptr;      //   field A images
+    double4* prm = nullptr;       // per evaluation: sources and their largest magnitudes per block
+    double4* bmax = nullptr;
+    uint8_t* fimg = nullptr;      //   field B images
+};
+
 struct RecScratch {
     double* part = nullptr;    // structure-factor partials
     size_t part_cap = 0;       // doubles
@@ -304,6 +326,7 @@ struct RecScratch {
     long want_epoch = 0;        // current position epoch (set by the engine)
     LowK low;
     TcK tc;
+    T7K t7;
 };
 struct RecFlags {
     int with_q, with_mu;

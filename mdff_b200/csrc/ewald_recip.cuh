@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "ewald_tc.cuh"
 #include "ewald_tc4.cuh"
+#include "ewald_tc7.cuh"
 
 namespace mdff {
 
@@ -968,6 +969,16 @@ size_t rec_scratch_doubles(int n, const KGrid& kg, size_t* fpart, int mixed) {
 // images); returns the number of kernels launched.
 int ensure_phase_tables(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz, RecScratch& rs) {
     if (rs.tab_epoch == rs.want_epoch) return 0;
+    if (rs.t7.on) {   // FP64 path
+        const T7K& t = rs.t7;
+        const long nxy = (long)t.nblk * (t.kx + t.ky + 2) * tc7::AP, nb = (long)t.nblk * (tc7::SA / 2) * (t.N / 2);
+        const long na = (long)t.ntile_f * 128 * (t.KZ / 16);
+        tc7::k_t7_xy<<<(unsigned)((nxy + 255) / 256), 256, 0, st>>>(n, t.nblk, sx, sy, t.kx, t.ky, t.xy);
+        tc7::k_t7_bimage<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(n, t.nblk, sz, t.kz, t.N, t.bimg);
+        tc7::k_t7f_aimage<<<(unsigned)((na + 255) / 256), 256, 0, st>>>(n, t.ntile_f, sz, t.kz, t.KZ, t.aimg);
+        rs.tab_epoch = rs.want_epoch;
+        return 3;
+    }
     const LowK& lk = rs.low;
     k_phase_table<<<(n + 127) / 128, 128, 0, st>>>(n, sx, sy, sz, rs.fixed, rs.tab,
                                                    lk.ncol > 0 && !lk.tc ? lk.tab : nullptr);
@@ -1032,6 +1043,39 @@ int launch_low_field(cudaStream_t st, int n, CellP c, bool grad, RecScratch& rs,
         k_kfield64_low<0><<<dim3((n + KF_THREADS - 1) / KF_THREADS, LK_SPLIT), KF_THREADS, 0, st>>>(
             n, rs.fixed, lk.tab, c, lk.col, lk.ncol, lk.nzmax, lk.aks, lk.fpart);
     return 1;
+}
+
+// The FP64 path on the tensor cores: structure factor to A_k S(k) (+ energy and
+// stress partials), and the field pass; each returns the kernels launched.
+int launch_t7_sfac(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz, const double* q,
+                   const double* mu, CellP c, const KGrid& kg, RecFlags fl, RecScratch& rs, Partials& part,
+                   DevScalars* d) {
+    const T7K& t = rs.t7;
+    int nk = ensure_phase_tables(st, n, sx, sy, sz, rs);
+    tc7::k_t7_params<<<(t.npad + 255) / 256, 256, 0, st>>>(n, t.npad, sx, sy, sz, q, mu, c, fl.with_q, fl.with_mu, t.prm,
+                                                           t.bmax);
+    tc7::k_sfac_t7<<<dim3(t.ntile, t.nsplit), tc7::THREADS, t.smem, st>>>(
+        t.nblk, t.bps, t.nin, t.bimg, t.xy, t.prm, t.bmax, t.pairs, t.trange, t.npair, t.kx, t.ky, t.kz, t.N, t.entmax,
+        rs.part, t.pstride, &d->tc_err);
+    const dim3 g(t.ntile, t.kz + 1);
+    tc7::k_t7_sreduce<<<g, 256, 0, st>>>(t.nsplit, t.N, t.npair, t.pstride, t.pairs, t.ky, t.kz, t.nzl, rs.part, kg.Ak,
+                                         kg.kcoe, c, rs.aks, kg.nrect, fl.energy, part.buf);
+    if (fl.energy) launch_reduce_partials(st, part.buf, t.ntile * (t.kz + 1), 7, d->rec, 0);
+    return nk + 3 + (fl.energy ? 1 : 0);
+}
+
+template <int NMOM>
+int launch_t7_field(cudaStream_t st, int n, CellP c, const KGrid& kg, RecScratch& rs, double scale, const double* q,
+                    const double* mu, double* ef, double* efg, double* fo, DevScalars* d) {
+    const T7K& t = rs.t7;
+    constexpr int NV = NMOM == 3 ? 9 : 3;
+    const int ncb = NMOM == 3 ? t.ncb3 : t.ncb2, grid = NMOM == 3 ? t.grid3 : t.grid2;
+    tc7::k_t7f_bimage<NMOM><<<ncb, tc7::NB * (t.KZ / 16), 0, st>>>(t.ncol, t.cols, t.kx, t.ky, t.kz, t.nzl, t.KZ, rs.aks,
+                                                                  kg.nrect, c, t.fimg);
+    tc7::k_kfield_t7<NMOM><<<grid, tc7::FTHREADS, NMOM == 3 ? t.smem_f3 : t.smem_f2, st>>>(
+        n, t.ntile_f, t.ncol, ncb, t.aimg, t.xy, t.fimg, t.kx, t.ky, t.KZ, c, rs.fpart, &d->tc_err);
+    tc7::k_t7_freduce<NV><<<(n + 31) / 32, 256, 0, st>>>(n, t.ntile_f, ncb, grid, rs.fpart, scale, q, mu, ef, efg, fo);
+    return 3;
 }
 
 #define CUDA_COPY_ACC(st, dst, src, bytes) cudaMemcpyAsync((dst), (src), (bytes), cudaMemcpyDeviceToDevice, (st))
@@ -1110,6 +1154,8 @@ void launch_ewald_rec(cudaStream_t st, int n, const double* sx, const double* sy
         }
         k_sfac_reduce<<<rb, 256, 0, st>>>(Pr, TM, nchunk32, kg.ncol, kg.nzl, kx, ky, kz, pre, pim, kg.Ak_hi, kg.kcoe, c,
                                           rs.aks, kg.nrect, fl.energy, part.buf);
+    } else if (rs.t7.on) {
+        nk = launch_t7_sfac(st, n, sx, sy, sz, q, mu, c, kg, fl, rs, part, d);
     } else {
         const bool sph = kg.nfitems > 0;
         dim3 g1(sph ? (kg.nfitems + SF_THREADS - 1) / SF_THREADS : L.nchunk * L.ncolblk, L.P);
@@ -1123,7 +1169,7 @@ void launch_ewald_rec(cudaStream_t st, int n, const double* sx, const double* sy
         k_sfac_reduce<<<rb, 256, 0, st>>>(L.P, L.CH, L.nchunk, kg.ncol, kg.nzl, kx, ky, kz, pre, pim, kg.Ak, kg.kcoe,
                                           c, rs.aks, kg.nrect, fl.energy, part.buf);
     }
-    if (fl.energy && !fl.reuse) launch_reduce_partials(st, part.buf, rb, 7, d->rec, 0);
+    if (fl.energy && !fl.reuse && !rs.t7.on) launch_reduce_partials(st, part.buf, rb, 7, d->rec, 0);
     if (low && !fl.reuse) {
         LowK& lk = rs.low;
         int Pl = lk.P;
@@ -1162,6 +1208,16 @@ void launch_ewald_rec(cudaStream_t st, int n, const double* sx, const double* sy
     nk = 1;
     dim3 g2((n + KF_THREADS - 1) / KF_THREADS, L.nsplit);
     const bool grad = fl.grad || (fl.forces && fl.with_mu);
+    const double scale = 2.0 * 4.0 * PI / c.omega;
+    if (!mixed && rs.t7.on) {
+        const double *fq = fl.with_q ? q : nullptr, *fm = fl.with_mu ? mu : nullptr;
+        double *oe = fl.field ? ef : nullptr, *of = fl.forces ? fo : nullptr;
+        nk = ensure_phase_tables(st, n, sx, sy, sz, rs);   // (a reused structure factor)
+        nk += grad ? launch_t7_field<3>(st, n, c, kg, rs, scale, fq, fm, oe, efg, of, d)
+                   : launch_t7_field<2>(st, n, c, kg, rs, scale, fq, fm, oe, efg, of, d);
+        prof->end(nk);
+        return;
+    }
     int nsplit_f = L.nsplit;
     if (mixed && rs.tc.on) {
         // field pass on the tensor cores: NQ column parts per atom
@@ -1215,7 +1271,6 @@ void launch_ewald_rec(cudaStream_t st, int n, const double* sx, const double* sy
                                                       sph ? kg.fzr : nullptr);
         nk++;
     }
-    const double scale = 2.0 * 4.0 * PI / c.omega;
     k_kfield_reduce<<<(n + 255) / 256, 256, 0, st>>>(n, nsplit_f, grad ? 1 : 0, rs.fpart, scale, fl.with_q ? q : nullptr,
                                                     fl.with_mu ? mu : nullptr, fl.field ? ef : nullptr, efg,
                                                     fl.forces ? fo : nullptr, low ? rs.low.fpart : nullptr,

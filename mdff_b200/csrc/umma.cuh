@@ -41,6 +41,7 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
 __host__ __device__ constexpr uint32_t idesc_s8(int M, int N) {
     return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
+constexpr uint32_t IDESC_A_U8 = 1u << 7;   // xor: A is unsigned
 // byte offset of element (r, k) of a K-major, no-swizzle 8-bit tile with R
 // rows (core matrices of 8 rows x 16 elements)
 __host__ __device__ __forceinline__ uint32_t kmajor_off_i8(int R, int r, int k) {
