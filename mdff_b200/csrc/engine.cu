@@ -4265,6 +4265,83 @@ void rmc_normalise(const RmcConst& k, const std::vector<int>& h, double* grr) {
     }
 }
 
+// Whether a neighbour list of radius rl has every atom of the cell at most once
+// within reach: else the pairs are all pairs.
+bool rmc_all_pairs(const mdff_ctx* ctx, double rl) {
+    return 2.0 * rl >= std::min(ctx->W[0], std::min(ctx->W[1], ctx->W[2]));
+}
+
+int rmc_cap(const mdff_ctx* ctx, double rl) {
+    return (int)std::min<double>(ctx->n - 1, 1.3 * 4.0 / 3.0 * PI * rl * rl * rl * ctx->n / ctx->cell.omega + 64);
+}
+
+// Full neighbour rows within rl of the fractional coordinates s by the cell
+// grid of the Verlet lists (its buffers are scratch between builds); nbr grows,
+// with cap, until the rows fit.
+int rmc_lists(mdff_ctx* ctx, const double* s, double rl, int& cap, int** nbr, int* cnt) {
+    const int n = ctx->n;
+    CellGrid& g = ctx->grid;
+    for (int d = 0; d < 3; ++d)
+        g.nc[d] = std::max(1, std::min((int)std::floor(ctx->W[d] / (rl * (1.0 + 1e-12))), 256));
+    g.ncell = g.nc[0] * g.nc[1] * g.nc[2];
+    if (g.ncell > g.ncell_alloc) {
+        TRY(dalloc(ctx, &g.cell_count, g.ncell));
+        TRY(dalloc(ctx, &g.cell_start, g.ncell + 1));
+        TRY(dalloc(ctx, &g.cell_cursor, g.ncell));
+        g.ncell_alloc = g.ncell;
+    }
+    launch_bin(ctx->st, n, s, s + n, s + 2 * (size_t)n, g);
+    for (int attempt = 0;; ++attempt) {
+        if (!*nbr) CK(cudaMallocAsync((void**)nbr, sizeof(int) * (size_t)n * cap, ctx->st));
+        CK(cudaMemsetAsync(ctx->d_overflow, 0, sizeof(int), ctx->st));
+        NList L;
+        L.nbr = *nbr;
+        L.cnt = cnt;
+        L.cap = cap;
+        launch_nlist(ctx->st, n, s, s + n, s + 2 * (size_t)n, ctx->cell, g, rl * rl, L, rl * rl, nullptr, ctx->d_overflow);
+        TRY(check_launch(ctx, "rmc list"));
+        int ovf = 0;
+        CK(cudaMemcpyAsync(&ovf, ctx->d_overflow, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
+        CK(cudaStreamSynchronize(ctx->st));
+        if (ovf <= cap) return MDFF_OK;
+        if (attempt > 3) return fail(ctx, MDFF_E_LISTOVF, "mdff_rmc: neighbour list capacity");
+        CK(cudaFreeAsync(*nbr, ctx->st));
+        *nbr = nullptr;
+        cap = std::min(n - 1, (int)(ovf * 1.2) + 32);
+    }
+}
+
+// Pair counts of the fractional coordinates s into hist (zeroed by the
+// caller), from neighbour rows that reach the cutoff (nbr), or over all pairs.
+// A grid of four blocks per SM keeps the shared counts' flushes few; 32 440 ions,
+// cut 10 A: 6.2 ms for one thread per atom over all pairs, 0.1 ms from the rows.
+int rmc_counts(mdff_ctx* ctx, const double* s, const RmcConst& k, const int* nbr, const int* cnt, int cap, int* hist) {
+    const int n = ctx->n;
+    const size_t smem = sizeof(int) * (size_t)k.ntype * k.ntype * k.nbins;
+    const int in_smem = smem <= 48 * 1024 ? 1 : 0;
+    const int blocks = std::min((n + 7) / 8, 4 * 148);
+    if (nbr)
+        k_gr_rows<true><<<blocks, 256, in_smem ? smem : 0, ctx->st>>>(n, s, ctx->type, ctx->cell, k.bin, nbr, cnt, cap,
+                                                                     in_smem, hist);
+    else
+        k_gr_rows<false><<<blocks, 256, in_smem ? smem : 0, ctx->st>>>(n, s, ctx->type, ctx->cell, k.bin, nullptr,
+                                                                      nullptr, 0, in_smem, hist);
+    return check_launch(ctx, "gr");
+}
+
+// The same with rows built for it where the cell has room for a list.
+int rmc_counts_of(mdff_ctx* ctx, const double* s, const RmcConst& k, double cut, int* hist) {
+    if (rmc_all_pairs(ctx, cut) || ctx->n < 2) return rmc_counts(ctx, s, k, nullptr, nullptr, 0, hist);
+    int cap = std::max(1, rmc_cap(ctx, cut));
+    int *nbr = nullptr, *cnt = nullptr;
+    CK(cudaMallocAsync((void**)&cnt, sizeof(int) * (size_t)ctx->n, ctx->st));
+    int rc = rmc_lists(ctx, s, cut, cap, &nbr, cnt);
+    if (rc == MDFF_OK) rc = rmc_counts(ctx, s, k, nbr, cnt, cap, hist);
+    if (nbr) cudaFreeAsync(nbr, ctx->st);
+    cudaFreeAsync(cnt, ctx->st);
+    return rc;
+}
+
 }  // namespace
 
 extern "C" {
@@ -4283,8 +4360,7 @@ int mdff_gr(mdff_ctx* ctx, double cut, double res, double* grr, int* nbins) {
     CK(cudaMallocAsync((void**)&h, sizeof(int) * (size_t)k.nrow * k.nbins, ctx->st));
     CK(cudaMemsetAsync(h, 0, sizeof(int) * (size_t)k.nrow * k.nbins, ctx->st));
     TRY(rmc_frac(ctx, s));
-    k_gr_full<<<nb(n), 256, 0, ctx->st>>>(n, s, ctx->type, ctx->cell, k.bin, h);
-    TRY(check_launch(ctx, "gr"));
+    TRY(rmc_counts_of(ctx, s, k, cut, h));
     std::vector<int> hh((size_t)k.nrow * k.nbins);
     CK(cudaMemcpyAsync(hh.data(), h, sizeof(int) * hh.size(), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaFreeAsync(s, ctx->st));
@@ -4331,49 +4407,41 @@ int mdff_rmc(mdff_ctx* ctx, const mdff_rmc_params* rp, const double* grr_exp, co
     else k_rmc_uniforms<<<(unsigned)((nu + 255) / 256), 256, 0, ctx->st>>>(nu, seed, uni);
     CK(cudaMemsetAsync(h, 0, sizeof(int) * ncount, ctx->st));
     TRY(rmc_frac(ctx, s));
-    k_gr_full<<<nb(n), 256, 0, ctx->st>>>(n, s, ctx->type, ctx->cell, k->bin, h);
-    TRY(check_launch(ctx, "rmc start"));
-    const int smem = (int)(ncount * sizeof(int));
-    CK(cudaFuncSetAttribute(k_rmc_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // the counts and their change in shared memory, or the change alone
+    const size_t nterm = (size_t)(k->npairs + 1) * k->nbins;
+    const int in_smem = 2 * nterm * sizeof(int) <= 200 * 1024 ? 1 : 0;
+    const int smem = (int)((in_smem ? 2 : 1) * nterm * sizeof(int));
+    CK(cudaFuncSetAttribute(k_rmc_chain<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CK(cudaFuncSetAttribute(k_rmc_chain<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     // neighbour lists of the chain: every atom within cut + skin; while no
     // atom has moved more than (skin - 3 max_displacement) / 2 from the
     // list's positions, a pair outside the list stays beyond cut at both ends
     // of any trial move.  When cut + skin reaches half the cell, the list
     // holds every atom and never expires.
     const double skin = 1.0;
-    const double wmin = std::min(ctx->W[0], std::min(ctx->W[1], ctx->W[2]));
-    const bool all_pairs = 2.0 * (rp->cut_rmc + skin) >= wmin;
-    const double rl = all_pairs ? 1e300 : rp->cut_rmc + skin;
+    const bool all_pairs = rmc_all_pairs(ctx, rp->cut_rmc + skin);
     const double dlim = all_pairs ? 1e300 : 0.5 * (skin - 3.0 * rp->max_displacement);
-    int cap = all_pairs ? std::max(1, n - 1)
-                        : (int)std::min<double>(n - 1, 1.3 * 4.0 / 3.0 * PI * rl * rl * rl * n / ctx->cell.omega + 64);
-    int *nbr = nullptr, *ncnt = nullptr, *ovf = nullptr;
+    int cap = all_pairs ? std::max(1, n - 1) : std::max(1, rmc_cap(ctx, rp->cut_rmc + skin));
+    int *nbr = nullptr, *ncnt = nullptr;
     double* sb = nullptr;
     CK(cudaMallocAsync((void**)&ncnt, sizeof(int) * (size_t)n, ctx->st));
-    CK(cudaMallocAsync((void**)&ovf, sizeof(int), ctx->st));
     CK(cudaMallocAsync((void**)&sb, sizeof(double) * 3 * (size_t)n, ctx->st));
     CK(cudaMemsetAsync(out, 0, sizeof(RmcOut), ctx->st));
-    int nbuild = 0;
     for (int launch = 0;; ++launch) {
-        for (int attempt = 0;; ++attempt) {   // build, growing the capacity if needed
-            if (!nbr) CK(cudaMallocAsync((void**)&nbr, sizeof(int) * (size_t)n * cap, ctx->st));
-            CK(cudaMemsetAsync(ovf, 0, sizeof(int), ctx->st));
-            k_rmc_list<<<nb(n), 256, 0, ctx->st>>>(n, s, ctx->cell, rl * rl, cap, nbr, ncnt, ovf);
-            TRY(check_launch(ctx, "rmc list"));
-            int ho_ovf = 0;
-            CK(cudaMemcpyAsync(&ho_ovf, ovf, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
-            CK(cudaStreamSynchronize(ctx->st));
-            if (ho_ovf <= cap) break;
-            if (attempt > 3) return fail(ctx, MDFF_E_LISTOVF, "mdff_rmc: neighbour list capacity");
-            CK(cudaFreeAsync(nbr, ctx->st));
-            nbr = nullptr;
-            cap = std::min(n - 1, (int)(ho_ovf * 1.2) + 32);
+        if (all_pairs) {
+            CK(cudaMallocAsync((void**)&nbr, sizeof(int) * (size_t)n * cap, ctx->st));
+            k_rmc_all<<<n, 256, 0, ctx->st>>>(n, cap, nbr, ncnt);
+        } else {
+            TRY(rmc_lists(ctx, s, rp->cut_rmc + skin, cap, &nbr, ncnt));
         }
-        ++nbuild;
+        if (launch == 0) TRY(rmc_counts(ctx, s, *k, all_pairs ? nullptr : nbr, ncnt, cap, h));
         CK(cudaMemcpyAsync(sb, s, sizeof(double) * 3 * (size_t)n, cudaMemcpyDeviceToDevice, ctx->st));
-        k_rmc_chain<<<1, RMC_THREADS, smem, ctx->st>>>(s, ctx->type, ctx->cell, kd, h, gexp, uni, nu,
-                                                       rp->acceptance_max, rp->max_trials, nbr, ncnt, cap, sb, dlim,
-                                                       out);
+#define CHAIN(F) k_rmc_chain<F><<<1, RMC_THREADS, smem, ctx->st>>>(s, ctx->type, ctx->cell, kd, h, gexp, uni, nu,         \
+                                                                   rp->acceptance_max, rp->max_trials, nbr, ncnt, cap, \
+                                                                   sb, dlim, in_smem, out)
+        if (all_pairs) CHAIN(false);
+        else CHAIN(true);
+#undef CHAIN
         TRY(check_launch(ctx, "rmc chain"));
         RmcOut st;
         CK(cudaMemcpyAsync(&st, out, sizeof st, cudaMemcpyDeviceToHost, ctx->st));
@@ -4384,8 +4452,7 @@ int mdff_rmc(mdff_ctx* ctx, const mdff_rmc_params* rp, const double* grr_exp, co
         CK(cudaMemcpyAsync(out, &st, sizeof st, cudaMemcpyHostToDevice, ctx->st));
         CK(cudaStreamSynchronize(ctx->st));
     }
-    (void)nbuild;
-    for (void* q : {(void*)nbr, (void*)ncnt, (void*)ovf, (void*)sb}) CK(cudaFreeAsync(q, ctx->st));
+    for (void* q : {(void*)nbr, (void*)ncnt, (void*)sb}) CK(cudaFreeAsync(q, ctx->st));
     k_rmc_dirkar<<<nb(n), 256, 0, ctx->st>>>(n, s, ctx->cell, ctx->x, ctx->y, ctx->z);
     RmcOut ho;
     std::vector<int> hh(ncount);
@@ -4590,7 +4657,7 @@ int mdff_rmc_efg(mdff_ctx* ctx, const mdff_rmc_params* rp, const mdff_rmc_efg_pa
     CK(cudaMemsetAsync(hd, 0, sizeof(int) * ngr, ctx->st));
     TRY(rmc_frac(ctx, s));
     k_rmc_dirkar<<<nb(n), 256, 0, ctx->st>>>(n, s, ctx->cell, ctx->x, ctx->y, ctx->z);
-    k_gr_full<<<nb(n), 256, 0, ctx->st>>>(n, s, ctx->type, ctx->cell, k->bin, hd);
+    TRY(rmc_counts_of(ctx, s, *k, rp->cut_rmc, hd));
     double *vl = nullptr, *vmean = nullptr, *vpart = nullptr, *vpsum = nullptr;
     int *vrank = nullptr, *verr = nullptr;
     const int vwb = (n * 32 + 255) / 256;   // blocks of the per-atom chi kernel (a warp per atom)
