@@ -134,6 +134,9 @@ struct mdff_ctx {
     // mixed path: per-step pair table of the dipole-dipole operator (A1, B2 per
     // Coulomb list entry), written by the charge pass of each force evaluation
     float2* ddtab = nullptr;
+    double2* ddtab64 = nullptr;          // FP64 path
+    double* ddrec64 = nullptr;           // [8n]
+    bool ddtab_off = false;              // FP64 path: no memory for the table, the operator is evaluated per pair
     int* ddnbr = nullptr;
     int* ddcnt = nullptr;
     uint4* ddrec = nullptr;              // [2n] gather records of the operator
@@ -526,9 +529,10 @@ DirFlags dir_flags(const mdff_ctx* ctx) {
 
 // Field of the induced dipoles: real space (dipole-dipole, undamped) +
 // reciprocal space + self term; src/field.f90:3354-3357.
-// Real-space part of the dipole field operator: FP64 (MODE 1 of
+// Real-space part of the dipole field operator, from the pair table of the
+// step's charge pass where there is one: FP64 (k_ewald_ddtab64, else MODE 1 of
 // k_ewald_dir) or, on the mixed path, FP32 arithmetic from the fixed-point
-// coordinates (k_ewald_dd32).
+// coordinates (k_ewald_ddtab, else k_ewald_dd32).
 void dd_field_real(mdff_ctx* ctx, const double* m, double* out) {
     const int n = ctx->n;
     ctx->prof.begin(PK_DIR);
@@ -544,11 +548,18 @@ void dd_field_real(mdff_ctx* ctx, const double* m, double* out) {
         ctx->prof.end(k);
         return;
     }
+    const NList& L = coul_list(ctx);
+    if (ctx->ddtab64 && ctx->ddtab_epoch == ctx->rs.want_epoch && ctx->ddtab_lcap == L.cap) {
+        launch_ewald_ddtab64(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, m, ctx->cell, ctx->ddnbr, ctx->ddcnt, L.cap,
+                             ctx->ddtab64, ctx->ddrec64, out, ctx->g_dd);
+        ctx->prof.end(2);
+        return;
+    }
     DirFlags f = dir_flags(ctx);
     f.dd = 1;
     f.field = 1;
-    launch_ewald_dir(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, ctx->type, nullptr, m, ctx->cell, coul_list(ctx), ctx->pc,
-                     f, out, nullptr, nullptr, ctx->part, ctx->dsc, ctx->g_dir);
+    launch_ewald_dir(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, ctx->type, nullptr, m, ctx->cell, L, ctx->pc, f, out,
+                     nullptr, nullptr, ctx->part, ctx->dsc, ctx->g_dir);
     ctx->prof.end(1);
 }
 
@@ -568,26 +579,41 @@ int induced_field(mdff_ctx* ctx, const double* m, double* out, bool self = true)
     return check_launch(ctx, "induced_field");
 }
 
-// On the mixed path, let this charge pass also write the dipole-dipole pair
-// table for the solver's operator (allocated for the current list capacity).
+// Let this charge pass also write the dipole-dipole pair table for the solver's
+// operator (allocated for the current list capacity), in FP32 on the mixed
+// path and in FP64 on the FP64 path.  Where the FP64 table does not fit in
+// device memory the operator goes on without it.
 int arm_ddtab(mdff_ctx* ctx, DirFlags& f) {
-    if (ctx->p.precision != MDFF_PREC_MIXED) return MDFF_OK;
+    const bool mixed = ctx->p.precision == MDFF_PREC_MIXED;
+    if (!mixed && ctx->ddtab_off) return MDFF_OK;
     const NList& L = coul_list(ctx);
     const size_t need = (size_t)ctx->n * L.cap;
     if (need > ctx->ddtab_cap) {
         if (ctx->ddtab) CK(cudaFree(ctx->ddtab));
+        if (ctx->ddtab64) CK(cudaFree(ctx->ddtab64));
         if (ctx->ddnbr) CK(cudaFree(ctx->ddnbr));
         ctx->ddtab = nullptr;
+        ctx->ddtab64 = nullptr;
         ctx->ddnbr = nullptr;
         ctx->ddtab_cap = 0;
-        cudaError_t e = cudaMalloc(&ctx->ddtab, sizeof(float2) * need);
+        cudaError_t e = mixed ? cudaMalloc(&ctx->ddtab, sizeof(float2) * need)
+                              : cudaMalloc(&ctx->ddtab64, sizeof(double2) * need);
         if (e == cudaSuccess) e = cudaMalloc(&ctx->ddnbr, sizeof(int) * need);
+        if (e != cudaSuccess && !mixed) {
+            cudaGetLastError();
+            cudaFree(ctx->ddtab64);
+            ctx->ddtab64 = nullptr;
+            ctx->ddtab_off = true;
+            return MDFF_OK;
+        }
         if (e != cudaSuccess) return fail(ctx, MDFF_E_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
         ctx->ddtab_cap = need;
     }
     if (!ctx->ddcnt) TRY(dalloc(ctx, &ctx->ddcnt, ctx->n));
-    if (!ctx->ddrec) TRY(dalloc(ctx, &ctx->ddrec, 2 * (size_t)ctx->n));
+    if (mixed && !ctx->ddrec) TRY(dalloc(ctx, &ctx->ddrec, 2 * (size_t)ctx->n));
+    if (!mixed && !ctx->ddrec64) TRY(dalloc(ctx, &ctx->ddrec64, 8 * (size_t)ctx->n));
     f.ddtab = ctx->ddtab;
+    f.ddtab64 = ctx->ddtab64;
     f.ddnbr = ctx->ddnbr;
     f.ddcnt = ctx->ddcnt;
     ctx->ddtab_epoch = ctx->rs.want_epoch;
@@ -974,6 +1000,21 @@ int autotune(mdff_ctx* ctx) {
             launch_ewald_rec(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, ctx->q, ctx->mu, ctx->cell, ctx->kg, fe, ctx->rs,
                              ctx->ef, nullptr, nullptr, ctx->part, ctx->dsc, &ctx->prof);
         }, muls, 3);
+    }
+    if (ctx->p.precision == MDFF_PREC_FP64 && ctx->npol > 0) {
+        DirFlags fs = dir_flags(ctx);
+        fs.qq = 1;
+        fs.damp = 1;
+        fs.field = 1;
+        TRY(arm_ddtab(ctx, fs));
+        if (fs.ddtab64) {
+            launch_ewald_dir(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, ctx->type, ctx->q, ctx->mu, ctx->cell, coul_list(ctx),
+                             ctx->pc, fs, ctx->Estat, nullptr, nullptr, ctx->part, ctx->dsc, ctx->g_dir);
+            ctx->g_dd = pick([&](int g) {
+                launch_ewald_ddtab64(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, ctx->mu, ctx->cell, ctx->ddnbr, ctx->ddcnt,
+                                     coul_list(ctx).cap, ctx->ddtab64, ctx->ddrec64, ctx->Eind, g);
+            }, gs, 3);
+        }
     }
     ctx->prof.on = prof_on;
     ctx->prof.launches = launches;
@@ -1555,6 +1596,9 @@ bool graph_eligible(const mdff_ctx* ctx) {
     if (p.lcoulomb && p.precision == MDFF_PREC_MIXED &&
         (!ctx->ddcnt || !ctx->ddrec || (size_t)ctx->n * coul_list(ctx).cap > ctx->ddtab_cap))
         return false;
+    if (p.lcoulomb && p.precision == MDFF_PREC_FP64 && ctx->npol > 0 && !ctx->ddtab_off &&
+        (!ctx->ddcnt || !ctx->ddrec64 || (size_t)ctx->n * coul_list(ctx).cap > ctx->ddtab_cap))
+        return false;
     return true;
 }
 
@@ -1563,7 +1607,7 @@ StepKey step_key(const mdff_ctx* ctx) {
     std::memset(&k, 0, sizeof k);
     k.ptr[0] = ctx->lv.nbr; k.ptr[1] = ctx->lv.cnt;
     k.ptr[2] = ctx->lc.nbr; k.ptr[3] = ctx->lc.cnt;
-    k.ptr[4] = ctx->ddtab;  k.ptr[5] = ctx->ddnbr;
+    k.ptr[4] = ctx->ddtab ? (const void*)ctx->ddtab : ctx->ddtab64;  k.ptr[5] = ctx->ddnbr;
     k.cap[0] = ctx->lv.cap; k.cap[1] = ctx->lc.cap; k.cap[2] = (int)std::min<size_t>(ctx->ddtab_cap, 0x7fffffff);
     k.cell = ctx->cell;
     k.g_dir = ctx->g_dir; k.g_dd = ctx->g_dd; k.p_mul = ctx->rs.p_mul; k.s_mul = ctx->rs.s_mul;
@@ -3011,6 +3055,7 @@ void mdff_destroy(mdff_ctx* ctx) {
         ctx->prof.release();
         free_all(ctx);
         if (ctx->ddtab) cudaFree(ctx->ddtab);
+        if (ctx->ddtab64) cudaFree(ctx->ddtab64);
         if (ctx->ddnbr) cudaFree(ctx->ddnbr);
         drop_graphs(ctx);
         cudaStreamDestroy(ctx->st);
@@ -3034,6 +3079,11 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
     ctx->lv = NList();
     ctx->lc = NList();
     ctx->grid = CellGrid();
+    ctx->ddcnt = nullptr;   // freed with the rest; the pair table itself is kept
+    ctx->ddrec = nullptr;
+    ctx->ddrec64 = nullptr;
+    ctx->ddtab_epoch = -1;
+    ctx->ddtab_off = false;
     ctx->have_system = ctx->have_list = ctx->forces_valid = ctx->md_started = false;
     const mdff_params& p = ctx->p;
     const int n = natm;

@@ -206,6 +206,7 @@ struct DirFlags {
     // entries inside the cutoff (ddnbr, ddcnt) with the undamped
     // dipole-dipole radial factors (A1, B2) of each entry in FP32 (ddtab)
     float2* ddtab;
+    double2* ddtab64;   // the same in FP64 (one of the two)
     int* ddnbr;
     int* ddcnt;
 };
@@ -350,6 +351,12 @@ void launch_ewald_dd32(cudaStream_t st, int n, const uint32_t* fx, const double*
 // rec is per-atom scratch of 8 words (fixed-point coordinates, FP32 dipole).
 void launch_ewald_ddtab(cudaStream_t st, int n, const uint32_t* fx, const double* mu, CellP c, const int* nbr,
                         const int* cnt, int cap, const float2* tab, uint4* rec, double* ef, int g = 16);
+
+// The FP64 path's form: FP64 pair table, records of 8 doubles (fractional
+// coordinates, dipole).
+void launch_ewald_ddtab64(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz,
+                          const double* mu, CellP c, const int* nbr, const int* cnt, int cap, const double2* tab,
+                          double* rec, double* ef, int g = 16);
 
 // Solver vector kernels.
 

@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256, MODE == 2 ? 3 : 2) k_ewald_dir(int n, con
             double rx = 0.0, ry = 0.0, rz = 0.0, d2 = 0.0;
             if (valid) d2 = pairvec_exact(c, si1, si2, si3, sx[j], sy[j], sz[j], rx, ry, rz);
             const bool in = valid && d2 <= fl.cutsq;
-            if (MODE != 1 && fl.ddtab) {
+            if (MODE != 1 && fl.ddnbr) {
                 const unsigned bal = (__ballot_sync(gmask, in) & gmask) >> g0;
                 pos = cbase + __popc(bal & ((1u << sub) - 1u));
                 if (in) fl.ddnbr[(size_t)i * cap + pos] = j;
@@ -79,6 +79,7 @@ __global__ void __launch_bounds__(256, MODE == 2 ? 3 : 2) k_ewald_dir(int n, con
             const double A1 = F1 * dm3;
             const double B2 = 3.0 * F2 * dm5;
             if (MODE != 1 && fl.ddtab) fl.ddtab[(size_t)i * cap + pos] = make_float2((float)A1, (float)B2);
+            if (MODE != 1 && fl.ddtab64) fl.ddtab64[(size_t)i * cap + pos] = make_double2(A1, B2);
             if (MODE == 2) {
                 double gi = 0.0;
                 if (fl.damp) {
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(256, MODE == 2 ? 3 : 2) k_ewald_dir(int n, con
                 S[3] += rx * fi1 + ry * fi0; S[4] += rx * fi2 + rz * fi0; S[5] += ry * fi2 + rz * fi1;
             }
         }
-        if (MODE != 1 && fl.ddtab && sub == 0) fl.ddcnt[i] = cbase;
+        if (MODE != 1 && fl.ddnbr && sub == 0) fl.ddcnt[i] = cbase;
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) E[k] = group_sum<G>(E[k]);
@@ -357,6 +358,89 @@ void launch_ewald_ddtab(cudaStream_t st, int n, const uint32_t* fx, const double
     k_dd_records<<<(n + 255) / 256, 256, 0, st>>>(n, fx, mu, rec);
     const int blocks = (int)(((size_t)n * g + 255) / 256);
 #define DDT(G) k_ewald_ddtab<G><<<blocks, 256, 0, st>>>(n, rec, c, nbr, cnt, cap, tab, ef)
+    if (g == 8) DDT(8);
+    else if (g == 32) DDT(32);
+    else DDT(16);
+#undef DDT
+}
+
+// FP64 path: the operator from an FP64 pair table, so that a solver iteration
+// evaluates no square root, exponential or erfc: 20 bytes of table and ~31 FP64
+// instructions per ordered pair, the image from the fractional coordinates
+// (d - rint(d); where the two images of a pair are equally far, T2 is the same
+// for both).  A1 and B2 are the charge pass's own doubles, so the operator is
+// MODE 1's to rounding and symmetric to the last bit.  Bound: the gathers of
+// 64-byte records through L2 (930 MB at 32 440 ions, rc 10 A) beside the table's
+// 290 MB from HBM: 117 us per application against 279 of MODE 1, 14 against 33
+// at 3 000 ions; the charge pass takes 64 us longer once a step.
+__global__ void k_dd_records64(int n, const double* __restrict__ sx, const double* __restrict__ sy,
+                               const double* __restrict__ sz, const double* __restrict__ mu, double4* __restrict__ rec) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    rec[2 * i] = make_double4(sx[i], sy[i], sz[i], 0.0);
+    rec[2 * i + 1] = make_double4(mu[i], mu[n + i], mu[2 * n + i], 0.0);
+}
+
+// four doubles in one 256-bit load
+__device__ __forceinline__ void ld_rec64(const double4* __restrict__ p, double& a, double& b, double& c) {
+    asm("{\n\t.reg .f64 d;\n\tld.global.nc.v4.f64 {%0, %1, %2, d}, [%3];\n\t}" : "=d"(a), "=d"(b), "=d"(c) : "l"(p));
+}
+
+template <int G>
+__global__ void __launch_bounds__(256) k_ewald_ddtab64(int n, const double4* __restrict__ rec, CellP c,
+                                                       const int* __restrict__ nbr, const int* __restrict__ cnt,
+                                                       int cap, const double2* __restrict__ tab,
+                                                       double* __restrict__ ef) {
+    const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const int sub = threadIdx.x & (G - 1);
+    const bool active = gid < n;
+    const int i = active ? gid : 0;
+    constexpr double M = 6755399441055744.0;   // 1.5 2^52: (d + M) - M = rint(d)
+    double E0 = 0.0, E1 = 0.0, E2 = 0.0;
+    if (active) {
+        double s1, s2, s3;
+        ld_rec64(rec + 2 * (size_t)i, s1, s2, s3);
+        const int m = cnt[i];
+        const int* row = nbr + (size_t)i * cap;
+        const double2* trow = tab + (size_t)i * cap;
+        auto term = [&](int j, double2 t) {
+            double p1, p2, p3, m0, m1, m2;
+            ld_rec64(rec + 2 * (size_t)j, p1, p2, p3);
+            ld_rec64(rec + 2 * (size_t)j + 1, m0, m1, m2);
+            double d0 = s1 - p1, d1 = s2 - p2, d2 = s3 - p3;
+            d0 -= (d0 + M) - M;
+            d1 -= (d1 + M) - M;
+            d2 -= (d2 + M) - M;
+            const double rx = fma(d2, c.A[2], fma(d1, c.A[1], d0 * c.A[0]));
+            const double ry = fma(d2, c.A[5], fma(d1, c.A[4], d0 * c.A[3]));
+            const double rz = fma(d2, c.A[8], fma(d1, c.A[7], d0 * c.A[6]));
+            const double rb = fma(rz, m2, fma(ry, m1, rx * m0)) * t.y;
+            E0 = fma(rx, rb, fma(-m0, t.x, E0));
+            E1 = fma(ry, rb, fma(-m1, t.x, E1));
+            E2 = fma(rz, rb, fma(-m2, t.x, E2));
+        };
+        int k = sub;
+        for (; k + G < m; k += 2 * G) {
+            const int ja = row[k], jb = row[k + G];
+            const double2 ta = __ldcs(trow + k), tb = __ldcs(trow + k + G);
+            term(ja, ta);
+            term(jb, tb);
+        }
+        if (k < m) term(row[k], __ldcs(trow + k));
+    }
+    E0 = group_sum<G>(E0);
+    E1 = group_sum<G>(E1);
+    E2 = group_sum<G>(E2);
+    if (active && sub == 0) { ef[i] = E0; ef[n + i] = E1; ef[2 * n + i] = E2; }
+}
+
+void launch_ewald_ddtab64(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz,
+                          const double* mu, CellP c, const int* nbr, const int* cnt, int cap, const double2* tab,
+                          double* rec, double* ef, int g) {
+    double4* r = reinterpret_cast<double4*>(rec);
+    k_dd_records64<<<(n + 255) / 256, 256, 0, st>>>(n, sx, sy, sz, mu, r);
+    const int blocks = (int)(((size_t)n * g + 255) / 256);
+#define DDT(G) k_ewald_ddtab64<G><<<blocks, 256, 0, st>>>(n, r, c, nbr, cnt, cap, tab, ef)
     if (g == 8) DDT(8);
     else if (g == 32) DDT(32);
     else DDT(16);
