@@ -674,7 +674,7 @@ int fused_initial_field(mdff_ctx* ctx) {
     launch_aks_accumulate(ctx->st, ctx->kg, ctx->rs, ctx->dsc, 1);
     k_axpy<<<nb(n3), 256, 0, ctx->st>>>(n3, 2.0 * selfa2(ctx), ctx->dip0, ctx->Estat);
     k_axpy<<<nb(n3), 256, 0, ctx->st>>>(n3, 2.0 * selfa2(ctx), ctx->mu_ind, ctx->Eind);
-    ctx->prof.end(ctx->rs.low.ncol > 0 ? 4 : 3);
+    ctx->prof.end(3);
     return check_launch(ctx, "fused_initial_field");
 }
 
@@ -819,7 +819,7 @@ int solve_dipoles(mdff_ctx* ctx) {
             // the same step on the structure factors (before rz advances)
             if (reuse) launch_aks_accumulate(ctx->st, ctx->kg, ctx->rs, d, 0);
             k_cg_direction2<<<nb(n3), 256, 0, ctx->st>>>(n3, ctx->cg_z, ctx->cg_d, d, ctx->part.buf, vb);
-            ctx->prof.end(3 + (reuse ? (ctx->rs.low.ncol > 0 ? 2 : 1) : 0));
+            ctx->prof.end(3 + (reuse ? 1 : 0));
             return check_launch(ctx, "pcg iteration");
         };
         if (ctx->capturing) {
@@ -1168,6 +1168,16 @@ int engforce_finish(mdff_ctx* ctx) {
     return MDFF_OK;
 }
 
+// The most CTAs that share a 128-atom tile when ntile x ncb units are cut into
+// `grid` ranges.
+size_t tile_slots(int ntile, int ncb, int grid) {
+    const long U = (long)ntile * ncb;
+    int m = 1;
+    for (int b = 0; b < ntile; ++b)
+        m = std::max(m, umma::range_of((long)b * ncb + ncb - 1, U, grid) - umma::range_of((long)b * ncb, U, grid) + 1);
+    return (size_t)m;
+}
+
 // Plan and buffers of the FP64 path's tensor-core reciprocal space for the
 // vectors with ak != 0; off (the CUDA-core kernels run) when kz > 31, where the
 // seven digit levels of one tile no longer fit tensor memory, or when a tile's
@@ -1225,15 +1235,8 @@ int plan_t7(mdff_ctx* ctx, const std::vector<double>& ak, size_t* part, size_t* 
     const tc7::FLayout f2(t.KZ, tc7::Cfg<2>::CB), f3(t.KZ, tc7::Cfg<3>::CB);
     t.smem_f2 = f2.smem_bytes();
     t.smem_f3 = f3.smem_bytes();
-    auto slots = [&](int ncb, int grid) {   // most CTAs that share a tile
-        const long U = (long)t.ntile_f * ncb;
-        int m = 1;
-        for (int b = 0; b < t.ntile_f; ++b)
-            m = std::max(m, tc7::cta_of((long)b * ncb + ncb - 1, U, grid) - tc7::cta_of((long)b * ncb, U, grid) + 1);
-        return (size_t)m;
-    };
     *part = (size_t)t.nsplit * 4 * t.N * t.pstride;
-    *fpart = (size_t)n * tc7::NQ * std::max(3 * slots(t.ncb2, t.grid2), 9 * slots(t.ncb3, t.grid3));
+    *fpart = (size_t)n * tc7::NQ * std::max(3 * tile_slots(t.ntile_f, t.ncb2, t.grid2), 9 * tile_slots(t.ntile_f, t.ncb3, t.grid3));
     const int ent = t.kx + t.ky + 2;
     TRY(dalloc(ctx, &t.pairs, pairs.size()));
     TRY(dalloc(ctx, &t.trange, tr.size()));
@@ -3483,7 +3486,8 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
         if (!ctx->rs.t7.on) {
             pc = std::max(tc_part, rec_scratch_doubles(n, kg, &fp, p.precision == MDFF_PREC_MIXED));
         }
-        fp = std::max(fp, (size_t)2 * tcf::NQ * 9 * n);   // tensor-core field pass: NQ column parts x 2 column slots
+        if (p.precision == MDFF_PREC_MIXED)   // tensor-core field pass: NQ column parts x 2 column slots
+            fp = std::max(fp, (size_t)2 * tcf::NQ * 9 * n);
         TRY(dalloc(ctx, &ctx->rs.part, pc));
         TRY(dalloc(ctx, &ctx->rs.fpart, fp));
         TRY(dalloc(ctx, &ctx->rs.aks, 2 * (size_t)kg.nrect));
@@ -3496,7 +3500,8 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
         ctx->rs.fpart_cap = fp;
     }
     int parts = std::max(16 * 1024, 12 * (int)(((size_t)n * 32 + 255) / 256));
-    if (p.lcoulomb) parts = std::max(parts, 7 * ctx->rs.t7.ntile * (ctx->rs.t7.kz + 1));
+    if (p.lcoulomb)   // energy and stress sums of the structure factor's reductions
+        parts = std::max(parts, 7 * std::max(ctx->rs.t7.ntile * (ctx->rs.t7.kz + 1), (ctx->kg.nrect + 31) / 32));
     TRY(dalloc(ctx, &ctx->part.buf, parts));
     ctx->part.capacity = parts;
     // neighbour lists

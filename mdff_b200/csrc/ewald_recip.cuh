@@ -116,28 +116,50 @@ __global__ void __launch_bounds__(SF_THREADS) k_sfac(int n, int natom_chunk, con
     }
 }
 
-// Sum the atom-chunk partials in order; A_k S(k); energy and stress per k
-// (src/field.f90:2742-2745, 2803-2815).
-__global__ void k_sfac_reduce(int P, int ch, int nchunk, int ncol, int nzl, int kx, int ky, int kz,
-                              const double* __restrict__ part_re, const double* __restrict__ part_im,
-                              const double* __restrict__ Ak, const double* __restrict__ kcoe, CellP c,
-                              double* __restrict__ aks, int nrect, int energy, double* partials) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+// Sum the atom-chunk partials; A_k S(k); energy and stress per k (src/field.f90:
+// 2742-2745, 2803-2815).  Block = 32 entries x 8 runs: sixteen partials at a time
+// are read together and added in their order (which decides the last bit).  A
+// thread per entry, its partials one after another, took 10.3 us at 64 partials
+// of 7 425 entries.
+__global__ void __launch_bounds__(256)
+    k_sfac_reduce(int P, int ch, int nchunk, int ncol, int nzl, int kx, int ky, int kz,
+                  const double* __restrict__ part_re, const double* __restrict__ part_im,
+                  const double* __restrict__ Ak, const double* __restrict__ kcoe, CellP c, double* __restrict__ aks,
+                  int nrect, int energy, double* partials) {
+    __shared__ double s[2][16][32];
+    const int lane = threadIdx.x & 31, run = threadIdx.x >> 5;
+    const int t = blockIdx.x * 32 + lane;
     const int total = ncol * nzl;
     double v[7] = {0, 0, 0, 0, 0, 0, 0};
+    double sr = 0.0, si = 0.0, ak = 0.0;
+    int col = 0, mz = 0, r = 0;
+    const size_t plane = (size_t)ncol * ch * nchunk;
     if (t < total) {
-        const int col = t % ncol;
-        const int mz = t / ncol;          // 0 .. nzl-1
-        const size_t plane = (size_t)ncol * ch * nchunk;
-        const size_t off = (size_t)mz * ncol + col;   // (h*ch + m) == mz
-        const int r = col * nzl + mz;
-        const double ak = Ak[r];
-        double sr = 0.0, si = 0.0;
+        col = t % ncol;
+        mz = t / ncol;          // 0 .. nzl-1
+        r = col * nzl + mz;
+        ak = Ak[r];
+    }
+    const size_t off = (size_t)mz * ncol + col;   // (h*ch + m) == mz
+    for (int base = 0; base < P; base += 16) {
         if (ak != 0.0)   // entries outside the work list have no partials
-            for (int p = 0; p < P; ++p) {
-                sr += part_re[(size_t)p * plane + off];
-                si += part_im[(size_t)p * plane + off];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int p = base + run + 8 * h;
+                if (p < P) {
+                    s[0][run + 8 * h][lane] = part_re[(size_t)p * plane + off];
+                    s[1][run + 8 * h][lane] = part_im[(size_t)p * plane + off];
+                }
             }
+        __syncthreads();
+        if (run < 2 && ak != 0.0)   // run 0 the real parts, run 1 the imaginary ones
+            for (int w = 0; w < min(16, P - base); ++w) sr += s[run][w][lane];
+        __syncthreads();
+    }
+    if (run == 1) s[1][0][lane] = sr;
+    __syncthreads();
+    if (run == 0 && t < total) {
+        si = s[1][0][lane];
         aks[r] = ak * sr;
         aks[nrect + r] = ak * si;
         if (energy && ak != 0.0) {
@@ -254,32 +276,63 @@ __global__ void __launch_bounds__(KF_THREADS) k_kfield(int n, const double* __re
     }
 }
 
-// Sum the column splits in order and scale by 2 (half mesh) * 4 pi / V.
-// ef (3n) += E_rec; efg (6n: xx yy zz xy xz yz) += G_rec; fo (3n) +=
-// q E_rec + G_rec mu.
-__global__ void k_kfield_reduce(int n, int nsplit, int grad, const double* __restrict__ fpart, double scale,
-                                const double* __restrict__ q, const double* __restrict__ mu, double* ef,
-                                double* efg, double* fo, const double* __restrict__ flow, int nlow) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int nv = grad ? 9 : 3;
-    double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int s = 0; s < nsplit; ++s)
-        for (int k = 0; k < nv; ++k) v[k] += fpart[((size_t)s * nv + k) * n + i];
-    for (int s = 0; s < nlow; ++s)
-        for (int k = 0; k < nv; ++k) v[k] += flow[((size_t)s * 9 + k) * n + i];
-    for (int k = 0; k < nv; ++k) v[k] *= scale;
+// Where an atom's field parts are: `np` parts for every atom, or (grid > 0) nq
+// parts from each of the CTAs that share the atom's 128-atom tile, the ntile x
+// ncb units being cut into `grid` ranges (umma::unit0).
+struct FieldParts {
+    int np, ntile, ncb, grid, nq;
+};
+
+// Sum the field parts and scale by 2 (half mesh) * 4 pi / V.  ef (3n) += E_rec;
+// efg (6n: xx yy zz xy xz yz) += G_rec; fo (3n) += q E_rec + G_rec mu.  flow: nlow
+// more parts, with room for nine components each.  Block = 32 atoms x 8 runs:
+// eight parts at a time are read together and added in their order (the order
+// decides the last bit, and the mixed path's results with it).  A thread per
+// atom, its parts one after another, took 9.3 us at 4 056 ions and 85 at 1 536.
+template <int NV>
+__global__ void __launch_bounds__(256)
+    k_kfield_reduce(int n, FieldParts fp, const double* __restrict__ fpart, double scale, const double* __restrict__ q,
+                    const double* __restrict__ mu, double* ef, double* efg, double* fo,
+                    const double* __restrict__ flow, int nlow) {
+    __shared__ double s[8][NV][32];
+    const int lane = threadIdx.x & 31, run = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    double v[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = 0.0;
+    int np = fp.np;
+    if (fp.grid > 0) {   // (32 atoms are of one 128-atom tile)
+        const long units = (long)fp.ntile * fp.ncb, t0 = (long)(blockIdx.x * 32 / 128) * fp.ncb;
+        np = (umma::range_of(t0 + fp.ncb - 1, units, fp.grid) - umma::range_of(t0, units, fp.grid) + 1) * fp.nq;
+    }
+    for (int base = 0; base < np + nlow; base += 8) {
+        const int p = base + run;
+        if (p < np + nlow && i < n) {
+            const double* o = p < np ? fpart + (size_t)p * NV * n : flow + (size_t)(p - np) * 9 * n;
+#pragma unroll
+            for (int k = 0; k < NV; ++k) s[run][k][lane] = o[(size_t)k * n + i];
+        }
+        __syncthreads();
+        if (run == 0)
+            for (int w = 0; w < min(8, np + nlow - base); ++w)
+#pragma unroll
+                for (int k = 0; k < NV; ++k) v[k] += s[w][k][lane];
+        __syncthreads();
+    }
+    if (run != 0 || i >= n) return;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] *= scale;
     if (ef) { ef[i] += v[0]; ef[n + i] += v[1]; ef[2 * n + i] += v[2]; }
-    if (grad && efg)
-        for (int k = 0; k < 6; ++k) efg[(size_t)k * n + i] += v[3 + k];
+    if (NV == 9 && efg)
+        for (int k = 0; k < 6; ++k) efg[(size_t)k * n + i] += v[(3 + k) % NV];
     if (fo) {
         const double qi = q ? q[i] : 0.0;
         double f0 = qi * v[0], f1 = qi * v[1], f2 = qi * v[2];
-        if (grad && mu) {
+        if (NV == 9 && mu) {
             const double m0 = mu[i], m1 = mu[n + i], m2 = mu[2 * n + i];
-            f0 += v[3] * m0 + v[6] * m1 + v[7] * m2;
-            f1 += v[6] * m0 + v[4] * m1 + v[8] * m2;
-            f2 += v[7] * m0 + v[8] * m1 + v[5] * m2;
+            f0 += v[3 % NV] * m0 + v[6 % NV] * m1 + v[7 % NV] * m2;
+            f1 += v[6 % NV] * m0 + v[4 % NV] * m1 + v[8 % NV] * m2;
+            f2 += v[7 % NV] * m0 + v[8 % NV] * m1 + v[5 % NV] * m2;
         }
         fo[i] += f0; fo[n + i] += f1; fo[2 * n + i] += f2;
     }
@@ -822,10 +875,17 @@ struct RecLaunch {
 
 // acc = src (copy), or acc += a src with a = rz / dAd, the step of the
 // current PCG iteration (read before the iteration's last kernel advances rz).
+// Two sets in one launch: m entries of src, then ml of srcl.
 __global__ void k_aks_axpy(int m, const DevScalars* __restrict__ sc, int copy, const double* __restrict__ src,
-                           double* __restrict__ acc) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= m) return;
+                           double* __restrict__ acc, int ml, const double* __restrict__ srcl,
+                           double* __restrict__ accl) {
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= m + ml) return;
+    if (t >= m) {
+        t -= m;
+        src = srcl;
+        acc = accl;
+    }
     if (copy) acc[t] = src[t];
     else acc[t] = fma(sc->rz / sc->dAd, src[t], acc[t]);
 }
@@ -895,11 +955,9 @@ __global__ void k_aks_energy_low(int ncol, int nzmax, const int* __restrict__ co
 // accumulators.
 void launch_aks_accumulate(cudaStream_t st, const KGrid& kg, RecScratch& rs, const DevScalars* d, int copy) {
     const int m = 2 * kg.nrect;
-    k_aks_axpy<<<(m + 255) / 256, 256, 0, st>>>(m, d, copy, rs.aks, rs.aks_acc);
-    if (rs.low.ncol > 0 && rs.low.aks_acc) {
-        const int ml = 2 * rs.low.ncol * rs.low.nzmax;
-        k_aks_axpy<<<(ml + 255) / 256, 256, 0, st>>>(ml, d, copy, rs.low.aks, rs.low.aks_acc);
-    }
+    const bool low = rs.low.ncol > 0 && rs.low.aks_acc;
+    const int ml = low ? 2 * rs.low.ncol * rs.low.nzmax : 0;
+    k_aks_axpy<<<(m + ml + 255) / 256, 256, 0, st>>>(m, d, copy, rs.aks, rs.aks_acc, ml, rs.low.aks, rs.low.aks_acc);
 }
 
 static RecLaunch plan(int n, const KGrid& kg) {
@@ -1074,7 +1132,8 @@ int launch_t7_field(cudaStream_t st, int n, CellP c, const KGrid& kg, RecScratch
                                                                   kg.nrect, c, t.fimg);
     tc7::k_kfield_t7<NMOM><<<grid, tc7::FTHREADS, NMOM == 3 ? t.smem_f3 : t.smem_f2, st>>>(
         n, t.ntile_f, t.ncol, ncb, t.aimg, t.xy, t.fimg, t.kx, t.ky, t.KZ, c, rs.fpart, &d->tc_err);
-    tc7::k_t7_freduce<NV><<<(n + 31) / 32, 256, 0, st>>>(n, t.ntile_f, ncb, grid, rs.fpart, scale, q, mu, ef, efg, fo);
+    const FieldParts fp{0, t.ntile_f, ncb, grid, tc7::NQ};
+    k_kfield_reduce<NV><<<(n + 31) / 32, 256, 0, st>>>(n, fp, rs.fpart, scale, q, mu, ef, efg, fo, nullptr, 0);
     return 3;
 }
 
@@ -1092,7 +1151,7 @@ void launch_ewald_rec(cudaStream_t st, int n, const double* sx, const double* sy
     const bool low = mixed && rs.low.ncol > 0;
     const int nchunk32 = (kg.nzl + TM - 1) / TM;
     const int total = kg.ncol * kg.nzl;
-    const int rb = (total + 255) / 256;
+    const int rb = (total + 255) / 256, rb32 = (total + 31) / 32;
     prof->begin(PK_SFAC);
     int nk = 2 + (fl.energy ? 1 : 0);
     if (fl.reuse) {
@@ -1152,7 +1211,7 @@ void launch_ewald_rec(cudaStream_t st, int n, const double* sx, const double* sy
                 k_sfac32<0><<<g1, SF_THREADS, 0, st>>>(n, L.natom_chunk, rs.fixed, rs.tab, q, mu, c, ky, kz, kg.ncol,
                                                          nchunk32, fl.with_q, kg.items, kg.nitems, pre, pim);
         }
-        k_sfac_reduce<<<rb, 256, 0, st>>>(Pr, TM, nchunk32, kg.ncol, kg.nzl, kx, ky, kz, pre, pim, kg.Ak_hi, kg.kcoe, c,
+        k_sfac_reduce<<<rb32, 256, 0, st>>>(Pr, TM, nchunk32, kg.ncol, kg.nzl, kx, ky, kz, pre, pim, kg.Ak_hi, kg.kcoe, c,
                                           rs.aks, kg.nrect, fl.energy, part.buf);
     } else if (rs.t7.on) {
         nk = launch_t7_sfac(st, n, sx, sy, sz, q, mu, c, kg, fl, rs, part, d);
@@ -1166,10 +1225,10 @@ void launch_ewald_rec(cudaStream_t st, int n, const double* sx, const double* sy
         else if (L.CH == 12) SFAC(12);
         else SFAC(8);
 #undef SFAC
-        k_sfac_reduce<<<rb, 256, 0, st>>>(L.P, L.CH, L.nchunk, kg.ncol, kg.nzl, kx, ky, kz, pre, pim, kg.Ak, kg.kcoe,
+        k_sfac_reduce<<<rb32, 256, 0, st>>>(L.P, L.CH, L.nchunk, kg.ncol, kg.nzl, kx, ky, kz, pre, pim, kg.Ak, kg.kcoe,
                                           c, rs.aks, kg.nrect, fl.energy, part.buf);
     }
-    if (fl.energy && !fl.reuse && !rs.t7.on) launch_reduce_partials(st, part.buf, rb, 7, d->rec, 0);
+    if (fl.energy && !fl.reuse && !rs.t7.on) launch_reduce_partials(st, part.buf, rb32, 7, d->rec, 0);
     if (low && !fl.reuse) {
         LowK& lk = rs.low;
         int Pl = lk.P;
@@ -1218,7 +1277,7 @@ void launch_ewald_rec(cudaStream_t st, int n, const double* sx, const double* sy
         prof->end(nk);
         return;
     }
-    int nsplit_f = L.nsplit;
+    FieldParts fparts{L.nsplit, 0, 0, 0, 0};
     if (mixed && rs.tc.on) {
         // field pass on the tensor cores: NQ column parts per atom
         const TcK& t = rs.tc;
@@ -1242,7 +1301,7 @@ void launch_ewald_rec(cudaStream_t st, int n, const double* sx, const double* sy
                                                                             t.KZ, t.XYW, c, rs.fpart, &d->tc_err);
             prof->detail_end(PD_TC_FIELD, 6.0 * 2.0 * n * (4.0 * t.nsph) * (2.0 * kg.nzl));
         }
-        nsplit_f = 2 * tcf::NQ;   // NQ column parts in each of the 2 column slots
+        fparts = FieldParts{2 * tcf::NQ, 0, 0, 0, 0};   // NQ column parts in each of the 2 column slots
         nk += 1;
         if (low) nk += launch_low_field(st, n, c, grad, rs, d, prof);
     } else if (mixed) {
@@ -1271,10 +1330,13 @@ void launch_ewald_rec(cudaStream_t st, int n, const double* sx, const double* sy
                                                       sph ? kg.fzr : nullptr);
         nk++;
     }
-    k_kfield_reduce<<<(n + 255) / 256, 256, 0, st>>>(n, nsplit_f, grad ? 1 : 0, rs.fpart, scale, fl.with_q ? q : nullptr,
-                                                    fl.with_mu ? mu : nullptr, fl.field ? ef : nullptr, efg,
-                                                    fl.forces ? fo : nullptr, low ? rs.low.fpart : nullptr,
-                                                    low ? (rs.low.tc ? tc4::NQ : LK_SPLIT) : 0);
+    const double *fq = fl.with_q ? q : nullptr, *fm = fl.with_mu ? mu : nullptr, *fl_low = low ? rs.low.fpart : nullptr;
+    double *oe = fl.field ? ef : nullptr, *of = fl.forces ? fo : nullptr;
+    const int nlow = low ? (rs.low.tc ? tc4::NQ : LK_SPLIT) : 0;
+    if (grad)
+        k_kfield_reduce<9><<<(n + 31) / 32, 256, 0, st>>>(n, fparts, rs.fpart, scale, fq, fm, oe, efg, of, fl_low, nlow);
+    else
+        k_kfield_reduce<3><<<(n + 31) / 32, 256, 0, st>>>(n, fparts, rs.fpart, scale, fq, fm, oe, efg, of, fl_low, nlow);
     prof->end(nk);
 }
 

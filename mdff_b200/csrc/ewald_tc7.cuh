@@ -514,14 +514,6 @@ struct FLayout {
     __host__ __device__ uint32_t smem_bytes() const { return b_off + NBS * stage_bytes + 128u; }
 };
 
-// The (tile, column block) units are cut into `grid` contiguous, nearly equal
-// ranges.  A tile's parts are numbered by the CTAs that touch it.
-__host__ __device__ __forceinline__ long unit0(int cta, long units, int grid) { return (long)cta * units / grid; }
-__host__ __device__ __forceinline__ int cta_of(long unit, long units, int grid) {
-    int c = (int)(((unit + 1) * grid - 1) / units);
-    return c;   // the largest c with unit0(c) <= unit
-}
-
 // Per position update: the A digit image of each 128-atom tile (K = (m, cos/sin), KZ bytes per row).
 __global__ void k_t7f_aimage(int n, int ntile, const double* __restrict__ sz, int kz, int KZ, uint8_t* __restrict__ img) {
     const int nch = KZ / 16;
@@ -654,7 +646,8 @@ __device__ __forceinline__ double join7(float d0, float d1, float d2, float d3, 
     return fma(fma(fma(a, 65536.0, b), 65536.0, c), 256.0, (double)__float_as_int(d6));
 }
 
-// `grid` CTAs over (tile, column block) units.  Writes
+// `grid` CTAs, each an equal contiguous range of the (tile, column block) units
+// (umma::unit0).  Writes
 // fpart[((slot * NQ + part) * nv + component) * n + i], slot counted from the
 // first CTA of the atom's tile, nv = 3 or 9.
 //
@@ -682,8 +675,8 @@ __global__ void __launch_bounds__(FTHREADS, 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const long units = (long)ntile * ncb;
     const int grid = gridDim.x;
-    const long u0 = unit0(blockIdx.x, units, grid);
-    const int cnt = (int)(unit0(blockIdx.x + 1, units, grid) - u0), tile0 = (int)(u0 / ncb), q0 = (int)(u0 % ncb);
+    const long u0 = umma::unit0(blockIdx.x, units, grid);
+    const int cnt = (int)(umma::unit0(blockIdx.x + 1, units, grid) - u0), tile0 = (int)(u0 / ncb), q0 = (int)(u0 % ncb);
     if (tid == 0) {
         umma::mbar_init(&afull, 1);
         umma::mbar_init(&afree, 1);
@@ -861,7 +854,7 @@ __global__ void __launch_bounds__(FTHREADS, 1)
             if (lane == 0) umma::mbar_arrive(&bempty[bs]);
             const bool last = q == ncb - 1 || it == cnt - 1;
             if (last && i < n) {   // the tile's segment is done
-                const int slot = (int)blockIdx.x - cta_of((long)tile * ncb, units, grid);
+                const int slot = (int)blockIdx.x - umma::range_of((long)tile * ncb, units, grid);
                 double* o = fpart + (size_t)(slot * NQ + part) * NV * n + i;
                 const double b3[3] = {2.0 * PI * c.B[2], 2.0 * PI * c.B[5], 2.0 * PI * c.B[8]};
                 for (int e = 0; e < 3; ++e) o[(size_t)e * n] = fma(b3[e], SI1, E[e]);
@@ -882,52 +875,6 @@ __global__ void __launch_bounds__(FTHREADS, 1)
     if (warp == 0) {
         umma::fence_after_sync();
         umma::tmem_dealloc(tmem, 512);
-    }
-}
-
-// The parts of each atom summed in a fixed order (eight interleaved runs of
-// parts, then the runs), scaled, and added to the field, the gradient and the
-// forces (src/field.f90:2776-2789).  Block = 32 atoms x 8 runs.
-template <int NV>
-__global__ void __launch_bounds__(256)
-    k_t7_freduce(int n, int ntile, int ncb, int grid, const double* __restrict__ fpart, double scale,
-                 const double* __restrict__ q, const double* __restrict__ mu, double* ef, double* efg, double* fo) {
-    __shared__ double s[8][NV][32];
-    const int lane = threadIdx.x & 31, run = threadIdx.x >> 5;
-    const int i = blockIdx.x * 32 + lane;
-    const long units = (long)ntile * ncb;
-    double v[NV];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) v[k] = 0.0;
-    if (i < n) {
-        const long t0 = (long)(i / 128) * ncb;
-        const int np = (cta_of(t0 + ncb - 1, units, grid) - cta_of(t0, units, grid) + 1) * NQ;
-        for (int p = run; p < np; p += 8)
-#pragma unroll
-            for (int k = 0; k < NV; ++k) v[k] += fpart[((size_t)p * NV + k) * n + i];
-    }
-#pragma unroll
-    for (int k = 0; k < NV; ++k) s[run][k][lane] = v[k];
-    __syncthreads();
-    if (run != 0 || i >= n) return;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        for (int w = 1; w < 8; ++w) v[k] += s[w][k][lane];
-        v[k] *= scale;
-    }
-    if (ef) { ef[i] += v[0]; ef[n + i] += v[1]; ef[2 * n + i] += v[2]; }
-    if (NV == 9 && efg)
-        for (int k = 0; k < 6; ++k) efg[(size_t)k * n + i] += v[(3 + k) % NV];
-    if (fo) {
-        const double qi = q ? q[i] : 0.0;
-        double f0 = qi * v[0], f1 = qi * v[1], f2 = qi * v[2];
-        if (NV == 9 && mu) {
-            const double m0 = mu[i], m1 = mu[n + i], m2 = mu[2 * n + i];
-            f0 += v[3 % NV] * m0 + v[6 % NV] * m1 + v[7 % NV] * m2;
-            f1 += v[6 % NV] * m0 + v[4 % NV] * m1 + v[8 % NV] * m2;
-            f2 += v[7 % NV] * m0 + v[8 % NV] * m1 + v[5 % NV] * m2;
-        }
-        fo[i] += f0; fo[n + i] += f1; fo[2 * n + i] += f2;
     }
 }
 

@@ -272,6 +272,14 @@ __device__ __forceinline__ void slices4x4(uint32_t w0, uint32_t w1, uint32_t w2,
     s1 = __byte_perm(u01, u23, 0x7632);
 }
 
+// `units` pieces of work cut into `grid` contiguous, nearly equal ranges: the
+// first unit of a range, and the range that holds a unit (the largest r with
+// unit0(r) <= unit).
+__host__ __device__ __forceinline__ long unit0(int r, long units, int grid) { return (long)r * units / grid; }
+__host__ __device__ __forceinline__ int range_of(long unit, long units, int grid) {
+    return (int)(((unit + 1) * grid - 1) / units);
+}
+
 // Conversions on the FP64 pipe instead of the conversion unit: 1.5 * 2^52
 // has a unit in the last place of 1, so v + M rounds v to the nearest
 // integer (ties to even, as cvt.rni) and its low word is that integer for
