@@ -23,6 +23,33 @@ __device__ __forceinline__ double pairvec_exact(const CellP& c, double si1, doub
     return __dadd_rn(__dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)), __dmul_rn(rz, rz));
 }
 
+// The same vector to rounding, for force sums whose cutoff is below half the
+// cell's narrowest width (GEOM_*, set by the host): the image by adding and
+// taking off 1.5 2^52 (d - rint(d); where the two images of a pair are equally
+// far, d = +-1/2, both are beyond the cutoff), fused products, and for a
+// diagonal cell matrix three products instead of nine.  18 or 24 FP64
+// instructions against 45.
+constexpr int GEOM_EXACT = 0, GEOM_GENERAL = 1, GEOM_DIAGONAL = 2;
+__device__ __forceinline__ double pairvec(int geom, const CellP& c, double si1, double si2, double si3, double sj1,
+                                          double sj2, double sj3, double& rx, double& ry, double& rz) {
+    if (geom == GEOM_EXACT) return pairvec_exact(c, si1, si2, si3, sj1, sj2, sj3, rx, ry, rz);
+    constexpr double M = 6755399441055744.0;
+    double d1 = si1 - sj1, d2 = si2 - sj2, d3 = si3 - sj3;
+    d1 -= (d1 + M) - M;
+    d2 -= (d2 + M) - M;
+    d3 -= (d3 + M) - M;
+    if (geom == GEOM_DIAGONAL) {
+        rx = d1 * c.A[0];
+        ry = d2 * c.A[4];
+        rz = d3 * c.A[8];
+    } else {
+        rx = fma(d3, c.A[2], fma(d2, c.A[1], d1 * c.A[0]));
+        ry = fma(d3, c.A[5], fma(d2, c.A[4], d1 * c.A[3]));
+        rz = fma(d3, c.A[8], fma(d2, c.A[7], d1 * c.A[6]));
+    }
+    return fma(rz, rz, fma(ry, ry, rx * rx));
+}
+
 // errfc (src/functions.f90:28-39): the reference's fitted erfc (Numerical
 // Recipes' Chebyshev approximation), selectable for bit-level parity studies.
 __device__ __forceinline__ double erfc_fit(double x) {
@@ -51,15 +78,27 @@ static __device__ const double c_erfcx[9][14] = {
     {1.66335348426821877e-01, -1.17998505802925941e-02, 8.08580680188634841e-04, -5.36792390766808417e-05, 3.46095538099348485e-06, -2.17170478094227272e-07, 1.32862326187598925e-08, -7.93740250497401040e-10, 4.63689003375204657e-11, -2.65200852373283976e-12, 1.48653925733325675e-13, -8.17503930574837552e-15, 4.45764831070709062e-16, -2.36471931146022244e-17},
     {1.45589721275038553e-01, -9.11406438318088270e-03, 5.54922220457831146e-04, -3.29262948463923468e-05, 1.90711868006086389e-06, -1.07987866137007266e-07, 5.98543099979860756e-09, -3.25114305970638778e-10, 1.73236948280893169e-11, -9.06373617437550905e-13, 4.65997853503172364e-14, -2.35626153976442944e-15, 1.18228113910100869e-16, -5.79197552373421933e-18},
     {1.29345274785987924e-01, -7.23608285365383297e-03, 3.95741642117046835e-04, -2.11864557360015355e-05, 1.11162170640691086e-06, -5.72221681771075831e-08, 2.89260098733738314e-09, -1.43713417692772748e-10, 7.02301408394134694e-12, -3.37808096316975056e-13, 1.60031161014207372e-14, -7.47136752260601365e-16, 3.46405779482777296e-17, -1.57285591596023904e-18}};
-__device__ __forceinline__ double erfc_ex2(double x, double ex2) {
+// tab: c_erfcx, or a block's copy of it in shared memory (ERFCX_LEN doubles): the
+// lanes of a warp are in different intervals, whose coefficients lie on different
+// banks there but on different lines in L1.
+constexpr int ERFCX_LEN = 9 * 14;
+__device__ __forceinline__ double erfc_ex2(double x, double ex2, const double* tab = &c_erfcx[0][0]) {
     if (!(x >= 0.0 && x < 4.5)) return erfc(x);
     const int j = (int)(x * 2.0);
     const double t = fma(x, 4.0, -(double)(2 * j + 1));
-    const double* c = c_erfcx[j];
-    double p = __ldg(c + 13);
+    const double* c = tab + 14 * j;
+    double p = c[13];
 #pragma unroll
-    for (int k = 12; k >= 0; --k) p = fma(p, t, __ldg(c + k));
+    for (int k = 12; k >= 0; --k) p = fma(p, t, c[k]);
     return ex2 * p;
+}
+
+// four doubles of a 32-byte record in one 256-bit load: a gather of records costs
+// one L1 request per warp instead of one per component
+__device__ __forceinline__ double4 ld_rec(const double4* __restrict__ p) {
+    double4 v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
 }
 
 // Inverse factorials 1/m! by the recurrence inv_m = inv_{m-1} / m in IEEE

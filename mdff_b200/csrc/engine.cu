@@ -94,6 +94,7 @@ struct mdff_ctx {
     double *sx = nullptr, *sy = nullptr, *sz = nullptr;
     double *xs = nullptr, *ys = nullptr, *zs = nullptr;
     int* type = nullptr;
+    double4 *rec = nullptr, *mrec = nullptr;   // gather records: (fractional coordinates, type), (dipole, charge)
     double *q = nullptr, *mass = nullptr, *alpha = nullptr, *inv_alpha = nullptr, *dip0 = nullptr;
     double *mu = nullptr, *mu_ind = nullptr, *Estat = nullptr, *Eind = nullptr, *E = nullptr;
     double *cg_r = nullptr, *cg_z = nullptr, *cg_d = nullptr, *cg_Ad = nullptr, *mu_save = nullptr;
@@ -135,7 +136,6 @@ struct mdff_ctx {
     // Coulomb list entry), written by the charge pass of each force evaluation
     float2* ddtab = nullptr;
     double2* ddtab64 = nullptr;          // FP64 path
-    double* ddrec64 = nullptr;           // [8n]
     bool ddtab_off = false;              // FP64 path: no memory for the table, the operator is evaluated per pair
     int* ddnbr = nullptr;
     int* ddcnt = nullptr;
@@ -388,6 +388,7 @@ void build_pair_consts(mdff_ctx* ctx, std::vector<PairConst>& tab) {
             P.db_j = p.dip_pol_damp_b[jt][it][jt];
             P.dc_j = p.dip_pol_damp_c[jt][it][jt];
             P.dk_j = p.dip_pol_damp_k[jt][it][jt];
+            P.qj = p.qch[jt];
             P.ldamp = (p.ldip_damping[it][it][jt] || p.ldip_damping[jt][it][jt]) ? 1 : 0;
         }
     ctx->ptail = ctx->ptail / ctx->u.press / ctx->cell.omega / 3.0;
@@ -517,6 +518,17 @@ inline int nb(int n, int t = 256) { return (n + t - 1) / t; }
 double selfa(const mdff_ctx* ctx) { return ctx->alphaES / std::sqrt(PI); }
 double selfa2(const mdff_ctx* ctx) { return 2.0 * selfa(ctx) * ctx->alphaES * ctx->alphaES / 3.0; }
 
+// How the force sums take pair vectors (common.cuh): the short form where the
+// cutoffs stay below half the cell's narrowest width, so that no pair inside
+// them has two images equally far.
+int geom_of(const mdff_ctx* ctx) {
+    const double wmin = std::min(ctx->W[0], std::min(ctx->W[1], ctx->W[2]));
+    if (!(2.0 * rlist_max(ctx, 0.0) < wmin * (1.0 - 1e-9))) return GEOM_EXACT;
+    const double* A = ctx->cell.A;
+    const bool diag = A[1] == 0.0 && A[2] == 0.0 && A[3] == 0.0 && A[5] == 0.0 && A[6] == 0.0 && A[7] == 0.0;
+    return diag ? GEOM_DIAGONAL : GEOM_GENERAL;
+}
+
 DirFlags dir_flags(const mdff_ctx* ctx) {
     DirFlags f;
     std::memset(&f, 0, sizeof f);
@@ -524,6 +536,8 @@ DirFlags dir_flags(const mdff_ctx* ctx) {
     f.alpha = ctx->alphaES;
     f.cutsq = ctx->cut_coul * ctx->cut_coul;
     f.erfc_ref = ctx->p.erfc_ref ? 1 : 0;
+    f.fast = ctx->p.precision == MDFF_PREC_FP64;
+    f.geom = geom_of(ctx);
     return f;
 }
 
@@ -550,15 +564,15 @@ void dd_field_real(mdff_ctx* ctx, const double* m, double* out) {
     }
     const NList& L = coul_list(ctx);
     if (ctx->ddtab64 && ctx->ddtab_epoch == ctx->rs.want_epoch && ctx->ddtab_lcap == L.cap) {
-        launch_ewald_ddtab64(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, m, ctx->cell, ctx->ddnbr, ctx->ddcnt, L.cap,
-                             ctx->ddtab64, ctx->ddrec64, out, ctx->g_dd);
+        launch_ewald_ddtab64(ctx->st, n, ctx->rec, ctx->mrec, m, ctx->cell, ctx->ddnbr, ctx->ddcnt, L.cap, ctx->ddtab64,
+                             out, ctx->g_dd);
         ctx->prof.end(2);
         return;
     }
     DirFlags f = dir_flags(ctx);
     f.dd = 1;
     f.field = 1;
-    launch_ewald_dir(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, ctx->type, nullptr, m, ctx->cell, L, ctx->pc, f, out,
+    launch_ewald_dir(ctx->st, n, ctx->rec, ctx->mrec, nullptr, m, ctx->cell, L, ctx->pc, f, out,
                      nullptr, nullptr, ctx->part, ctx->dsc, ctx->g_dir);
     ctx->prof.end(1);
 }
@@ -611,7 +625,6 @@ int arm_ddtab(mdff_ctx* ctx, DirFlags& f) {
     }
     if (!ctx->ddcnt) TRY(dalloc(ctx, &ctx->ddcnt, ctx->n));
     if (mixed && !ctx->ddrec) TRY(dalloc(ctx, &ctx->ddrec, 2 * (size_t)ctx->n));
-    if (!mixed && !ctx->ddrec64) TRY(dalloc(ctx, &ctx->ddrec64, 8 * (size_t)ctx->n));
     f.ddtab = ctx->ddtab;
     f.ddtab64 = ctx->ddtab64;
     f.ddnbr = ctx->ddnbr;
@@ -633,7 +646,7 @@ int static_field(mdff_ctx* ctx) {
     f.field = 1;
     TRY(arm_ddtab(ctx, f));
     ctx->prof.begin(PK_DIR);
-    launch_ewald_dir(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, ctx->type, ctx->q, ctx->dip0, ctx->cell, coul_list(ctx),
+    launch_ewald_dir(ctx->st, n, ctx->rec, ctx->mrec, ctx->q, ctx->dip0, ctx->cell, coul_list(ctx),
                      ctx->pc, f, ctx->Estat, nullptr, nullptr, ctx->part, ctx->dsc, ctx->g_dir);
     ctx->prof.end(2);
     RecFlags rf{1, ctx->any_dip0 ? 1 : 0, 1, 0, 0, 0, ctx->p.precision, 0};
@@ -660,7 +673,7 @@ int fused_initial_field(mdff_ctx* ctx) {
     f.field = 1;
     TRY(arm_ddtab(ctx, f));
     ctx->prof.begin(PK_DIR);
-    launch_ewald_dir(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, ctx->type, ctx->q, ctx->dip0, ctx->cell, coul_list(ctx),
+    launch_ewald_dir(ctx->st, n, ctx->rec, ctx->mrec, ctx->q, ctx->dip0, ctx->cell, coul_list(ctx),
                      ctx->pc, f, ctx->Estat, nullptr, nullptr, ctx->part, ctx->dsc, ctx->g_dir);
     ctx->prof.end(2);
     dd_field_real(ctx, ctx->mu_ind, ctx->Eind);
@@ -970,7 +983,7 @@ int autotune(mdff_ctx* ctx) {
     f.field = 1;
     f.forces = 1;
     ctx->g_dir = pick([&](int g) {
-        launch_ewald_dir(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, ctx->type, ctx->q, ctx->mu, ctx->cell, coul_list(ctx),
+        launch_ewald_dir(ctx->st, n, ctx->rec, ctx->mrec, ctx->q, ctx->mu, ctx->cell, coul_list(ctx),
                          ctx->pc, f, ctx->ef, nullptr, ctx->fcoul, ctx->part, ctx->dsc, g);
     }, gs, 3);
     if (ctx->p.precision == MDFF_PREC_MIXED) {
@@ -981,7 +994,7 @@ int autotune(mdff_ctx* ctx) {
         fs.damp = 1;
         fs.field = 1;
         TRY(arm_ddtab(ctx, fs));
-        launch_ewald_dir(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, ctx->type, ctx->q, ctx->mu, ctx->cell, coul_list(ctx),
+        launch_ewald_dir(ctx->st, n, ctx->rec, ctx->mrec, ctx->q, ctx->mu, ctx->cell, coul_list(ctx),
                          ctx->pc, fs, ctx->Estat, nullptr, nullptr, ctx->part, ctx->dsc, ctx->g_dir);
         ctx->g_dd = pick([&](int g) {
             launch_ewald_ddtab(ctx->st, n, ctx->rs.fixed, ctx->mu, ctx->cell, ctx->ddnbr, ctx->ddcnt,
@@ -1008,11 +1021,11 @@ int autotune(mdff_ctx* ctx) {
         fs.field = 1;
         TRY(arm_ddtab(ctx, fs));
         if (fs.ddtab64) {
-            launch_ewald_dir(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, ctx->type, ctx->q, ctx->mu, ctx->cell, coul_list(ctx),
+            launch_ewald_dir(ctx->st, n, ctx->rec, ctx->mrec, ctx->q, ctx->mu, ctx->cell, coul_list(ctx),
                              ctx->pc, fs, ctx->Estat, nullptr, nullptr, ctx->part, ctx->dsc, ctx->g_dir);
             ctx->g_dd = pick([&](int g) {
-                launch_ewald_ddtab64(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, ctx->mu, ctx->cell, ctx->ddnbr, ctx->ddcnt,
-                                     coul_list(ctx).cap, ctx->ddtab64, ctx->ddrec64, ctx->Eind, g);
+                launch_ewald_ddtab64(ctx->st, n, ctx->rec, ctx->mrec, ctx->mu, ctx->cell, ctx->ddnbr, ctx->ddcnt,
+                                     coul_list(ctx).cap, ctx->ddtab64, ctx->Eind, g);
             }, gs, 3);
         }
     }
@@ -1035,16 +1048,21 @@ int engforce_device(mdff_ctx* ctx) {
     if (!p.lvnlist) TRY(build_lists(ctx, 0.0));
     else if (!ctx->have_list) TRY(build_lists(ctx, p.skindiff));   // lists dropped (an interrupted RMC chain)
     ctx->prof.begin(PK_OTHER);
-    launch_frac(ctx->st, n, ctx->x, ctx->y, ctx->z, ctx->cell, ctx->sx, ctx->sy, ctx->sz);
+    k_frac_rec<<<nb(n), 256, 0, ctx->st>>>(n, ctx->x, ctx->y, ctx->z, ctx->type, ctx->cell, ctx->sx, ctx->sy, ctx->sz,
+                                           ctx->rec);
     ctx->prof.end(1);
     ctx->rs.want_epoch++;   // positions may have changed: rebuild the phase tables
     if (p.autotune && !ctx->tuned) TRY(autotune(ctx));
     std::memset(&ctx->en, 0, sizeof ctx->en);
     bool nonb = p.lnmlj || p.lbmhft || p.lbmhftd || p.lmorse;
     if (nonb) {
-        PairFlags fl{p.lnmlj, p.lbmhft, p.lbmhftd, p.lmorse, p.trunc, ctx->ntype};
+        int lj126 = 1;
+        for (int a = 0; a < ctx->ntype; ++a)
+            for (int b = 0; b < ctx->ntype; ++b) lj126 &= p.plj[a][b] == 6.0 && p.qlj[a][b] == 12.0;
+        PairFlags fl{p.lnmlj, p.lbmhft, p.lbmhftd, p.lmorse, p.trunc, ctx->ntype, lj126, geom_of(ctx),
+                     p.precision == MDFF_PREC_FP64};
         ctx->prof.begin(PK_PAIR);
-        launch_pair(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, ctx->type, ctx->cell, ctx->lv, ctx->pc, fl, ctx->fx, ctx->fy,
+        launch_pair(ctx->st, n, ctx->rec, ctx->cell, ctx->lv, ctx->pc, fl, ctx->fx, ctx->fy,
                     ctx->fz, ctx->part, ctx->dsc);
         ctx->prof.end(2);
     } else {
@@ -1077,7 +1095,7 @@ int engforce_device(mdff_ctx* ctx) {
         CK(cudaMemsetAsync(ctx->ef, 0, sizeof(double) * n3, ctx->st));
         if (efg) CK(cudaMemsetAsync(ctx->efg, 0, sizeof(double) * 6 * n, ctx->st));
         ctx->prof.begin(PK_DIR);
-        launch_ewald_dir(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, ctx->type, ctx->q, ctx->mu, ctx->cell, coul_list(ctx),
+        launch_ewald_dir(ctx->st, n, ctx->rec, ctx->mrec, ctx->q, ctx->mu, ctx->cell, coul_list(ctx),
                          ctx->pc, f, ctx->ef, ctx->efg, ctx->fcoul, ctx->part, ctx->dsc, ctx->g_dir);
         ctx->prof.end(2);
         RecFlags rf{ctx->any_q ? 1 : 0, dip ? 1 : 0, p.doefield ? 1 : 0, (efg || dip) ? 1 : 0, 1, 1, p.precision,
@@ -1600,7 +1618,7 @@ bool graph_eligible(const mdff_ctx* ctx) {
         (!ctx->ddcnt || !ctx->ddrec || (size_t)ctx->n * coul_list(ctx).cap > ctx->ddtab_cap))
         return false;
     if (p.lcoulomb && p.precision == MDFF_PREC_FP64 && ctx->npol > 0 && !ctx->ddtab_off &&
-        (!ctx->ddcnt || !ctx->ddrec64 || (size_t)ctx->n * coul_list(ctx).cap > ctx->ddtab_cap))
+        (!ctx->ddcnt || (size_t)ctx->n * coul_list(ctx).cap > ctx->ddtab_cap))
         return false;
     return true;
 }
@@ -3084,7 +3102,6 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
     ctx->grid = CellGrid();
     ctx->ddcnt = nullptr;   // freed with the rest; the pair table itself is kept
     ctx->ddrec = nullptr;
-    ctx->ddrec64 = nullptr;
     ctx->ddtab_epoch = -1;
     ctx->ddtab_off = false;
     ctx->have_system = ctx->have_list = ctx->forces_valid = ctx->md_started = false;
@@ -3139,6 +3156,8 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
     TRY(dalloc(ctx, &ctx->hist, (size_t)ctx->nhist * 3 * n));
     TRY(dalloc(ctx, &ctx->coef, PLAN_LEN));
     TRY(dalloc(ctx, &ctx->type, n));
+    TRY(dalloc(ctx, &ctx->rec, n));
+    TRY(dalloc(ctx, &ctx->mrec, n));
     TRY(dalloc(ctx, &ctx->pc, NT * NT));
     TRY(dalloc(ctx, &ctx->dsc, 1));
     TRY(dalloc(ctx, &ctx->d_overflow, 1));

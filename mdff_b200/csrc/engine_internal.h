@@ -40,6 +40,7 @@ struct PairConst {
     int dk_i, dk_j;
     int ldamp;   // ldip_damping(ti,ti,tj) .or. ldip_damping(tj,ti,tj)
     int pad;
+    double qj;   // charge of type tj
 };
 
 // Per-kernel-group timing with CUDA events on the context's stream (the
@@ -188,9 +189,11 @@ void launch_skin_check(cudaStream_t st, int n, const double* sx, const double* s
                        Partials& part, DevScalars* d);
 
 // Short-range pair loop: LJ / BMH(FTD) / Morse, forces written (not added).
-struct PairFlags { int lj, bmh, bmhftd, morse, trunc, ntype; };
-void launch_pair(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz, const int* type,
-                 CellP c, const NList& l, const PairConst* pc, PairFlags fl,
+// lj126: every type pair has the exponents 6 and 12; geom: GEOM_* (common.cuh)
+// fast: the short forms of the pair arithmetic (FP64 path)
+struct PairFlags { int lj, bmh, bmhftd, morse, trunc, ntype, lj126, geom, fast; };
+// rec: (fractional coordinates, type) of k_frac_rec.
+void launch_pair(cudaStream_t st, int n, const double4* rec, CellP c, const NList& l, const PairConst* pc, PairFlags fl,
                  double* fx, double* fy, double* fz, Partials& part, DevScalars* d);
 
 // Real-space multipole Ewald (charges + dipoles).
@@ -202,6 +205,8 @@ struct DirFlags {
     double alpha;          // Ewald alpha
     double cutsq;          // verlet_coul%cut^2
     int erfc_ref;          // use the reference's fitted erfc
+    int fast;              // short forms of the pair arithmetic (FP64 path)
+    int geom;              // GEOM_* (common.cuh)
     // optional output of the charge pass: the Coulomb list compacted to the
     // entries inside the cutoff (ddnbr, ddcnt) with the undamped
     // dipole-dipole radial factors (A1, B2) of each entry in FP32 (ddtab)
@@ -210,8 +215,9 @@ struct DirFlags {
     int* ddnbr;
     int* ddcnt;
 };
-void launch_ewald_dir(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz,
-                      const int* type, const double* q, const double* mu, CellP c, const NList& l,
+// rec: (fractional coordinates, type) of k_frac_rec; mrec: scratch for (dipole, charge).
+void launch_ewald_dir(cudaStream_t st, int n, const double4* rec, double4* mrec, const double* q, const double* mu,
+                      CellP c, const NList& l,
                       const PairConst* pc, DirFlags fl,
                       double* ef, double* efg, double* f, Partials& part, DevScalars* d, int g = 16);
 
@@ -352,11 +358,9 @@ void launch_ewald_dd32(cudaStream_t st, int n, const uint32_t* fx, const double*
 void launch_ewald_ddtab(cudaStream_t st, int n, const uint32_t* fx, const double* mu, CellP c, const int* nbr,
                         const int* cnt, int cap, const float2* tab, uint4* rec, double* ef, int g = 16);
 
-// The FP64 path's form: FP64 pair table, records of 8 doubles (fractional
-// coordinates, dipole).
-void launch_ewald_ddtab64(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz,
-                          const double* mu, CellP c, const int* nbr, const int* cnt, int cap, const double2* tab,
-                          double* rec, double* ef, int g = 16);
+// The FP64 path's form: FP64 pair table and k_ewald_dir's records.
+void launch_ewald_ddtab64(cudaStream_t st, int n, const double4* rec, double4* mrec, const double* mu, CellP c,
+                          const int* nbr, const int* cnt, int cap, const double2* tab, double* ef, int g = 16);
 
 // Solver vector kernels.
 

@@ -26,14 +26,18 @@ namespace mdff {
 //         energy, stress or block partials; the field is MODE 0's, bit for bit.
 // MODE 3: MODE 0 without the field gradient (every step but the EFG steps),
 //         so its registers are not sized for it.
-template <int G, int MODE>
-__global__ void __launch_bounds__(256, MODE == 2 ? 3 : 2) k_ewald_dir(int n, const double* __restrict__ sx, const double* __restrict__ sy,
-                                                   const double* __restrict__ sz, const int* __restrict__ type,
-                                                   const double* __restrict__ q, const double* __restrict__ mu,
-                                                   CellP c, const int* __restrict__ nbr, const int* __restrict__ cnt,
-                                                   int cap, const PairConst* __restrict__ pc, DirFlags fl,
-                                                   double* __restrict__ ef, double* __restrict__ efg,
-                                                   double* __restrict__ fo, double* part) {
+// FA: pair vectors, 1/d and d/3 in the short forms (FP64 path).  The mixed path
+// keeps the reference's expressions and their rounding: its 24-bit operands turn
+// a last-bit change of the dipoles into 1e-9 of the forces a step later.
+template <int G, int MODE, bool FA>
+__global__ void __launch_bounds__(256, MODE == 2 ? 3 : 2)
+    k_ewald_dir(int n, const double4* __restrict__ rec, const double4* __restrict__ mrec, CellP c,
+                const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
+                const PairConst* __restrict__ pc, DirFlags fl, double* __restrict__ ef, double* __restrict__ efg,
+                double* __restrict__ fo, double* part) {
+    __shared__ double s_erfcx[ERFCX_LEN];
+    for (int k = threadIdx.x; k < ERFCX_LEN; k += blockDim.x) s_erfcx[k] = (&c_erfcx[0][0])[k];
+    __syncthreads();
     const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
     const int sub = threadIdx.x & (G - 1);
     const bool active = gid < n;
@@ -44,11 +48,11 @@ __global__ void __launch_bounds__(256, MODE == 2 ? 3 : 2) k_ewald_dir(int n, con
     double E[3] = {0, 0, 0}, Gd[6] = {0, 0, 0, 0, 0, 0}, F[3] = {0, 0, 0};
     double u = 0.0, S[6] = {0, 0, 0, 0, 0, 0};
     if (active) {
-        const double si1 = sx[i], si2 = sy[i], si3 = sz[i];
-        const int ti = type[i];
-        const double qi = (MODE == 0 || MODE == 3) ? q[i] : 0.0;
-        const double mi0 = MODE == 2 ? 0.0 : mu[i], mi1 = MODE == 2 ? 0.0 : mu[n + i],
-                     mi2 = MODE == 2 ? 0.0 : mu[2 * n + i];
+        const double4 ri = ld_rec(rec + i);
+        const int ti = (int)__double_as_longlong(ri.w);
+        double4 mi = make_double4(0.0, 0.0, 0.0, 0.0);
+        if (MODE != 2) mi = ld_rec(mrec + i);
+        const double mi0 = mi.x, mi1 = mi.y, mi2 = mi.z, qi = mi.w;
         const int m = cnt[i];
         const int* row = nbr + (size_t)i * cap;
         // pair table: the lanes of the group compact the entries inside the
@@ -56,12 +60,23 @@ __global__ void __launch_bounds__(256, MODE == 2 ? 3 : 2) k_ewald_dir(int n, con
         const int g0 = (threadIdx.x & 31) & ~(G - 1);
         const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << g0);
         int cbase = 0, pos = 0;
+        // the record one neighbour ahead, the index two ahead: their latency under
+        // the arithmetic of this one (past the row's end: atom i itself)
+        int jn = sub < m ? row[sub] : i, jn2 = sub + G < m ? row[sub + G] : i;
+        double4 rn = ld_rec(rec + jn);
         for (int k0 = 0; k0 < m; k0 += G) {
-            const int k = k0 + sub;
+            const int k = k0 + sub, j = jn;
             const bool valid = k < m;
-            const int j = valid ? row[k] : i;
-            double rx = 0.0, ry = 0.0, rz = 0.0, d2 = 0.0;
-            if (valid) d2 = pairvec_exact(c, si1, si2, si3, sx[j], sy[j], sz[j], rx, ry, rz);
+            const double4 rj = rn;
+            jn = jn2;
+            rn = ld_rec(rec + jn);
+            jn2 = k + 2 * G < m ? row[k + 2 * G] : i;
+            double4 mj = make_double4(0.0, 0.0, 0.0, 0.0);
+            if (FA && MODE != 2) mj = ld_rec(mrec + j);
+            double rx, ry, rz;
+            const double d2 = FA ? pairvec(fl.geom, c, ri.x, ri.y, ri.z, rj.x, rj.y, rj.z, rx, ry, rz)
+                                 : pairvec_exact(c, ri.x, ri.y, ri.z, rj.x, rj.y, rj.z, rx, ry, rz);
+            const int tj = (int)__double_as_longlong(rj.w);
             const bool in = valid && d2 <= fl.cutsq;
             if (MODE != 1 && fl.ddnbr) {
                 const unsigned bal = (__ballot_sync(gmask, in) & gmask) >> g0;
@@ -70,10 +85,12 @@ __global__ void __launch_bounds__(256, MODE == 2 ? 3 : 2) k_ewald_dir(int n, con
                 cbase += __popc(bal);
             }
             if (!in) continue;
-            const double d = sqrt(d2);
-            const double dm1 = 1.0 / d, dm2 = dm1 * dm1, dm3 = dm1 * dm2, dm5 = dm3 * dm2, dm7 = dm5 * dm2;
+            const double dm1f = FA ? rsqrt(d2) : 0.0;
+            const double d = FA ? d2 * dm1f : sqrt(d2);
+            const double dm1 = FA ? dm1f : 1.0 / d;
+            const double dm2 = dm1 * dm1, dm3 = dm1 * dm2, dm5 = dm3 * dm2, dm7 = dm5 * dm2;
             const double ex2 = exp(-a2 * d2), expon = ex2 * rsqpi;
-            const double F0 = fl.erfc_ref ? erfc_fit(a * d) : erfc_ex2(a * d, ex2);
+            const double F0 = fl.erfc_ref ? erfc_fit(a * d) : erfc_ex2(a * d, ex2, s_erfcx);
             const double F1 = F0 + 2.0 * a * d * expon;
             const double F2 = F1 + c43a3 * d2 * d * expon;
             const double A1 = F1 * dm3;
@@ -82,19 +99,20 @@ __global__ void __launch_bounds__(256, MODE == 2 ? 3 : 2) k_ewald_dir(int n, con
             if (MODE != 1 && fl.ddtab64) fl.ddtab64[(size_t)i * cap + pos] = make_double2(A1, B2);
             if (MODE == 2) {
                 double gi = 0.0;
+                const PairConst& P = pc[ti * NT + tj];
                 if (fl.damp) {
-                    const PairConst& P = pc[ti * NT + type[j]];
                     if (P.ldamp && P.dc_i != 0.0) {   // c = 0 gives f = 1 exactly
                         double f1, gd;
                         tt_damp_d(P.db_i, P.dc_i, d, P.dk_i, f1, gd);
                         gi = 1.0 - f1;
                     }
                 }
-                const double s = q[j] * (F1 - gi) * dm3;
+                const double s = P.qj * (F1 - gi) * dm3;
                 E[0] += s * rx; E[1] += s * ry; E[2] += s * rz;
                 continue;
             }
-            const double mj0 = mu[j], mj1 = mu[n + j], mj2 = mu[2 * n + j];
+            if (!FA) mj = ld_rec(mrec + j);   // (here: loaded earlier, the compiler fuses other products)
+            const double mj0 = mj.x, mj1 = mj.y, mj2 = mj.z, qj = mj.w;
             const double rmj = rx * mj0 + ry * mj1 + rz * mj2;
             if (MODE == 1) {
                 E[0] += rx * rmj * B2 - mj0 * A1;
@@ -102,8 +120,6 @@ __global__ void __launch_bounds__(256, MODE == 2 ? 3 : 2) k_ewald_dir(int n, con
                 E[2] += rz * rmj * B2 - mj2 * A1;
                 continue;
             }
-            const int tj = type[j];
-            const double qj = q[j];
             const double rmi = rx * mi0 + ry * mi1 + rz * mi2;
             const double F3 = F2 + c815a5 * d2 * d2 * d * expon;
             const double C3 = 15.0 * F3 * dm7;
@@ -176,7 +192,8 @@ __global__ void __launch_bounds__(256, MODE == 2 ? 3 : 2) k_ewald_dir(int n, con
                 fi2 += rz * s - (qi * mj2 - qj * mi2) * A1;
                 if (ldamp) {
                     u += 0.5 * (-qi * gj * dm3 * rmj + qj * gi * dm3 * rmi);
-                    const double F2d = gi + (d / 3.0) * gdi, F2d2 = gj + (d / 3.0) * gdj;
+                    const double d3 = FA ? d * (1.0 / 3.0) : d / 3.0;
+                    const double F2d = gi + d3 * gdi, F2d2 = gj + d3 * gdj;
                     const double Bi = 3.0 * F2d * dm5, Ai = gi * dm3;     // T2d  (damping at i)
                     const double Bj = 3.0 * F2d2 * dm5, Aj = gj * dm3;    // T2d2 (damping at j)
                     // qj T2d mu_i - qi T2d2 mu_j
@@ -364,30 +381,25 @@ void launch_ewald_ddtab(cudaStream_t st, int n, const uint32_t* fx, const double
 #undef DDT
 }
 
+// (dipole, charge) of each atom for k_ewald_dir.
+__global__ void k_dir_records(int n, const double* __restrict__ mu, const double* __restrict__ q,
+                              double4* __restrict__ mrec) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) mrec[i] = make_double4(mu[i], mu[n + i], mu[2 * n + i], q ? q[i] : 0.0);
+}
+
 // FP64 path: the operator from an FP64 pair table, so that a solver iteration
 // evaluates no square root, exponential or erfc: 20 bytes of table and ~31 FP64
 // instructions per ordered pair, the image from the fractional coordinates
 // (d - rint(d); where the two images of a pair are equally far, T2 is the same
 // for both).  A1 and B2 are the charge pass's own doubles, so the operator is
 // MODE 1's to rounding and symmetric to the last bit.  Bound: the gathers of
-// 64-byte records through L2 (930 MB at 32 440 ions, rc 10 A) beside the table's
+// two 32-byte records a pair through L2 (930 MB at 32 440 ions, rc 10 A) beside the table's
 // 290 MB from HBM: 117 us per application against 279 of MODE 1, 14 against 33
 // at 3 000 ions; the charge pass takes 64 us longer once a step.
-__global__ void k_dd_records64(int n, const double* __restrict__ sx, const double* __restrict__ sy,
-                               const double* __restrict__ sz, const double* __restrict__ mu, double4* __restrict__ rec) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    rec[2 * i] = make_double4(sx[i], sy[i], sz[i], 0.0);
-    rec[2 * i + 1] = make_double4(mu[i], mu[n + i], mu[2 * n + i], 0.0);
-}
-
-// four doubles in one 256-bit load
-__device__ __forceinline__ void ld_rec64(const double4* __restrict__ p, double& a, double& b, double& c) {
-    asm("{\n\t.reg .f64 d;\n\tld.global.nc.v4.f64 {%0, %1, %2, d}, [%3];\n\t}" : "=d"(a), "=d"(b), "=d"(c) : "l"(p));
-}
-
 template <int G>
-__global__ void __launch_bounds__(256) k_ewald_ddtab64(int n, const double4* __restrict__ rec, CellP c,
+__global__ void __launch_bounds__(256) k_ewald_ddtab64(int n, const double4* __restrict__ rec,
+                                                       const double4* __restrict__ mrec, CellP c,
                                                        const int* __restrict__ nbr, const int* __restrict__ cnt,
                                                        int cap, const double2* __restrict__ tab,
                                                        double* __restrict__ ef) {
@@ -398,16 +410,14 @@ __global__ void __launch_bounds__(256) k_ewald_ddtab64(int n, const double4* __r
     constexpr double M = 6755399441055744.0;   // 1.5 2^52: (d + M) - M = rint(d)
     double E0 = 0.0, E1 = 0.0, E2 = 0.0;
     if (active) {
-        double s1, s2, s3;
-        ld_rec64(rec + 2 * (size_t)i, s1, s2, s3);
+        const double4 ri = ld_rec(rec + i);
         const int m = cnt[i];
         const int* row = nbr + (size_t)i * cap;
         const double2* trow = tab + (size_t)i * cap;
         auto term = [&](int j, double2 t) {
-            double p1, p2, p3, m0, m1, m2;
-            ld_rec64(rec + 2 * (size_t)j, p1, p2, p3);
-            ld_rec64(rec + 2 * (size_t)j + 1, m0, m1, m2);
-            double d0 = s1 - p1, d1 = s2 - p2, d2 = s3 - p3;
+            const double4 p = ld_rec(rec + j), mj = ld_rec(mrec + j);
+            const double m0 = mj.x, m1 = mj.y, m2 = mj.z;
+            double d0 = ri.x - p.x, d1 = ri.y - p.y, d2 = ri.z - p.z;
             d0 -= (d0 + M) - M;
             d1 -= (d1 + M) - M;
             d2 -= (d2 + M) - M;
@@ -434,13 +444,11 @@ __global__ void __launch_bounds__(256) k_ewald_ddtab64(int n, const double4* __r
     if (active && sub == 0) { ef[i] = E0; ef[n + i] = E1; ef[2 * n + i] = E2; }
 }
 
-void launch_ewald_ddtab64(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz,
-                          const double* mu, CellP c, const int* nbr, const int* cnt, int cap, const double2* tab,
-                          double* rec, double* ef, int g) {
-    double4* r = reinterpret_cast<double4*>(rec);
-    k_dd_records64<<<(n + 255) / 256, 256, 0, st>>>(n, sx, sy, sz, mu, r);
+void launch_ewald_ddtab64(cudaStream_t st, int n, const double4* rec, double4* mrec, const double* mu, CellP c,
+                          const int* nbr, const int* cnt, int cap, const double2* tab, double* ef, int g) {
+    k_dir_records<<<(n + 255) / 256, 256, 0, st>>>(n, mu, nullptr, mrec);
     const int blocks = (int)(((size_t)n * g + 255) / 256);
-#define DDT(G) k_ewald_ddtab64<G><<<blocks, 256, 0, st>>>(n, r, c, nbr, cnt, cap, tab, ef)
+#define DDT(G) k_ewald_ddtab64<G><<<blocks, 256, 0, st>>>(n, rec, mrec, c, nbr, cnt, cap, tab, ef)
     if (g == 8) DDT(8);
     else if (g == 32) DDT(32);
     else DDT(16);
@@ -459,21 +467,23 @@ void launch_ewald_dd32(cudaStream_t st, int n, const uint32_t* fx, const double*
 }
 
 // g: lanes per atom (8, 16 or 32; the autotuner's choice).
-void launch_ewald_dir(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz,
-                      const int* type, const double* q, const double* mu, CellP c, const NList& l,
-                      const PairConst* pc, DirFlags fl, double* ef, double* efg, double* f, Partials& part,
-                      DevScalars* d, int g) {
+void launch_ewald_dir(cudaStream_t st, int n, const double4* rec, double4* mrec, const double* q, const double* mu,
+                      CellP c, const NList& l, const PairConst* pc, DirFlags fl, double* ef, double* efg, double* f,
+                      Partials& part, DevScalars* d, int g) {
     const int threads = 256;
     const int blocks = (int)(((size_t)n * g + threads - 1) / threads);
-#define DIR(G, M, P) k_ewald_dir<G, M><<<blocks, threads, 0, st>>>(n, sx, sy, sz, type, q, mu, c, l.nbr, l.cnt, l.cap, \
-                                                                   pc, fl, ef, efg, f, P)
-    if (!q) {
-        if (g == 8) DIR(8, 1, nullptr);
-        else if (g == 32) DIR(32, 1, nullptr);
-        else DIR(16, 1, nullptr);
+    const bool charges_only = q && fl.qq && fl.field && !fl.qd && !fl.dd && !fl.efg && !fl.forces;
+    if (!charges_only) k_dir_records<<<(n + 255) / 256, 256, 0, st>>>(n, mu, q, mrec);
+#define DIRF(G, M, P, F) k_ewald_dir<G, M, F><<<blocks, threads, 0, st>>>(n, rec, mrec, c, l.nbr, l.cnt, l.cap, pc, fl, \
+                                                                         ef, efg, f, P)
+#define DIR(G, M, P) do { if (fl.fast) DIRF(G, M, P, true); else DIRF(G, M, P, false); } while (0)
+    if (!q) {   // (FP64 path)
+        if (g == 8) DIRF(8, 1, nullptr, true);
+        else if (g == 32) DIRF(32, 1, nullptr, true);
+        else DIRF(16, 1, nullptr, true);
         return;
     }
-    if (fl.qq && fl.field && !fl.qd && !fl.dd && !fl.efg && !fl.forces) {   // the charges' field alone
+    if (charges_only) {   // the charges' field alone
         if (g == 8) DIR(8, 2, nullptr);
         else if (g == 32) DIR(32, 2, nullptr);
         else DIR(16, 2, nullptr);
@@ -486,6 +496,7 @@ void launch_ewald_dir(cudaStream_t st, int n, const double* sx, const double* sy
     } else if (g == 8) DIR(8, 0, part.buf);
     else if (g == 32) DIR(32, 0, part.buf);
     else DIR(16, 0, part.buf);
+#undef DIRF
 #undef DIR
     launch_reduce_partials(st, part.buf, blocks, 8, d->dir, 0);
 }

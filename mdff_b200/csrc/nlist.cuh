@@ -27,6 +27,21 @@ void launch_frac(cudaStream_t st, int n, const double* x, const double* y, const
     k_frac<<<(n + 255) / 256, 256, 0, st>>>(n, x, y, z, c, sx, sy, sz);
 }
 
+// The same with the record (fractional coordinates, type as bits) that the pair
+// kernels gather.
+__global__ void k_frac_rec(int n, const double* __restrict__ x, const double* __restrict__ y,
+                           const double* __restrict__ z, const int* __restrict__ type, CellP c, double* sx, double* sy,
+                           double* sz, double4* rec) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double X = x[i], Y = y[i], Z = z[i];
+    const double a = __dadd_rn(__dadd_rn(__dmul_rn(X, c.B[0]), __dmul_rn(Y, c.B[3])), __dmul_rn(Z, c.B[6]));
+    const double b = __dadd_rn(__dadd_rn(__dmul_rn(X, c.B[1]), __dmul_rn(Y, c.B[4])), __dmul_rn(Z, c.B[7]));
+    const double d = __dadd_rn(__dadd_rn(__dmul_rn(X, c.B[2]), __dmul_rn(Y, c.B[5])), __dmul_rn(Z, c.B[8]));
+    sx[i] = a; sy[i] = b; sz[i] = d;
+    rec[i] = make_double4(a, b, d, __longlong_as_double((long long)type[i]));
+}
+
 // read_pos.f90:148-150: kardir, periodicbc (x - NINT(x)), dirkar, in place.
 __global__ void k_wrap(int n, double* x, double* y, double* z, CellP c) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -31,9 +31,110 @@ __device__ __forceinline__ double ipow_half(double x, double p) {
     return pow(x, h);
 }
 
+// Lennard-Jones 12-6 alone, or BMH / BMHFTD alone, without the other
+// potentials' registers and the exact expressions of k_pair: one rsqrt instead
+// of a square root and four divisions, one e^{-BD r} and one polynomial for both
+// damping orders, the virial from the stress sums.
+// KIND 0: Lennard-Jones 12-6, 1: BMH, 2: BMHFTD.
+template <int G, int KIND>
+__global__ void __launch_bounds__(256, KIND == 0 ? 4 : 3)
+    k_pair1(int n, const double4* __restrict__ rec, CellP c, const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
+            const PairConst* __restrict__ pc, PairFlags fl, double* fx, double* fy, double* fz, double* part) {
+    constexpr InvFact IF;
+    const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const int sub = threadIdx.x & (G - 1);
+    const bool active = gid < n;
+    const int i = active ? gid : 0;
+    double f0 = 0.0, f1 = 0.0, f2 = 0.0, ue = 0.0;
+    double tau[6] = {0, 0, 0, 0, 0, 0};
+    if (active) {
+        const double4 ri = ld_rec(rec + i);
+        const PairConst* Pi = pc + (int)__double_as_longlong(ri.w) * NT;
+        const int m = cnt[i];
+        const int* row = nbr + (size_t)i * cap;
+        // the record one neighbour ahead, the index two ahead: their latency under
+        // the arithmetic of this one
+        double4 rn = ld_rec(rec + (sub < m ? row[sub] : i));
+        int jn = sub + G < m ? row[sub + G] : i;
+        for (int k = sub; k < m; k += G) {
+            const double4 rj = rn;
+            rn = ld_rec(rec + jn);
+            jn = k + 2 * G < m ? row[k + 2 * G] : i;
+            double rx, ry, rz;
+            const double rsq = pairvec(fl.geom, c, ri.x, ri.y, ri.z, rj.x, rj.y, rj.z, rx, ry, rz);
+            const PairConst& P = Pi[(int)__double_as_longlong(rj.w)];
+            if (!(rsq < P.rcutsq)) continue;
+            double w;
+            if (KIND == 0) {
+                const double sr2 = P.sigsq / rsq, srp = sr2 * sr2 * sr2, srq = srp * srp;
+                double u = P.epsp * (P.plj * srq - P.qlj * srp);
+                if (fl.trunc == 1) u -= P.uc;
+                if (fl.trunc == 2) u += P.uc1 * rsq - P.uc2;
+                w = P.fc * (srq - srp) * sr2;
+                ue += u;
+            } else {
+                if (P.A == 0.0) continue;
+                const double dm1 = rsqrt(rsq), d = rsq * dm1, ir2 = dm1 * dm1;
+                const double erh = P.A * exp(-P.B * d);
+                double ir6 = ir2 * ir2 * ir2;
+                double ir8 = ir6 * ir2;
+                ir6 *= P.C;
+                ir8 *= P.D;
+                double w0 = P.B * erh, i68 = ir6 + ir8, i6d = 6.0 * ir6, i8d = 8.0 * ir8;
+                if (KIND == 2) {   // Tang-Toennies damping of orders 6 and 8 (tt_damp_d with c = 1)
+                    const double br = P.BD * d, e = exp(-br), e1 = e * P.BD;
+                    double term = 1.0, sum = 1.0;
+#pragma unroll
+                    for (int q = 1; q <= 6; ++q) {
+                        term *= br;
+                        sum = fma(term, IF.v[q], sum);
+                    }
+                    const double f6 = 1.0 - sum * e;
+                    w0 = fma(ir6, term * IF.v[6] * e1, w0);
+                    term *= br;
+                    sum = fma(term, IF.v[7], sum);
+                    term *= br;
+                    sum = fma(term, IF.v[8], sum);
+                    const double f8 = 1.0 - sum * e;
+                    w0 = fma(ir8, term * IF.v[8] * e1, w0);
+                    ir6 *= f6;
+                    ir8 *= f8;
+                    i68 = ir6 + ir8;
+                    i6d = 6.0 * ir6;
+                    i8d = 8.0 * ir8;
+                }
+                w = fma(-(i6d + i8d), dm1, w0) * dm1;
+                ue += erh - i68;
+            }
+            f0 = fma(w, rx, f0);
+            f1 = fma(w, ry, f1);
+            f2 = fma(w, rz, f2);
+            const double wx = w * rx, wy = w * ry;
+            tau[0] = fma(wx, rx, tau[0]);
+            tau[1] = fma(wy, ry, tau[1]);
+            tau[2] = fma(w * rz, rz, tau[2]);
+            tau[3] = fma(wx, ry, tau[3]);
+            tau[4] = fma(wx, rz, tau[4]);
+            tau[5] = fma(wy, rz, tau[5]);
+        }
+    }
+    f0 = group_sum<G>(f0);
+    f1 = group_sum<G>(f1);
+    f2 = group_sum<G>(f2);
+    if (active && sub == 0) {
+        fx[i] = f0;
+        fy[i] = f1;
+        fz[i] = f2;
+    }
+    // u and virial in the slots of the potential: u_lj vir_lj u_bmh vir_bmh u_mor vir_mor, then the stress
+    const double u = 0.5 * ue, vir = 0.5 * (tau[0] + tau[1] + tau[2]);
+    double v[12] = {KIND == 0 ? u : 0.0, KIND == 0 ? vir : 0.0, KIND == 0 ? 0.0 : u, KIND == 0 ? 0.0 : vir, 0.0, 0.0,
+                    0.5 * tau[0], 0.5 * tau[1], 0.5 * tau[2], 0.5 * tau[3], 0.5 * tau[4], 0.5 * tau[5]};
+    block_partials<12>(v, part);
+}
+
 template <int G>
-__global__ void __launch_bounds__(256) k_pair(int n, const double* __restrict__ sx, const double* __restrict__ sy,
-                                              const double* __restrict__ sz, const int* __restrict__ type, CellP c,
+__global__ void __launch_bounds__(256) k_pair(int n, const double4* __restrict__ rec, CellP c,
                                               const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
                                               const PairConst* __restrict__ pc, PairFlags fl, double* fx,
                                               double* fy, double* fz, double* part) {
@@ -45,15 +146,20 @@ __global__ void __launch_bounds__(256) k_pair(int n, const double* __restrict__ 
     double acc[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};   // u_lj vir_lj u_bmh vir_bmh u_mor vir_mor tau(6 -> 4 more below)
     double tau[6] = {0, 0, 0, 0, 0, 0};
     if (active) {
-        const double si1 = sx[i], si2 = sy[i], si3 = sz[i];
-        const int ti = type[i];
+        const double4 ri = ld_rec(rec + i);
+        const int ti = (int)__double_as_longlong(ri.w);
         const int m = cnt[i];
         const int* row = nbr + (size_t)i * cap;
+        // the record one neighbour ahead, the index two ahead
+        double4 rn = ld_rec(rec + (sub < m ? row[sub] : i));
+        int jn = sub + G < m ? row[sub + G] : i;
         for (int k = sub; k < m; k += G) {
-            const int j = row[k];
+            const double4 rj = rn;
+            rn = ld_rec(rec + jn);
+            jn = k + 2 * G < m ? row[k + 2 * G] : i;
             double rx, ry, rz;
-            const double rsq = pairvec_exact(c, si1, si2, si3, sx[j], sy[j], sz[j], rx, ry, rz);
-            const PairConst& P = pc[ti * NT + type[j]];
+            const double rsq = pairvec_exact(c, ri.x, ri.y, ri.z, rj.x, rj.y, rj.z, rx, ry, rz);
+            const PairConst& P = pc[ti * NT + (int)__double_as_longlong(rj.w)];
             if (!(rsq < P.rcutsq)) continue;
             double w = 0.0;
             if (fl.lj) {
@@ -122,13 +228,27 @@ __global__ void __launch_bounds__(256) k_pair(int n, const double* __restrict__ 
     block_partials<12>(v, part);
 }
 
-void launch_pair(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz, const int* type,
-                 CellP c, const NList& l, const PairConst* pc, PairFlags fl, double* fx, double* fy, double* fz,
+void launch_pair(cudaStream_t st, int n, const double4* rec, CellP c, const NList& l, const PairConst* pc, PairFlags fl, double* fx, double* fy, double* fz,
                  Partials& part, DevScalars* d) {
-    constexpr int G = 8;
     const int threads = 256;
-    const int blocks = (int)(((size_t)n * G + threads - 1) / threads);
-    k_pair<G><<<blocks, threads, 0, st>>>(n, sx, sy, sz, type, c, l.nbr, l.cnt, l.cap, pc, fl, fx, fy, fz, part.buf);
+    auto grid = [&](int g) { return (int)(((size_t)n * g + threads - 1) / threads); };
+    int blocks;
+    const bool bm = fl.bmh || fl.bmhftd;
+    const int kind = !fl.fast ? -1 : fl.lj && !bm && !fl.morse && fl.lj126 ? 0 : (bm && !fl.lj && !fl.morse ? (fl.bmhftd ? 2 : 1) : -1);
+#define PAIR1(G, K) k_pair1<G, K><<<blocks, threads, 0, st>>>(n, rec, c, l.nbr, l.cnt, l.cap, pc, fl, fx, fy, fz, part.buf)
+    // lanes per atom: a warp each until the atoms alone fill the SMs
+    const bool wide = n < 24000;
+    if (kind >= 0) {
+        blocks = grid(wide ? 32 : 8);
+        if (kind == 0) { if (wide) PAIR1(32, 0); else PAIR1(8, 0); }
+        else if (kind == 1) { if (wide) PAIR1(32, 1); else PAIR1(8, 1); }
+        else { if (wide) PAIR1(32, 2); else PAIR1(8, 2); }
+    } else {
+        constexpr int G = 8;
+        blocks = grid(G);
+        k_pair<G><<<blocks, threads, 0, st>>>(n, rec, c, l.nbr, l.cnt, l.cap, pc, fl, fx, fy, fz, part.buf);
+    }
+#undef PAIR1
     // u_lj vir_lj u_bmh vir_bmh u_mor vir_mor, then the stress sums
     launch_reduce_partials(st, part.buf, blocks, 12, d->nonb, 0);
 }
