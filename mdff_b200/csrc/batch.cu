@@ -40,11 +40,14 @@ using namespace mdff;
 
 namespace {
 
-constexpr int CHUNK = 128;     // atoms per reciprocal-space block
-constexpr int NZC = 8;         // nz values per thread in the structure factor
-constexpr int KT = 128;        // threads of the reciprocal-space blocks
-constexpr int CT = 16;         // k-columns staged per tile in the field kernel
-constexpr int KF_LPA = 4;      // lanes per atom in the field kernel (columns interleaved)
+constexpr int CHUNK = 128;     // atoms per structure-factor partial
+constexpr int KT = 64;         // threads of the structure factor's blocks
+constexpr int AB = 16;         // atoms per block of the phase tables
+constexpr int AP = AB + 1;     // values per table entry, padded: entries 272 bytes apart, no bank conflicts
+constexpr int FCH = 64;        // atoms per block of the field kernel
+constexpr int FT = 128;        // its threads
+constexpr int FCG = FT / 32;   // warps that share the atoms
+constexpr int FPP = 2 * FCG;   // column pairs per stage of coefficients
 constexpr int NTYB = 2;        // types supported by the gradient kernels
 
 
@@ -55,12 +58,17 @@ struct BCfg {
     int kmax[3];
     int ncol, nzl, nrect;
     int cs, ce;            // chunks [cs, ce)
+    int npair, coff;       // column pairs (nx, +-ny); first coefficient
+    int W, mc;             // phase-table entries per atom; m values per structure-factor item
+    long toff;             // first phase-table value
     int npol;
     double rc2, alpha, selfa, selfa2;
     double cF, cS;         // loss weights
 };
 
 struct BChunk { int c, a0, na; long poff; };
+
+struct BJob { int chunk, item0, nitem; };
 
 struct BPair {
     double A, B, C, D, BD;
@@ -73,6 +81,15 @@ struct BFlags {
     int bmh, bmhftd, morse, coul, erfc_ref;
     double cu, press;
 };
+
+__device__ __forceinline__ void cp_async16(void* smem, const void* g) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 
 inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 
@@ -687,146 +704,241 @@ __global__ void __launch_bounds__(256) k_b_grad_rows(int N, const int* __restric
 // reciprocal space
 // --------------------------------------------------------------------------
 
-// Pass 1: structure-factor partials of one chunk of atoms over its
-// configuration's k rectangle.  One thread per (k-column, run of NZC nz);
-// the phase e^{2 pi i n.s} of a run's first nz is the product X[nx] Y[ny]
-// Z0[run] of per-atom tables in shared memory (one sincospi per atom and
-// table entry, built by the block), then a rotation by e^{2 pi i s_z} per
-// further nz.  Amplitudes:
-//   MODE 0: q            MODE 1: i k.mu          MODE 2: q + i k.mu
-//   MODE 3: (k.R)(q + i k.mu)   (the adjoint structure factor)
-// Dynamic shared memory: CHUNK x phw_max double2 (the tables of the block's
-// atoms, one row per atom: X[0..kx], Y[-ky..ky], Z0[run]).
-template <int MODE>
-__global__ void __launch_bounds__(KT) k_b_sfac(const BChunk* __restrict__ chunks, const BCfg* __restrict__ cf,
-                                               const int* __restrict__ conv, int N, const double* __restrict__ sx,
-                                               const double* __restrict__ sy, const double* __restrict__ sz,
-                                               const double* __restrict__ q, const double* __restrict__ mu,
-                                               const double* __restrict__ R, double* __restrict__ part_re,
-                                               double* __restrict__ part_im) {
-    __shared__ double t_q[CHUNK], t_cz[CHUNK], t_sn[CHUNK];
-    __shared__ double t_u[3][CHUNK], t_v[3][CHUNK];
-    extern __shared__ double2 t_ph[];
-    const BChunk ch = chunks[blockIdx.x];
-    if (conv && conv[ch.c]) return;
-    const BCfg& C = cf[ch.c];
+// Phase tables of a batch, made once (its positions do not move): per 16-atom
+// block and entry AP values, e^{2 pi i n s_x} (n = 0..kx), e^{2 pi i n s_y}
+// (n = 0..ky), (cos, sin)(m t) and m times them (t = 2 pi s_z, m = 0..kz); atoms
+// past the configuration's end get 0.
+__global__ void k_b_tables(const int2* __restrict__ blks, const BCfg* __restrict__ cf, const double* __restrict__ sx,
+                           const double* __restrict__ sy, const double* __restrict__ sz, double2* __restrict__ tab) {
+    const int2 B = blks[blockIdx.x];
+    const BCfg& C = cf[B.x];
     const int kx = C.kmax[0], ky = C.kmax[1], kz = C.kmax[2];
-    const int nzch = (C.nzl + NZC - 1) / NZC;
-    const int W = (kx + 1) + (2 * ky + 1) + nzch;
-    for (int a = threadIdx.x; a < ch.na; a += blockDim.x) {
-        const int ia = ch.a0 + a;
-        double sn, cs;
-        sincospi(2.0 * sz[ia], &sn, &cs);
-        t_cz[a] = cs; t_sn[a] = sn;
-        t_q[a] = (MODE == 1) ? 0.0 : q[ia];
-        double m0 = 0, m1 = 0, m2 = 0, r0 = 0, r1 = 0, r2 = 0;
-        if (MODE != 0) { m0 = mu[ia]; m1 = mu[N + ia]; m2 = mu[2 * N + ia]; }
-        if (MODE == 3) { r0 = R[ia]; r1 = R[N + ia]; r2 = R[2 * N + ia]; }
-        // 2 pi b_d . v with b_d = column d of B: k.v = nx u0 + ny u1 + nz u2
-        for (int dcol = 0; dcol < 3; ++dcol) {
-            t_u[dcol][a] = 2.0 * PI * (C.cell.B[dcol] * m0 + C.cell.B[3 + dcol] * m1 + C.cell.B[6 + dcol] * m2);
-            t_v[dcol][a] = 2.0 * PI * (C.cell.B[dcol] * r0 + C.cell.B[3 + dcol] * r1 + C.cell.B[6 + dcol] * r2);
-        }
-    }
-    for (int t = threadIdx.x; t < ch.na * W; t += blockDim.x) {
-        const int a = t / W, e = t % W, ia = ch.a0 + a;
-        double arg;
-        if (e <= kx) arg = (double)e * sx[ia];
-        else if (e <= kx + 1 + 2 * ky) arg = (double)(e - (kx + 1) - ky) * sy[ia];
-        else arg = (double)(-kz + (e - (kx + 2 + 2 * ky)) * NZC) * sz[ia];
-        double sn, cs;
-        sincospi(2.0 * arg, &sn, &cs);
-        t_ph[t] = make_double2(cs, sn);
-    }
-    __syncthreads();
-    const int items = C.ncol * nzch;
-    double* pre = part_re + ch.poff;
-    double* pim = part_im + ch.poff;
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-        const int col = it / nzch, zc = it % nzch;
-        const int ix = col / (2 * ky + 1), iy = col % (2 * ky + 1);
-        const double nx = (double)ix;
-        const double ny = (double)(iy - ky);
-        const int m0 = zc * NZC;
-        const double nz0 = (double)(-kz + m0);
-        const int ex = ix, ey = kx + 1 + iy, ez = kx + 2 + 2 * ky + zc;
-        double are[NZC], aim[NZC];
-#pragma unroll
-        for (int m = 0; m < NZC; ++m) { are[m] = 0.0; aim[m] = 0.0; }
-        for (int a = 0; a < ch.na; ++a) {
-            const double2 X = t_ph[a * W + ex], Y = t_ph[a * W + ey], Z = t_ph[a * W + ez];
-            const double xr = fma(X.x, Y.x, -X.y * Y.y), xi = fma(X.x, Y.y, X.y * Y.x);
-            double er = fma(xr, Z.x, -xi * Z.y), ei = fma(xr, Z.y, xi * Z.x);
-            const double rc = t_cz[a], rs = t_sn[a];
-            const double qa = t_q[a];
-            double km = nx * t_u[0][a] + ny * t_u[1][a] + nz0 * t_u[2][a];
-            double kr = nx * t_v[0][a] + ny * t_v[1][a] + nz0 * t_v[2][a];
-            const double du = t_u[2][a], dv = t_v[2][a];
-#pragma unroll
-            for (int m = 0; m < NZC; ++m) {
-                double ar = qa, ai = km;
-                if (MODE == 3) { ar *= kr; ai *= kr; }
-                are[m] += ar * er - ai * ei;
-                aim[m] += ar * ei + ai * er;
-                const double t = er * rc - ei * rs;
-                ei = er * rs + ei * rc;
-                er = t;
-                km += du;
-                kr += dv;
+    double2* o = tab + C.toff + (size_t)(B.y / AB) * C.W * AP;
+    for (int t = threadIdx.x; t < C.W * AP; t += blockDim.x) {
+        const int e = t / AP, al = t % AP;
+        double2 v = make_double2(0.0, 0.0);
+        if (al < AB && B.y + al < C.n) {
+            const int i = C.off + B.y + al;
+            const int m = e - (kx + ky + 2);
+            if (e <= kx) phase((double)e, sx[i], v.x, v.y);
+            else if (m < 0) phase((double)(e - kx - 1), sy[i], v.x, v.y);
+            else if (m <= kz) phase((double)m, sz[i], v.x, v.y);
+            else {
+                const double f = (double)(m - kz - 1);
+                phase(f, sz[i], v.x, v.y);
+                v.x *= f;
+                v.y *= f;
             }
         }
-        const int mlim = min(NZC, C.nzl - m0);
-        for (int m = 0; m < mlim; ++m) {
-            pre[(size_t)col * C.nzl + m0 + m] = are[m];
-            pim[(size_t)col * C.nzl + m0 + m] = aim[m];
-        }
+        o[t] = v;
     }
 }
 
+// Amplitudes of the structure factors:
+//   MODE 0: q            MODE 1: i k.mu          MODE 2: q + i k.mu
+//   MODE 3: (k.R)(q + i k.mu)   (the adjoint structure factor)
+// each a polynomial in nz whose coefficients, times X Y, make up a real-basis sum:
+//   U = sum_a A0 cos(m t) - A1 m sin(m t) + A2 m^2 cos(m t),
+//   V = sum_a A0 sin(m t) + A1 m cos(m t) + A2 m^2 sin(m t),  S(nx, ny, +-m) = U +- i V,
+// with A0, A1, A2 complex and made once per (atom, column) for both signs of ny
+// and of nz: 16 FMAs an atom for four k-vectors (MODE 1, 2), where the complex
+// form takes 40 with the phase's advance along nz.
+template <int MODE, int MC>
+__device__ __forceinline__ void sfac_items(const BCfg& C, const BChunk& ch, int item0, int nitem,
+                                           const double2* __restrict__ tab, const double4* s_p, const double4* s_v,
+                                           double2* buf, double4* __restrict__ part) {
+    const int ky = C.kmax[1], kz = C.kmax[2];
+    const bool active = threadIdx.x < nitem;
+    const int it = item0 + (active ? threadIdx.x : 0);
+    const int pi = it % C.npair, m0 = it / C.npair * MC;
+    const int nx = pi / (ky + 1), ny = pi % (ky + 1);
+    const int ex = nx * AP, ey = (C.kmax[0] + 1 + ny) * AP, ez = (C.kmax[0] + ky + 2 + m0) * AP;
+    const int es = ez + (kz + 1) * AP;   // (m past kz: what lies there is computed with and not written)
+    const double fx = (double)nx, fy = (double)ny;
+    double U[MC][4], V[MC][4];
+#pragma unroll
+    for (int m = 0; m < MC; ++m)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) U[m][r] = V[m][r] = 0.0;
+    const int len = C.W * AP, nb = (ch.na + AB - 1) / AB;
+    const double2* src = tab + C.toff + (size_t)((ch.a0 - C.off) / AB) * len;
+    auto fetch = [&](int b) {
+        double2* d = buf + (b & 1) * len;
+        for (int t = threadIdx.x; t < len; t += KT) cp_async16(d + t, src + (size_t)b * len + t);
+        cp_async_commit();
+    };
+    fetch(0);
+    for (int b = 0; b < nb; ++b) {
+        if (b + 1 < nb) fetch(b + 1);
+        else cp_async_commit();
+        cp_async_wait<1>();
+        __syncthreads();
+        const double2* row = buf + (b & 1) * len;
+        const int na = min(AB, ch.na - b * AB);
+        for (int a = 0; a < na; ++a) {
+            const double2 X = row[ex + a], Y = row[ey + a];
+            const double4 P = s_p[b * AB + a];
+            const double yy = X.y * Y.y, xy = X.x * Y.y;
+            const double pr = fma(X.x, Y.x, -yy), qr = fma(X.x, Y.x, yy);      // X Y, X conj(Y)
+            const double pm = fma(X.y, Y.x, xy), qm = fma(X.y, Y.x, -xy);
+            double A0[4], A1[4], A2[4];
+            if (MODE == 0) {
+                A0[0] = P.x * pr; A0[1] = P.x * pm; A0[2] = P.x * qr; A0[3] = P.x * qm;
+            } else {
+                const double t1 = fx * P.y, kp = fma(fy, P.z, t1), km = fma(-fy, P.z, t1);
+                double arp = P.x, aip = kp, arm = P.x, aim = km;               // amplitude at nz = 0
+                if (MODE == 3) {
+                    const double4 R = s_v[b * AB + a];
+                    const double t2 = fx * R.x, rp = fma(fy, R.y, t2), rm = fma(-fy, R.y, t2);
+                    arp *= rp; aip *= rp; arm *= rm; aim *= rm;
+                    // the nz coefficient O: A1 = -i O; the nz^2 one: i r3 m3
+                    const double o0 = R.z * P.x, op = fma(rp, P.w, R.z * kp), om = fma(rm, P.w, R.z * km);
+                    A1[0] = fma(pr, op, pm * o0); A1[1] = fma(pm, op, -pr * o0);
+                    A1[2] = fma(qr, om, qm * o0); A1[3] = fma(qm, om, -qr * o0);
+                    const double o2 = R.z * P.w;
+                    A2[0] = -pm * o2; A2[1] = pr * o2; A2[2] = -qm * o2; A2[3] = qr * o2;
+                } else {
+                    A1[0] = pr * P.w; A1[1] = pm * P.w; A1[2] = qr * P.w; A1[3] = qm * P.w;
+                }
+                if (MODE == 1) {
+                    A0[0] = -pm * kp; A0[1] = pr * kp; A0[2] = -qm * km; A0[3] = qr * km;
+                } else {
+                    A0[0] = fma(pr, arp, -pm * aip); A0[1] = fma(pr, aip, pm * arp);
+                    A0[2] = fma(qr, arm, -qm * aim); A0[3] = fma(qr, aim, qm * arm);
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < MC; ++m) {
+                const double2 cs = row[ez + m * AP + a];
+                double2 ms;
+                if (MODE != 0) ms = row[es + m * AP + a];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    U[m][r] = fma(A0[r], cs.x, U[m][r]);
+                    V[m][r] = fma(A0[r], cs.y, V[m][r]);
+                    if (MODE != 0) {
+                        U[m][r] = fma(-A1[r], ms.y, U[m][r]);
+                        V[m][r] = fma(A1[r], ms.x, V[m][r]);
+                    }
+                    if (MODE == 3) {
+                        const double t = A2[r] * (double)(m0 + m);
+                        U[m][r] = fma(t, ms.x, U[m][r]);
+                        V[m][r] = fma(t, ms.y, V[m][r]);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (!active) return;
+    double4* o = part + ch.poff + (size_t)2 * pi * (kz + 1) + m0;
+#pragma unroll
+    for (int m = 0; m < MC; ++m) {
+        if (m0 + m > kz) break;
+        o[m] = make_double4(U[m][0] - V[m][1], U[m][1] + V[m][0], U[m][0] + V[m][1], U[m][1] - V[m][0]);
+        o[m + kz + 1] = make_double4(U[m][2] - V[m][3], U[m][3] + V[m][2], U[m][2] + V[m][3], U[m][3] - V[m][2]);
+    }
+}
+
+// Pass 1: structure-factor partials of one chunk of atoms.  A thread takes one
+// column pair (nx, +-ny) and C.mc values of m = |nz|, a block up to KT of these
+// items; the chunk's tables come through shared memory in 16-atom stages, two in
+// flight.  part: per chunk [pair][sign of ny][m] S at +m and at -m.
+// Bound by the FP64 pipe (about half of its rate: 16 FMAs and two 16-byte shared
+// reads, two clocks each, per m).  64 configurations of 200-2000 ions (69 642), kmax 7-13,
+// MODE 1: 133 us against 362 for complex phases advanced along nz (an eighth of a
+// column's nz a thread, tables made by every block); MODE 0 81, MODE 2 137.  128 threads a
+// block: 153 (64 and their barrier leave more blocks to a scheduler); 32: 138;
+// 32-atom stages: 144.  m values per item: 4, 5 or 6, whichever wastes least
+// (7: registers spill, 159).
 template <int MODE>
-__global__ void k_b_sfac_reduce(int nrect_tot, const int* __restrict__ rcfg, const BCfg* __restrict__ cf,
+__global__ void __launch_bounds__(KT, 6)
+    k_b_sfac(const BJob* __restrict__ jobs, const BChunk* __restrict__ chunks, const BCfg* __restrict__ cf,
+             const int* __restrict__ conv, int N, const double2* __restrict__ tab, const double* __restrict__ q,
+             const double* __restrict__ mu, const double* __restrict__ R, double4* __restrict__ part) {
+    __shared__ double4 s_p[CHUNK];
+    __shared__ double4 s_v[MODE == 3 ? CHUNK : 1];
+    extern __shared__ __align__(16) double2 buf[];
+    const BJob job = jobs[blockIdx.x];
+    const BChunk ch = chunks[job.chunk];
+    if (conv && conv[ch.c]) return;
+    const BCfg& C = cf[ch.c];
+    for (int a = threadIdx.x; a < ch.na; a += KT) {
+        const int ia = ch.a0 + a;
+        // 2 pi b_d . v with b_d = column d of B: k.v = nx u0 + ny u1 + nz u2
+        auto dual = [&](const double* v, int d) {
+            return 2.0 * PI * (C.cell.B[d] * v[ia] + C.cell.B[3 + d] * v[N + ia] + C.cell.B[6 + d] * v[2 * N + ia]);
+        };
+        const double qa = MODE == 1 ? 0.0 : q[ia];
+        s_p[a] = MODE == 0 ? make_double4(qa, 0.0, 0.0, 0.0) : make_double4(qa, dual(mu, 0), dual(mu, 1), dual(mu, 2));
+        if (MODE == 3) s_v[a] = make_double4(dual(R, 0), dual(R, 1), dual(R, 2), 0.0);
+    }
+    switch (C.mc) {   // (the first stage's barrier covers s_p)
+        case 4: sfac_items<MODE, 4>(C, ch, job.item0, job.nitem, tab, s_p, s_v, buf, part); break;
+        case 5: sfac_items<MODE, 5>(C, ch, job.item0, job.nitem, tab, s_p, s_v, buf, part); break;
+        default: sfac_items<MODE, 6>(C, ch, job.item0, job.nitem, tab, s_p, s_v, buf, part); break;
+    }
+}
+
+// Sums over chunks in order, then the coefficients C_k, stored per (column pair,
+// sign of ny, m) as what the field needs of C(+m) and C(-m):
+// (C+ + C-, i (C+ - C-)).  ccfg: configuration of each coefficient.
+template <int MODE>
+__global__ void k_b_sfac_reduce(int ncoef_tot, const int* __restrict__ ccfg, const BCfg* __restrict__ cf,
                                 const BChunk* __restrict__ chunks, const int* __restrict__ conv,
-                                const double* __restrict__ part_re, const double* __restrict__ part_im,
-                                const double* __restrict__ Ak, const double* __restrict__ kcoe,
-                                const double* __restrict__ Sres, BFlags fl, double* rho_re, double* rho_im,
-                                double* C_re, double* C_im) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nrect_tot) return;
-    const int c = rcfg[e];
+                                const double4* __restrict__ part, const double* __restrict__ Ak,
+                                const double* __restrict__ kcoe, const double* __restrict__ Sres, BFlags fl,
+                                double* rho_re, double* rho_im, double4* __restrict__ coef) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= ncoef_tot) return;
+    const int c = ccfg[g];
     if (conv && conv[c]) return;
     const BCfg& Cf = cf[c];
-    const int l = e - Cf.roff;
-    double sr = 0.0, si = 0.0;
-    for (int ch = Cf.cs; ch < Cf.ce; ++ch) {
-        const long o = chunks[ch].poff + l;
-        sr += part_re[o];
-        si += part_im[o];
-    }
-    const double A = Ak[e];
-    if (MODE == 1) { rho_re[e] = sr; rho_im[e] = si; }
-    if (MODE != 2) {
-        C_re[e] = A * sr;
-        C_im[e] = -A * si;
+    const int l = g - Cf.coff, ky = Cf.kmax[1], kz = Cf.kmax[2];
+    const int m = l % (kz + 1), sg = (l / (kz + 1)) & 1, pi = l / (2 * (kz + 1));
+    const int ix = pi / (ky + 1), iy = pi % (ky + 1);
+    if (sg && iy == 0) {   // the same column again
+        coef[g] = make_double4(0.0, 0.0, 0.0, 0.0);
         return;
     }
-    const int nzl = Cf.nzl, ky = Cf.kmax[1], kz = Cf.kmax[2];
-    const int col = l / nzl;
-    const double nx = (double)(col / (2 * ky + 1)), ny = (double)(col % (2 * ky + 1) - ky);
-    const double nz = (double)(l % nzl - kz);
+    double sr[2] = {0.0, 0.0}, si[2] = {0.0, 0.0};   // S at +m, -m
+#pragma unroll 4
+    for (int ch = Cf.cs; ch < Cf.ce; ++ch) {
+        const double4 v = part[chunks[ch].poff + l];
+        sr[0] += v.x; si[0] += v.y;
+        sr[1] += v.z; si[1] += v.w;
+    }
+    const double nx = (double)ix, ny = (double)(sg ? -iy : iy);
+    const int e0 = Cf.roff + (ix * (2 * ky + 1) + ky + (sg ? -iy : iy)) * Cf.nzl + kz;
     const double* B = Cf.cell.B;
-    const double k0 = 2.0 * PI * (nx * B[0] + ny * B[1] + nz * B[2]);
-    const double k1 = 2.0 * PI * (nx * B[3] + ny * B[4] + nz * B[5]);
-    const double k2 = 2.0 * PI * (nx * B[6] + ny * B[7] + nz * B[8]);
-    const double* S = Sres + c * 9;
-    const double kSk = k0 * (S[0] * k0 + S[1] * k1 + S[2] * k2) + k1 * (S[3] * k0 + S[4] * k1 + S[5] * k2) +
-                       k2 * (S[6] * k0 + S[7] * k1 + S[8] * k2);
-    const double sk = (S[0] + S[4] + S[8]) - kcoe[e] * kSk;
-    const double tpi_V = 2.0 * PI / Cf.cell.omega;
-    const double a1 = -2.0 * fl.cu * 2.0 * tpi_V;           // -2 cu fpi_V
-    const double a2 = -2.0 * fl.cu / fl.press * 2.0 * tpi_V / Cf.cell.omega * sk;   // -2 c_s s_k
-    // a1 i conj(sigma) = a1 (si + i sr);  a2 conj(rho)
-    C_re[e] = A * (a1 * si + a2 * rho_re[e]);
-    C_im[e] = A * (a1 * sr - a2 * rho_im[e]);
+    double cr[2], ci[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int e = e0 + (u ? -m : m);
+        const double A = Ak[e];
+        if (MODE == 1) { rho_re[e] = sr[u]; rho_im[e] = si[u]; }
+        if (MODE != 2) {
+            cr[u] = A * sr[u];
+            ci[u] = -A * si[u];
+        } else {
+            const double nz = (double)(u ? -m : m);
+            const double k0 = 2.0 * PI * (nx * B[0] + ny * B[1] + nz * B[2]);
+            const double k1 = 2.0 * PI * (nx * B[3] + ny * B[4] + nz * B[5]);
+            const double k2 = 2.0 * PI * (nx * B[6] + ny * B[7] + nz * B[8]);
+            const double* S = Sres + c * 9;
+            const double kSk = k0 * (S[0] * k0 + S[1] * k1 + S[2] * k2) + k1 * (S[3] * k0 + S[4] * k1 + S[5] * k2) +
+                               k2 * (S[6] * k0 + S[7] * k1 + S[8] * k2);
+            const double sk = (S[0] + S[4] + S[8]) - kcoe[e] * kSk;
+            const double tpi_V = 2.0 * PI / Cf.cell.omega;
+            const double a1 = -2.0 * fl.cu * 2.0 * tpi_V;           // -2 cu fpi_V
+            const double a2 = -2.0 * fl.cu / fl.press * 2.0 * tpi_V / Cf.cell.omega * sk;   // -2 c_s s_k
+            // a1 i conj(sigma) = a1 (si + i sr);  a2 conj(rho)
+            cr[u] = A * (a1 * si[u] + a2 * rho_re[e]);
+            ci[u] = A * (a1 * sr[u] - a2 * rho_im[e]);
+        }
+    }
+    coef[g] = m == 0 ? make_double4(cr[0], ci[0], 0.0, 0.0)
+                     : make_double4(cr[0] + cr[1], ci[0] + ci[1], ci[1] - ci[0], cr[0] - cr[1]);
 }
 
 // Energy and stress sums of the final structure factor per configuration:
@@ -877,86 +989,180 @@ __global__ void k_b_rec_sums(const BCfg* __restrict__ cf, const double* __restri
     }
 }
 
-// Pass 2: per atom of the chunk, V = scale sum_k k Im(C_k e^{ik.r}) and, with
-// GRAD, G = scale sum_k k k^T Re(C_k e^{ik.r}) (xx yy zz xy xz yz).  scale is
-// 2 fpi_V of the configuration when SCALE_FPI, else 1.  V is written, or added
-// with ADD.
+// Pass 2: per atom, V = scale sum_k k Im(C_k e^{ik.r}) and, with GRAD,
+// G = scale sum_k k k^T Re(C_k e^{ik.r}) (xx yy zz xy xz yz).  scale is 2 fpi_V
+// of the configuration when SCALE_FPI, else 1.  V is written, or added with ADD.
+//
+// Per column the moments F_j = sum_m m^j (cos(m t), sin(m t)) . coefficients,
+// real basis (8 FMAs for the two signs of nz, 12 with GRAD, where the complex
+// form takes 22 or 40), then one product with X Y; the wave vectors come in
+// after the sum over columns.  A block takes 64 atoms, two a lane, and each of
+// its warps every fourth pair of column pairs: four columns (two with GRAD) of two
+// atoms at once, so that a coefficient read from shared memory (a uniform
+// 16-byte read takes two of its clocks) feeds eight products.  Coefficients come
+// in 16-column stages, two in flight.
+// Bound by shared-memory and L1 reads beside the FP64 pipe.  The 64 configurations above: 131 us
+// (205 with the gradient) against 302 for complex phases, four lanes an atom; one
+// atom a lane 154, 64 threads a block 161, eight columns a warp 137.
 template <int GRAD, int ADD, int SCALE_FPI>
-__global__ void __launch_bounds__(KT * KF_LPA) k_b_kfield(const BChunk* __restrict__ chunks, const BCfg* __restrict__ cf,
-                                                 const int* __restrict__ conv, int N, const double* __restrict__ sx,
-                                                 const double* __restrict__ sy, const double* __restrict__ sz,
-                                                 const double* __restrict__ C_re, const double* __restrict__ C_im,
-                                                 double* __restrict__ V, double* __restrict__ Gout) {
-    extern __shared__ double smem[];
-    const BChunk ch = chunks[blockIdx.x];
-    if (conv && conv[ch.c]) return;
-    const BCfg& C = cf[ch.c];
-    const int nzl = C.nzl, ky = C.kmax[1], kz = C.kmax[2];
-    double* t_re = smem;
-    double* t_im = smem + CT * nzl;
-    const int t = threadIdx.x / KF_LPA, sub = threadIdx.x % KF_LPA;   // atom, lane among the atom's
-    const bool active = t < ch.na;
-    const int ia = ch.a0 + (active ? t : 0);
-    const double s1 = sx[ia], s2 = sy[ia], s3 = sz[ia];
-    double rs, rc;
-    sincospi(2.0 * s3, &rs, &rc);
-    const double* B = C.cell.B;
-    const double bz0 = 2.0 * PI * B[2], bz1 = 2.0 * PI * B[5], bz2 = 2.0 * PI * B[8];
-    double E0 = 0, E1 = 0, E2 = 0, G[6] = {0, 0, 0, 0, 0, 0};
-    for (int c0 = 0; c0 < C.ncol; c0 += CT) {
-        const int nc = min(CT, C.ncol - c0);
+__global__ void __launch_bounds__(FT, 3)
+    k_b_kfield(const int2* __restrict__ jobs, const BCfg* __restrict__ cf, const int* __restrict__ conv, int N,
+               const double2* __restrict__ tab, const double4* __restrict__ coef, double* __restrict__ V,
+               double* __restrict__ Gout) {
+    constexpr int NS = GRAD ? 9 : 3;
+    constexpr int NP = GRAD ? 1 : 2, NU = 2 * NP;   // column pairs, columns at once
+    extern __shared__ __align__(16) double2 buf[];
+    __shared__ double red[FCG - 1][NS][FCH];
+    const int2 job = jobs[blockIdx.x];
+    if (conv && conv[job.x]) return;
+    const BCfg& C = cf[job.x];
+    const int kx = C.kmax[0], ky = C.kmax[1], nm = C.kmax[2] + 1;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double2* row[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int a = min(job.y + 32 * h + lane, C.n - 1);
+        row[h] = tab + C.toff + (size_t)(a / AB) * C.W * AP + a % AB;
+    }
+    const int ez = (kx + ky + 2) * AP;
+    const double2* src = reinterpret_cast<const double2*>(coef + C.coff);
+    const int plen = 4 * nm, stage = FPP * plen, npass = (C.npair + FPP - 1) / FPP;   // double2 per pair, per stage
+    auto fetch = [&](int p) {
+        const int len = min(FPP, C.npair - p * FPP) * plen;
+        double2* d = buf + (p & 1) * stage;
+        for (int t = threadIdx.x; t < len; t += FT) cp_async16(d + t, src + (size_t)p * stage + t);
+        cp_async_commit();
+    };
+    double S[2][NS];
+#pragma unroll
+    for (int k = 0; k < NS; ++k) S[0][k] = S[1][k] = 0.0;
+    fetch(0);
+    for (int p = 0; p < npass; ++p) {
+        if (p + 1 < npass) fetch(p + 1);
+        else cp_async_commit();
+        cp_async_wait<1>();
         __syncthreads();
-        for (int k = threadIdx.x; k < nc * nzl; k += blockDim.x) {
-            const int e = C.roff + c0 * nzl + k;
-            t_re[k] = C_re[e];
-            t_im[k] = C_im[e];
+#pragma unroll 1
+        for (int pp = 0; pp < 2; pp += NP) {
+            const int pi = p * FPP + 2 * warp + pp;
+            if (pi >= C.npair) break;
+            const double2* cb = buf + (p & 1) * stage + (2 * warp + pp) * plen;
+            const int off1 = NP == 2 && pi + 1 < C.npair ? plen : 0;   // an odd last pair: computed twice, added once
+            double F0r[2][NU], F0i[2][NU], F1r[2][NU], F1i[2][NU], F2r[2][NU], F2i[2][NU];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int u = 0; u < NU; ++u) F0r[h][u] = F0i[h][u] = F1r[h][u] = F1i[h][u] = F2r[h][u] = F2i[h][u] = 0.0;
+            double mf = 0.0;
+#pragma unroll 2
+            for (int m = 0; m < nm; ++m, mf += 1.0) {
+                double2 z[2];
+                double mc[2], ms[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    z[h] = row[h][ez + m * AP];
+                    mc[h] = mf * z[h].x;
+                    ms[h] = mf * z[h].y;
+                }
+#pragma unroll
+                for (int u = 0; u < NU; ++u) {
+                    const double2* k = cb + (u >> 1) * off1 + ((u & 1) * nm + m) * 2;
+                    const double2 P = k[0], Q = k[1];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        F0r[h][u] = fma(z[h].x, P.x, F0r[h][u]);
+                        F0i[h][u] = fma(z[h].x, P.y, F0i[h][u]);
+                        F1r[h][u] = fma(mc[h], Q.y, F1r[h][u]);
+                        F1i[h][u] = fma(ms[h], P.x, F1i[h][u]);
+                        F0r[h][u] = fma(z[h].y, Q.x, F0r[h][u]);
+                        F0i[h][u] = fma(z[h].y, Q.y, F0i[h][u]);
+                        F1r[h][u] = fma(-ms[h], P.y, F1r[h][u]);
+                        F1i[h][u] = fma(-mc[h], Q.x, F1i[h][u]);
+                        if (GRAD) {
+                            const double m2c = mf * mc[h], m2s = mf * ms[h];
+                            F2r[h][u] = fma(m2c, P.x, F2r[h][u]);
+                            F2i[h][u] = fma(m2c, P.y, F2i[h][u]);
+                            F2r[h][u] = fma(m2s, Q.x, F2r[h][u]);
+                            F2i[h][u] = fma(m2s, Q.y, F2i[h][u]);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int v = 0; v < NP; ++v) {
+                if (v == 1 && pi + 1 >= C.npair) break;
+                const int ix = (pi + v) / (ky + 1), iy = (pi + v) % (ky + 1);
+                const double nx = (double)ix;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const double2 X = row[h][ix * AP], Y = row[h][(kx + 1 + iy) * AP];
+                    const double yy = X.y * Y.y, xy = X.x * Y.y;
+#pragma unroll
+                    for (int sg = 0; sg < 2; ++sg) {
+                        const int u = 2 * v + sg;
+                        const double ny = sg ? -(double)iy : (double)iy;
+                        const double ur = fma(X.x, Y.x, sg ? yy : -yy), ui = fma(X.y, Y.x, sg ? -xy : xy);
+                        const double i0 = fma(ur, F0i[h][u], ui * F0r[h][u]), i1 = fma(ur, F1i[h][u], ui * F1r[h][u]);
+                        S[h][0] = fma(nx, i0, S[h][0]);
+                        S[h][1] = fma(ny, i0, S[h][1]);
+                        S[h][2] += i1;
+                        if (GRAD) {
+                            const double r0 = fma(ur, F0r[h][u], -ui * F0i[h][u]), r1 = fma(ur, F1r[h][u], -ui * F1i[h][u]);
+                            const double r2 = fma(ur, F2r[h][u], -ui * F2i[h][u]);
+                            const double xr = nx * r0, yr = ny * r0;
+                            double* Q = S[h] + NS - 6;   // nx nx, ny ny, nz nz, nx ny, nx nz, ny nz
+                            Q[0] = fma(nx, xr, Q[0]);
+                            Q[1] = fma(ny, yr, Q[1]);
+                            Q[2] += r2;
+                            Q[3] = fma(ny, xr, Q[3]);
+                            Q[4] = fma(nx, r1, Q[4]);
+                            Q[5] = fma(ny, r1, Q[5]);
+                        }
+                    }
+                }
+            }
         }
         __syncthreads();
-        if (!active) continue;
-        for (int cc = sub; cc < nc; cc += KF_LPA) {
-            const int col = c0 + cc;
-            const double nx = (double)(col / (2 * ky + 1)), ny = (double)(col % (2 * ky + 1) - ky);
-            double sn, cs;
-            sincospi(2.0 * (nx * s1 + ny * s2 - (double)kz * s3), &sn, &cs);
-            double er = cs, ei = sn;
-            double k0 = 2.0 * PI * (nx * B[0] + ny * B[1]) - (double)kz * bz0;
-            double k1 = 2.0 * PI * (nx * B[3] + ny * B[4]) - (double)kz * bz1;
-            double k2 = 2.0 * PI * (nx * B[6] + ny * B[7]) - (double)kz * bz2;
-            const double* cr = t_re + cc * nzl;
-            const double* ci = t_im + cc * nzl;
-            for (int m = 0; m < nzl; ++m) {
-                const double zr = cr[m] * er - ci[m] * ei;
-                const double zi = cr[m] * ei + ci[m] * er;
-                E0 += k0 * zi; E1 += k1 * zi; E2 += k2 * zi;
-                if (GRAD) {
-                    G[0] += k0 * k0 * zr; G[1] += k1 * k1 * zr; G[2] += k2 * k2 * zr;
-                    G[3] += k0 * k1 * zr; G[4] += k0 * k2 * zr; G[5] += k1 * k2 * zr;
-                }
-                const double tt = er * rc - ei * rs;
-                ei = er * rs + ei * rc;
-                er = tt;
-                k0 += bz0; k1 += bz1; k2 += bz2;
+    }
+    if (warp > 0)
+#pragma unroll
+        for (int k = 0; k < NS; ++k) {
+            red[warp - 1][k][lane] = S[0][k];
+            red[warp - 1][k][32 + lane] = S[1][k];
+        }
+    __syncthreads();
+    if (warp > 0) return;
+    const double* B = C.cell.B;
+    const double sc = (SCALE_FPI ? 2.0 * (4.0 * PI / C.cell.omega) : 1.0) * 2.0 * PI;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int al = 32 * h + lane;
+        if (job.y + al >= C.n) break;
+        const int ia = C.off + job.y + al;
+#pragma unroll
+        for (int k = 0; k < NS; ++k)
+#pragma unroll
+            for (int w = 0; w < FCG - 1; ++w) S[h][k] += red[w][k][al];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double v = sc * (B[3 * d] * S[h][0] + B[3 * d + 1] * S[h][1] + B[3 * d + 2] * S[h][2]);
+            if (ADD) V[(size_t)d * N + ia] += v;
+            else V[(size_t)d * N + ia] = v;
+        }
+        if (GRAD) {
+            const double* Q = S[h] + NS - 6;
+            const int pd[6] = {0, 1, 2, 0, 0, 1}, pe[6] = {0, 1, 2, 1, 2, 2};
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                const double* b = B + 3 * pd[k];
+                const double* e = B + 3 * pe[k];
+                const double v = b[0] * (Q[0] * e[0] + Q[3] * e[1] + Q[4] * e[2]) +
+                                 b[1] * (Q[3] * e[0] + Q[1] * e[1] + Q[5] * e[2]) +
+                                 b[2] * (Q[4] * e[0] + Q[5] * e[1] + Q[2] * e[2]);
+                Gout[(size_t)k * N + ia] = sc * 2.0 * PI * v;
             }
         }
     }
-    // the atom's lanes are adjacent: sum them by a fixed xor tree
-#pragma unroll
-    for (int o = 1; o < KF_LPA; o <<= 1) {
-        E0 += __shfl_xor_sync(0xffffffffu, E0, o);
-        E1 += __shfl_xor_sync(0xffffffffu, E1, o);
-        E2 += __shfl_xor_sync(0xffffffffu, E2, o);
-        if (GRAD)
-            for (int k = 0; k < 6; ++k) G[k] += __shfl_xor_sync(0xffffffffu, G[k], o);
-    }
-    if (!active || sub != 0) return;
-    const double sc = SCALE_FPI ? 2.0 * (4.0 * PI / C.cell.omega) : 1.0;
-    if (ADD) {
-        V[ia] += sc * E0; V[N + ia] += sc * E1; V[2 * N + ia] += sc * E2;
-    } else {
-        V[ia] = sc * E0; V[N + ia] = sc * E1; V[2 * N + ia] = sc * E2;
-    }
-    if (GRAD)
-        for (int k = 0; k < 6; ++k) Gout[(size_t)k * N + ia] = sc * G[k];
 }
 
 // --------------------------------------------------------------------------
@@ -1263,9 +1469,14 @@ struct mdff_batch {
     BChunk* chunk = nullptr;
     int nchunk = 0;
     long part_len = 0;
-    int nrect_tot = 0, nzl_max = 1;
-    int phw_max = 1;       // widest per-atom phase table of the structure factor (X, Y, Z0 entries)
-    int* rcfg = nullptr;
+    int nrect_tot = 0, ncoef_tot = 0;
+    std::vector<BJob> hjob;      // structure factor: (chunk, items), the longest first
+    std::vector<int2> hfjob;     // field: (configuration, first atom), the longest first
+    BJob* job = nullptr;
+    int2* fjob = nullptr;
+    size_t sm_sfac = 0, sm_field = 0;
+    int* ccfg = nullptr;
+    double2* tab = nullptr;      // phase tables (k_b_tables)
     int* cfg_of = nullptr;
     int* type = nullptr;
     double *x = nullptr, *y = nullptr, *z = nullptr, *sx = nullptr, *sy = nullptr, *sz = nullptr;
@@ -1274,8 +1485,8 @@ struct mdff_batch {
     int* overflow = nullptr;
     BPair* pc = nullptr;
     double *Ak = nullptr, *kcoe = nullptr;
-    double *rho_re = nullptr, *rho_im = nullptr, *C_re = nullptr, *C_im = nullptr;
-    double *part_re = nullptr, *part_im = nullptr;
+    double *rho_re = nullptr, *rho_im = nullptr;
+    double4 *part = nullptr, *coef = nullptr;
     // per-atom vectors
     double *f = nullptr, *fpair = nullptr, *fdir = nullptr, *Erec = nullptr, *G = nullptr;
     double *Estat = nullptr, *mu = nullptr, *Eind = nullptr;
@@ -1466,20 +1677,18 @@ int upload_params(mdff_batch* b, const mdff_params& pin) {
 // coefficients C_k (RMODE of k_b_sfac_reduce).
 template <int MODE, int RMODE>
 int structure_factor(mdff_batch* b, const int* conv, const double* mu) {
-    const size_t sm = sizeof(double2) * (size_t)CHUNK * b->phw_max;
-    k_b_sfac<MODE><<<b->nchunk, KT, sm, b->st>>>(b->chunk, b->cfg, conv, b->N, b->sx, b->sy, b->sz, b->q, mu, b->R,
-                                                 b->part_re, b->part_im);
-    k_b_sfac_reduce<RMODE><<<nblk(b->nrect_tot, 256), 256, 0, b->st>>>(b->nrect_tot, b->rcfg, b->cfg, b->chunk, conv,
-                                                                       b->part_re, b->part_im, b->Ak, b->kcoe, b->Sres,
-                                                                       b->fl, b->rho_re, b->rho_im, b->C_re, b->C_im);
+    k_b_sfac<MODE><<<(unsigned)b->hjob.size(), KT, b->sm_sfac, b->st>>>(b->job, b->chunk, b->cfg, conv, b->N, b->tab, b->q,
+                                                                        mu, b->R, b->part);
+    k_b_sfac_reduce<RMODE><<<nblk(b->ncoef_tot, 128), 128, 0, b->st>>>(b->ncoef_tot, b->ccfg, b->cfg, b->chunk, conv,
+                                                                       b->part, b->Ak, b->kcoe, b->Sres, b->fl,
+                                                                       b->rho_re, b->rho_im, b->coef);
     return blaunch(b, "structure factor");
 }
 
 template <int GRAD, int ADD, int SCALE>
 int kfield(mdff_batch* b, const int* conv, double* V, double* G) {
-    size_t sm = sizeof(double) * 2 * CT * b->nzl_max;
-    k_b_kfield<GRAD, ADD, SCALE><<<b->nchunk, KT * KF_LPA, sm, b->st>>>(b->chunk, b->cfg, conv, b->N, b->sx, b->sy,
-                                                                        b->sz, b->C_re, b->C_im, V, G);
+    k_b_kfield<GRAD, ADD, SCALE><<<(unsigned)b->hfjob.size(), FT, b->sm_field, b->st>>>(b->fjob, b->cfg, conv, b->N, b->tab,
+                                                                                        b->coef, V, G);
     return blaunch(b, "kfield");
 }
 
@@ -1982,6 +2191,9 @@ int mdff_batch_create(const mdff_params* p, int nconf, const int* natm, const in
     long off = 0;
     int roff = 0;
     int cap_est = 32;
+    int krect_max = 1;       // widest k rectangle, in X + Y + eighths of nz entries
+    long tab_len = 0;
+    std::vector<int2> blks;  // (configuration, first atom) of the phase tables' blocks
     for (int c = 0; c < nconf; ++c) {
         BCfg& C = b->hcfg[c];
         std::memset(&C, 0, sizeof C);
@@ -2006,8 +2218,22 @@ int mdff_batch_create(const mdff_params* p, int nconf, const int* natm, const in
         C.nrect = C.ncol * C.nzl;
         C.roff = roff;
         roff += C.nrect;
-        b->nzl_max = std::max(b->nzl_max, C.nzl);
-        b->phw_max = std::max(b->phw_max, (C.kmax[0] + 1) + (2 * C.kmax[1] + 1) + (C.nzl + NZC - 1) / NZC);
+        krect_max = std::max(krect_max, (C.kmax[0] + 1) + (2 * C.kmax[1] + 1) + (C.nzl + 7) / 8);
+        const int nm = C.kmax[2] + 1;
+        C.npair = (C.kmax[0] + 1) * (C.kmax[1] + 1);
+        C.coff = b->ncoef_tot;
+        b->ncoef_tot += 2 * C.npair * nm;
+        C.W = C.kmax[0] + 1 + C.kmax[1] + 1 + 2 * nm;
+        C.toff = tab_len;
+        tab_len += (long)((C.n + AB - 1) / AB) * C.W * AP;
+        // m values per item: the fewest products, ~20 to make an amplitude and 16 for
+        // each m, padding counted
+        C.mc = 4;
+        auto cost = [&](int mc) { return (nm + mc - 1) / mc * (20 + 16 * mc); };
+        for (int mc = 5; mc <= 6; ++mc)
+            if (cost(mc) < cost(C.mc)) C.mc = mc;
+        b->sm_sfac = std::max(b->sm_sfac, sizeof(double2) * (2 * C.W + 6) * AP);   // (6: m values past kz of the last item)
+        b->sm_field = std::max(b->sm_field, sizeof(double2) * 2 * FPP * 4 * nm);
         double dens = natm[c] / C.cell.omega;
         int est = (int)(dens * 4.0 / 3.0 * PI * rc[c] * rc[c] * rc[c] * 1.3) + 32;
         cap_est = std::max(cap_est, std::min(est, natm[c]));
@@ -2018,11 +2244,27 @@ int mdff_batch_create(const mdff_params* p, int nconf, const int* natm, const in
             ch.a0 = C.off + a0;
             ch.na = std::min(CHUNK, C.n - a0);
             ch.poff = b->part_len;
-            b->part_len += C.nrect;
+            b->part_len += 2 * C.npair * nm;
+            // the chunk's items in blocks of whole warps, as even as they go
+            const int items = C.npair * ((nm + C.mc - 1) / C.mc), nj = (items + KT - 1) / KT;
+            const int per = ((items + nj - 1) / nj + 31) / 32 * 32;
+            for (int i0 = 0; i0 < items; i0 += per)
+                b->hjob.push_back({(int)b->hchunk.size(), i0, std::min(per, items - i0)});
             b->hchunk.push_back(ch);
         }
         C.ce = (int)b->hchunk.size();
+        for (int a0 = 0; a0 < C.n; a0 += FCH) b->hfjob.push_back(make_int2(c, a0));
+        for (int a0 = 0; a0 < C.n; a0 += AB) blks.push_back(make_int2(c, a0));
     }
+    // the longest jobs first, so that the last ones to run are short
+    std::stable_sort(b->hjob.begin(), b->hjob.end(), [&](const BJob& u, const BJob& v) {
+        auto t = [&](const BJob& j) { const BChunk& h = b->hchunk[j.chunk]; return h.na * (20 + 16 * b->hcfg[h.c].mc); };
+        return t(u) > t(v);
+    });
+    std::stable_sort(b->hfjob.begin(), b->hfjob.end(), [&](const int2& u, const int2& v) {
+        auto t = [&](const int2& j) { return b->hcfg[j.x].npair * (b->hcfg[j.x].kmax[2] + 3); };
+        return t(u) > t(v);
+    });
     b->nrect_tot = roff;
     b->nchunk = (int)b->hchunk.size();
     b->hconv.assign(nconf, 0);
@@ -2031,7 +2273,12 @@ int mdff_batch_create(const mdff_params* p, int nconf, const int* natm, const in
     auto A = [&](auto** ptr, size_t n) { if (r == MDFF_OK) r = balloc(b, ptr, n); };
     A(&b->cfg, nconf);
     A(&b->chunk, b->nchunk);
-    A(&b->rcfg, b->nrect_tot);
+    A(&b->ccfg, b->ncoef_tot);
+    A(&b->job, b->hjob.size());
+    A(&b->fjob, b->hfjob.size());
+    A(&b->tab, tab_len);
+    int2* dblks = nullptr;
+    A(&dblks, blks.size());
     A(&b->cfg_of, N);
     A(&b->type, N);
     for (double** v : {&b->x, &b->y, &b->z, &b->sx, &b->sy, &b->sz, &b->q, &b->alpha, &b->inv_alpha, &b->e_pair,
@@ -2044,9 +2291,9 @@ int mdff_batch_create(const mdff_params* p, int nconf, const int* natm, const in
     A(&b->s_pair, 6 * N);
     A(&b->s_dir, 6 * N);
     A(&b->pc, NT * NT);
-    for (double** v : {&b->Ak, &b->kcoe, &b->rho_re, &b->rho_im, &b->C_re, &b->C_im}) A(v, b->nrect_tot);
-    A(&b->part_re, b->part_len);
-    A(&b->part_im, b->part_len);
+    for (double** v : {&b->Ak, &b->kcoe, &b->rho_re, &b->rho_im}) A(v, b->nrect_tot);
+    A(&b->part, b->part_len);
+    A(&b->coef, b->ncoef_tot);
     A(&b->conv, nconf);
     A(&b->sc, nconf);
     A(&b->red, 40 * nconf);
@@ -2062,7 +2309,7 @@ int mdff_batch_create(const mdff_params* p, int nconf, const int* natm, const in
     A(&b->gsum, 64);
     if (r) return bad(r);
     // host tables
-    std::vector<int> hcfg_of(N), ht(N), hr(b->nrect_tot);
+    std::vector<int> hcfg_of(N), ht(N), hcc(b->ncoef_tot);
     std::vector<double> hak(b->nrect_tot, 0.0), hkc(b->nrect_tot, 0.0);
     for (int c = 0; c < nconf; ++c) {
         const BCfg& C = b->hcfg[c];
@@ -2072,8 +2319,8 @@ int mdff_batch_create(const mdff_params* p, int nconf, const int* natm, const in
             ht[i] = itype[i] - 1;
         }
         const double a2 = C.alpha * C.alpha;
+        std::fill_n(hcc.begin() + C.coff, 2 * C.npair * (C.kmax[2] + 1), c);
         for (int l = 0; l < C.nrect; ++l) {
-            hr[C.roff + l] = c;
             int col = l / C.nzl, nx = col / (2 * C.kmax[1] + 1), ny = col % (2 * C.kmax[1] + 1) - C.kmax[1];
             int nz = l % C.nzl - C.kmax[2];
             bool keep = nx > 0 || (nx == 0 && ny > 0) || (nx == 0 && ny == 0 && nz > 0);
@@ -2089,7 +2336,10 @@ int mdff_batch_create(const mdff_params* p, int nconf, const int* natm, const in
         }
     }
     if ((e = cudaMemcpyAsync(b->chunk, b->hchunk.data(), sizeof(BChunk) * b->nchunk, cudaMemcpyHostToDevice, b->st)) ||
-        (e = cudaMemcpyAsync(b->rcfg, hr.data(), sizeof(int) * b->nrect_tot, cudaMemcpyHostToDevice, b->st)) ||
+        (e = cudaMemcpyAsync(b->ccfg, hcc.data(), sizeof(int) * b->ncoef_tot, cudaMemcpyHostToDevice, b->st)) ||
+        (e = cudaMemcpyAsync(b->job, b->hjob.data(), sizeof(BJob) * b->hjob.size(), cudaMemcpyHostToDevice, b->st)) ||
+        (e = cudaMemcpyAsync(b->fjob, b->hfjob.data(), sizeof(int2) * b->hfjob.size(), cudaMemcpyHostToDevice, b->st)) ||
+        (e = cudaMemcpyAsync(dblks, blks.data(), sizeof(int2) * blks.size(), cudaMemcpyHostToDevice, b->st)) ||
         (e = cudaMemcpyAsync(b->cfg_of, hcfg_of.data(), sizeof(int) * N, cudaMemcpyHostToDevice, b->st)) ||
         (e = cudaMemcpyAsync(b->type, ht.data(), sizeof(int) * N, cudaMemcpyHostToDevice, b->st)) ||
         (e = cudaMemcpyAsync(b->Ak, hak.data(), sizeof(double) * b->nrect_tot, cudaMemcpyHostToDevice, b->st)) ||
@@ -2134,16 +2384,15 @@ int mdff_batch_create(const mdff_params* p, int nconf, const int* natm, const in
         if (attempt == 3) return bad(bfail(b, MDFF_E_LISTOVF, "batch: neighbour list capacity exceeded"));
         cap = (int)(ovf * 1.25) + 32;
     }
-    {   // the structure factor's per-atom phase tables live in dynamic shared memory
-        const size_t sm = sizeof(double2) * (size_t)CHUNK * b->phw_max;
-        if (sm > 200 * 1024)
-            return bad(bfail(b, MDFF_E_UNSUPPORTED, "batch: k rectangle too large for the structure factor's tables"));
-        cudaError_t e2 = cudaFuncSetAttribute(k_b_sfac<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e2 == cudaSuccess) e2 = cudaFuncSetAttribute(k_b_sfac<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e2 == cudaSuccess) e2 = cudaFuncSetAttribute(k_b_sfac<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e2 == cudaSuccess) e2 = cudaFuncSetAttribute(k_b_sfac<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e2 != cudaSuccess) return bad(bfail(b, MDFF_E_CUDA, cudaGetErrorString(e2)));
-    }
+    if (sizeof(double2) * (size_t)CHUNK * krect_max > 200 * 1024)
+        return bad(bfail(b, MDFF_E_UNSUPPORTED, "batch: k rectangle too large for the structure factor's tables"));
+    // one shared-memory limit for every batch of the process, whatever its sizes
+    for (const void* f : {(const void*)k_b_sfac<0>, (const void*)k_b_sfac<1>, (const void*)k_b_sfac<2>, (const void*)k_b_sfac<3>,
+                          (const void*)k_b_kfield<0, 1, 1>, (const void*)k_b_kfield<1, 0, 1>, (const void*)k_b_kfield<0, 1, 0>})
+        if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024)))
+            return bad(bfail(b, MDFF_E_CUDA, cudaGetErrorString(e)));
+    k_b_tables<<<(unsigned)blks.size(), 256, 0, b->st>>>(dblks, b->cfg, b->sx, b->sy, b->sz, b->tab);
+    if (int r2 = blaunch(b, "batch tables")) return bad(r2);
     if (int r2 = build_ddtab(b)) return bad(r2);
     return MDFF_OK;
 }

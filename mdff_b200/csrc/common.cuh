@@ -50,6 +50,12 @@ __device__ __forceinline__ double pairvec(int geom, const CellP& c, double si1, 
     return fma(rz, rz, fma(ry, ry, rx * rx));
 }
 
+// e^{2 pi i n s}: n s mod 1 with the product's rounding error carried along
+__device__ __forceinline__ void phase(double n, double s, double& c, double& sn) {
+    const double p = n * s, e = fma(n, s, -p);
+    sincospi(2.0 * ((p - rint(p)) + e), &sn, &c);
+}
+
 // errfc (src/functions.f90:28-39): the reference's fitted erfc (Numerical
 // Recipes' Chebyshev approximation), selectable for bit-level parity studies.
 __device__ __forceinline__ double erfc_fit(double x) {

@@ -72,12 +72,6 @@ __device__ __forceinline__ void slices7(unsigned long long a, unsigned long long
     umma::slices4x4((uint32_t)a, (uint32_t)b, (uint32_t)c, (uint32_t)d, s[3], s[4], s[5], s[6]);
 }
 
-// e^{2 pi i n s}: n s mod 1 with the product's rounding error carried along
-__device__ __forceinline__ void phase(double n, double s, double& c, double& sn) {
-    const double p = n * s, e = fma(n, s, -p);
-    sincospi(2.0 * ((p - rint(p)) + e), &sn, &c);
-}
-
 __device__ __forceinline__ bool wait(uint64_t* b, uint32_t parity, int* err, int code, volatile int* stop) {
     if (umma::mbar_wait_ns(b, parity, WAIT_NS, stop)) return true;
     if (!*stop) atomicOr(err, code);
