@@ -63,6 +63,7 @@ struct BCfg {
     long toff;             // first phase-table value
     int npol;
     double rc2, alpha, selfa, selfa2;
+    int geom;              // GEOM_* (common.cuh)
     double cF, cS;         // loss weights
 };
 
@@ -74,7 +75,9 @@ struct BPair {
     double A, B, C, D, BD;
     double eps, rho, sig, rs;
     double db_i, dc_i, db_j, dc_j;
-    int dk_i, dk_j, ldamp, pad;
+    int dk_i, dk_j, ldamp;
+    int sym;               // the damping of (tj, ti) is that of (ti, tj) with i and j swapped
+    double qi, qj;         // charges of the two types
 };
 
 struct BFlags {
@@ -100,7 +103,8 @@ inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 // read_pos.f90:148-150 (kardir, periodicbc, dirkar) and kardir, per atom with
 // its configuration's cell; the engine's exact operation order.
 __global__ void k_b_wrap_frac(int N, const int* __restrict__ cfg_of, const BCfg* __restrict__ cf, double* x, double* y,
-                              double* z, double* sx, double* sy, double* sz) {
+                              double* z, const int* __restrict__ type, double* sx, double* sy, double* sz,
+                              double4* rec) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     const CellP& c = cf[cfg_of[i]].cell;
@@ -118,6 +122,14 @@ __global__ void k_b_wrap_frac(int N, const int* __restrict__ cfg_of, const BCfg*
     sx[i] = __dadd_rn(__dadd_rn(__dmul_rn(X, c.B[0]), __dmul_rn(Y, c.B[3])), __dmul_rn(Z, c.B[6]));
     sy[i] = __dadd_rn(__dadd_rn(__dmul_rn(X, c.B[1]), __dmul_rn(Y, c.B[4])), __dmul_rn(Z, c.B[7]));
     sz[i] = __dadd_rn(__dadd_rn(__dmul_rn(X, c.B[2]), __dmul_rn(Y, c.B[5])), __dmul_rn(Z, c.B[8]));
+    // gather record of the pair kernels
+    rec[i] = make_double4(sx[i], sy[i], sz[i], __longlong_as_double((long long)type[i]));
+}
+
+// A vector per atom ([3][N]) as 32-byte records, for the kernels that gather it.
+__global__ void k_b_records(int N, const double* __restrict__ v, double4* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < N) out[i] = make_double4(v[i], v[N + i], v[2 * N + i], 0.0);
 }
 
 // Full neighbour rows within rc of each configuration (all pairs of the
@@ -158,18 +170,27 @@ __global__ void k_b_nlist(int N, const int* __restrict__ cfg_of, const BCfg* __r
 // short-range pairs
 // --------------------------------------------------------------------------
 
-__device__ __forceinline__ void tt_fd(double b, double r, int k, double& f, double& fd) { tt_damp_d(b, 1.0, r, k, f, fd); }
-
 // Tang-Toennies pieces and their derivatives with respect to b and c:
 // g = 1 - f = c e^{-x} sum_{m<=k} x^m/m!, gd = f' = c b e^{-x} x^k/k!, x = b r.
 struct TTD { double g, gd, g_b, g_c, gd_b, gd_c; };
 __device__ __forceinline__ TTD tt_deriv(double b, double c, double r, int k) {
+    constexpr InvFact IF;
     const double x = b * r, e = exp(-x);
     double term = 1.0, sum = 1.0, inv = 1.0;
-    for (int m = 1; m <= k; ++m) {
-        inv = inv / (double)m;
-        term = term * x;
-        sum = fma(term, inv, sum);
+    if (k <= 16) {   // 1/m! from the table: a division a term took longer than the rest of it
+#pragma unroll
+        for (int m = 1; m <= 16; ++m) {
+            if (m > k) break;
+            inv = IF.v[m];
+            term = term * x;
+            sum = fma(term, inv, sum);
+        }
+    } else {
+        for (int m = 1; m <= k; ++m) {
+            inv = inv / (double)m;
+            term = term * x;
+            sum = fma(term, inv, sum);
+        }
     }
     const double tk = term * inv;
     TTD t;
@@ -182,12 +203,39 @@ __device__ __forceinline__ TTD tt_deriv(double b, double c, double r, int k) {
     return t;
 }
 
+// The neighbours of atom i's row for the lanes of its group: the record one
+// neighbour ahead, the index two ahead, so that a gather's latency lies under the
+// arithmetic of the neighbour before it.
+template <int G>
+struct Row {
+    const int* row;
+    const double4* rec;
+    int m, i, k, j, jn, jn2;
+    double4 r, rn;
+    __device__ __forceinline__ Row(const int* row_, const double4* rec_, int m_, int i_, int sub)
+        : row(row_), rec(rec_), m(m_), i(i_), k(sub - G) {
+        jn = sub < m ? row[sub] : i;
+        jn2 = sub + G < m ? row[sub + G] : i;
+        rn = ld_rec(rec + jn);
+    }
+    __device__ __forceinline__ bool next() {
+        k += G;
+        if (k >= m) return false;
+        j = jn;
+        r = rn;
+        jn = jn2;
+        rn = ld_rec(rec + jn);
+        jn2 = k + 2 * G < m ? row[k + 2 * G] : i;
+        return true;
+    }
+    __device__ __forceinline__ int type() const { return (int)__double_as_longlong(r.w); }
+};
+
 // Forces (written), per-atom energy and stress sums (half per ordered pair).
 template <int G>
 __global__ void __launch_bounds__(256) k_b_pair(int N, const int* __restrict__ cfg_of, const BCfg* __restrict__ cf,
-                                                const double* __restrict__ sx, const double* __restrict__ sy,
-                                                const double* __restrict__ sz, const int* __restrict__ type,
-                                                const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
+                                                const double4* __restrict__ rec, const int* __restrict__ nbr,
+                                                const int* __restrict__ cnt, int cap,
                                                 const BPair* __restrict__ pc, BFlags fl, double* __restrict__ f,
                                                 double* __restrict__ e_atom, double* __restrict__ s_atom) {
     const int gid = (int)(((long)blockIdx.x * blockDim.x + threadIdx.x) / G);
@@ -197,46 +245,34 @@ __global__ void __launch_bounds__(256) k_b_pair(int N, const int* __restrict__ c
     const BCfg& C = cf[cfg_of[i]];
     double F[3] = {0, 0, 0}, u = 0.0, S[6] = {0, 0, 0, 0, 0, 0};
     if (active) {
-        const double si1 = sx[i], si2 = sy[i], si3 = sz[i];
-        const int ti = type[i];
-        const int m = cnt[i];
-        const int* row = nbr + (size_t)i * cap;
-        for (int k = sub; k < m; k += G) {
-            const int j = row[k];
+        const double4 ri = ld_rec(rec + i);
+        const BPair* Pi = pc + (int)__double_as_longlong(ri.w) * NT;
+        const CellP cell = C.cell;
+        const int geom = C.geom;
+        const double rc2 = C.rc2;
+        Row<G> nb(nbr + (size_t)i * cap, rec, cnt[i], i, sub);
+        while (nb.next()) {
             double rx, ry, rz;
-            const double rsq = pairvec_exact(C.cell, si1, si2, si3, sx[j], sy[j], sz[j], rx, ry, rz);
-            if (!(rsq < C.rc2)) continue;
-            const BPair& P = pc[ti * NT + type[j]];
+            const double rsq = pairvec(geom, cell, ri.x, ri.y, ri.z, nb.r.x, nb.r.y, nb.r.z, rx, ry, rz);
+            if (!(rsq < rc2)) continue;
+            const BPair& P = Pi[nb.type()];
+            const double dm1 = rsqrt(rsq), d = rsq * dm1;
             double w = 0.0;
-            const double d = sqrt(rsq);
             if ((fl.bmh || fl.bmhftd) && P.A != 0.0) {
-                const double ir2 = 1.0 / rsq;
-                const double erh = P.A * exp(-P.B * d);
-                double ir6 = ir2 * ir2 * ir2;
-                double ir8 = ir6 * ir2;
-                ir6 *= P.C;
-                ir8 *= P.D;
-                double ir6d = ir6, ir8d = ir8, fd6 = 0.0, fd8 = 0.0;
-                if (fl.bmhftd) {
-                    double f6, f8;
-                    tt_fd(P.BD, d, 6, f6, fd6);
-                    tt_fd(P.BD, d, 8, f8, fd8);
-                    ir6d = ir6 * f6;
-                    ir8d = ir8 * f8;
-                }
-                w += (P.B * erh - 6.0 * ir6d / d - 8.0 * ir8d / d + ir6 * fd6 + ir8 * fd8) / d;
-                u += 0.5 * (erh - ir6d - ir8d);
+                double ub;
+                w = bmh_pair(fl.bmhftd, P.A, P.B, P.C, P.D, P.BD, d, dm1, ub);
+                u += ub;
             }
             if (fl.morse) {
                 const double e = exp(-d * P.rho) * P.rs;
                 const double em1 = e - 1.0;
-                u += 0.5 * P.eps * (em1 * em1 - 1.0);
-                w += 2.0 * P.eps * P.rho * e * em1 / d;
+                u += P.eps * (em1 * em1 - 1.0);
+                w += 2.0 * P.eps * P.rho * e * em1 * dm1;
             }
-            F[0] += w * rx; F[1] += w * ry; F[2] += w * rz;
-            const double hw = 0.5 * w;
-            S[0] += hw * rx * rx; S[1] += hw * ry * ry; S[2] += hw * rz * rz;
-            S[3] += hw * rx * ry; S[4] += hw * rx * rz; S[5] += hw * ry * rz;
+            const double wx = w * rx, wy = w * ry;
+            F[0] += wx; F[1] += wy; F[2] = fma(w, rz, F[2]);
+            S[0] = fma(wx, rx, S[0]); S[1] = fma(wy, ry, S[1]); S[2] = fma(w * rz, rz, S[2]);
+            S[3] = fma(wx, ry, S[3]); S[4] = fma(wx, rz, S[4]); S[5] = fma(wy, rz, S[5]);
         }
     }
 #pragma unroll
@@ -246,8 +282,8 @@ __global__ void __launch_bounds__(256) k_b_pair(int N, const int* __restrict__ c
     u = group_sum<G>(u);
     if (active && sub == 0) {
         for (int k = 0; k < 3; ++k) f[(size_t)k * N + i] = F[k];
-        e_atom[i] = u;
-        for (int k = 0; k < 6; ++k) s_atom[(size_t)k * N + i] = S[k];
+        e_atom[i] = 0.5 * u;
+        for (int k = 0; k < 6; ++k) s_atom[(size_t)k * N + i] = 0.5 * S[k];
     }
 }
 
@@ -255,20 +291,21 @@ __global__ void __launch_bounds__(256) k_b_pair(int N, const int* __restrict__ c
 // real-space Ewald
 // --------------------------------------------------------------------------
 
-struct PairG { double d, A1, B2, C3, F0; };
+struct PairG { double d, dm3, dm5, A1, B2, C3, F0; };
 
-__device__ __forceinline__ PairG ewald_radial(double d2, double a, int erfc_ref) {
+__device__ __forceinline__ PairG ewald_radial(double d2, double a, int erfc_ref, const double* tab) {
     const double rsqpi = 0.56418958354775628695;
     const double a2 = a * a, a3 = a2 * a, a5 = a3 * a2;
     PairG g;
-    const double d = sqrt(d2);
-    const double dm1 = 1.0 / d, dm2 = dm1 * dm1, dm3 = dm1 * dm2, dm5 = dm3 * dm2, dm7 = dm5 * dm2;
+    const double dm1 = rsqrt(d2), d = d2 * dm1, dm2 = dm1 * dm1, dm3 = dm1 * dm2, dm5 = dm3 * dm2, dm7 = dm5 * dm2;
     const double ex2 = exp(-a2 * d2), expon = ex2 * rsqpi;
-    const double F0 = erfc_ref ? erfc_fit(a * d) : erfc_ex2(a * d, ex2);
+    const double F0 = erfc_ref ? erfc_fit(a * d) : erfc_ex2(a * d, ex2, tab);
     const double F1 = F0 + 2.0 * a * d * expon;
     const double F2 = F1 + (4.0 * a3 / 3.0) * d2 * d * expon;
     const double F3 = F2 + (8.0 * a5 / 15.0) * d2 * d2 * d * expon;
     g.d = d;
+    g.dm3 = dm3;
+    g.dm5 = dm5;
     g.F0 = F0 * dm1;
     g.A1 = F1 * dm3;
     g.B2 = 3.0 * F2 * dm5;
@@ -281,9 +318,11 @@ __device__ __forceinline__ PairG ewald_radial(double d2, double a, int erfc_ref)
 // A1 = F1/r^3, B2 = 3 F2/r^5 of the undamped dipole field are computed once
 // (k_b_ddtab_build) and every application of the operator in the forward and
 // adjoint solves is a gather: E_i = sum_j r (r.mu_j) B2 - mu_j A1.  Entries are
-// stored per quantity ([5][N cap]: rx ry rz A1 B2), FP64, or FP32 when the
-// batch runs mixed (the products then in FP32, the sums in FP64).  Rows are
-// compacted to the neighbours within rc in list order.
+// stored per quantity, FP64 ([4][N cap]: sqrt(B2) r, A1), or FP32 when the batch
+// runs mixed ([5][N cap]: rx ry rz A1 B2; the products then in FP32, the sums in
+// FP64).  Rows are compacted to the neighbours within rc in list order.  Bound by
+// the table's bytes: 28 million pairs (64 configurations, 69 642 ions) 152 us, 193 with
+// r and B2 apart.
 template <int G, typename T>
 __global__ void __launch_bounds__(256) k_b_ddtab_build(int N, const int* __restrict__ cfg_of,
                                                        const BCfg* __restrict__ cf, const double* __restrict__ sx,
@@ -311,14 +350,22 @@ __global__ void __launch_bounds__(256) k_b_ddtab_build(int N, const int* __restr
         const unsigned bal = (__ballot_sync(gmask, in) & gmask) >> g0;
         const int pos = base + __popc(bal & ((1u << sub) - 1u));
         if (in) {
-            const PairG g = ewald_radial(d2, C.alpha, erfc_ref);
+            const PairG g = ewald_radial(d2, C.alpha, erfc_ref, &c_erfcx[0][0]);
             const size_t e = (size_t)i * cap + pos;
             dnbr[e] = j;
-            tab[e] = (T)rx;
-            tab[NC + e] = (T)ry;
-            tab[2 * NC + e] = (T)rz;
-            tab[3 * NC + e] = (T)g.A1;
-            tab[4 * NC + e] = (T)g.B2;
+            if constexpr (sizeof(T) == 8) {
+                const double w = sqrt(g.B2);
+                tab[e] = w * rx;
+                tab[NC + e] = w * ry;
+                tab[2 * NC + e] = w * rz;
+                tab[3 * NC + e] = g.A1;
+            } else {
+                tab[e] = (T)rx;
+                tab[NC + e] = (T)ry;
+                tab[2 * NC + e] = (T)rz;
+                tab[3 * NC + e] = (T)g.A1;
+                tab[4 * NC + e] = (T)g.B2;
+            }
         }
         base += __popc(bal);
     }
@@ -342,9 +389,10 @@ __global__ void __launch_bounds__(256) k_b_ddtab(int N, const int* __restrict__ 
         for (int k = sub; k < m; k += G) {
             const size_t e = (size_t)i * cap + k;
             const int j = dnbr[e];
-            const T rx = tab[e], ry = tab[NC + e], rz = tab[2 * NC + e], A1 = tab[3 * NC + e], B2 = tab[4 * NC + e];
+            const T rx = tab[e], ry = tab[NC + e], rz = tab[2 * NC + e], A1 = tab[3 * NC + e];
             const T mj0 = (T)v[j], mj1 = (T)v[N + j], mj2 = (T)v[2 * N + j];
-            const T rb = (rx * mj0 + ry * mj1 + rz * mj2) * B2;
+            T rb = rx * mj0 + ry * mj1 + rz * mj2;
+            if constexpr (sizeof(T) == 4) rb = rb * tab[4 * NC + e];
             V0 += (double)(rx * rb - mj0 * A1);
             V1 += (double)(ry * rb - mj1 * A1);
             V2 += (double)(rz * rb - mj2 * A1);
@@ -358,64 +406,66 @@ __global__ void __launch_bounds__(256) k_b_ddtab(int N, const int* __restrict__ 
 
 // MODE 0: damped field of the charges (static field b of the dipole solve,
 //         src/field.f90:3270-3272).
-// MODE 1: field of the dipoles mu, undamped (the operator T, src/field.f90:3354).
 // MODE 2: forces, energy and stress of charges + dipoles with the damped
 //         charge-dipole terms (the final multipole_ES call).
+// (MODE 1, the dipole operator, is k_b_ddtab.)
+// The kernels over neighbour rows are bound by the FP64 pipe.  28 million pairs (64
+// configurations, 69 642 ions), us, with exact pair vectors, square roots,
+// divisions (one per damping term in the gradients) and 8-byte gathers -> now:
+// k_b_pair 478 -> 290, k_b_dir 0 542 -> 340, k_b_dir 2 809 -> 700, k_b_dir_adj 1 774 -> 1 000,
+// k_b_grad_rows 1 563 -> 635.  Eight lanes an atom instead of 16 change them by 3 %.
 template <int G, int MODE>
-__global__ void __launch_bounds__(256) k_b_dir(int N, const int* __restrict__ cfg_of, const BCfg* __restrict__ cf,
-                                               const int* __restrict__ conv, const double* __restrict__ sx,
-                                               const double* __restrict__ sy, const double* __restrict__ sz,
-                                               const int* __restrict__ type, const double* __restrict__ q,
-                                               const double* __restrict__ mu, const int* __restrict__ nbr,
-                                               const int* __restrict__ cnt, int cap, const BPair* __restrict__ pc,
-                                               BFlags fl, double* __restrict__ out, double* __restrict__ e_atom,
-                                               double* __restrict__ s_atom) {
+__global__ void __launch_bounds__(256, 2)
+    k_b_dir(int N, const int* __restrict__ cfg_of, const BCfg* __restrict__ cf, const double4* __restrict__ rec,
+            const double4* __restrict__ mrec, const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
+            const BPair* __restrict__ pc, BFlags fl, double* __restrict__ out, double* __restrict__ e_atom,
+            double* __restrict__ s_atom) {
+    __shared__ double s_erfcx[ERFCX_LEN];
+    for (int k = threadIdx.x; k < ERFCX_LEN; k += blockDim.x) s_erfcx[k] = (&c_erfcx[0][0])[k];
+    __syncthreads();
     const int gid = (int)(((long)blockIdx.x * blockDim.x + threadIdx.x) / G);
     const int sub = threadIdx.x & (G - 1);
-    bool active = gid < N;
+    const bool active = gid < N;
     const int i = active ? gid : 0;
-    const int c = cfg_of[i];
-    if (conv && conv[c]) active = false;
-    const BCfg& C = cf[c];
+    const BCfg& C = cf[cfg_of[i]];
     double V[3] = {0, 0, 0}, u = 0.0, S[6] = {0, 0, 0, 0, 0, 0};
     if (active) {
-        const double si1 = sx[i], si2 = sy[i], si3 = sz[i];
-        const int ti = type[i];
-        const double qi = MODE == 1 ? 0.0 : q[i];
-        const double mi0 = MODE == 0 ? 0.0 : mu[i], mi1 = MODE == 0 ? 0.0 : mu[N + i], mi2 = MODE == 0 ? 0.0 : mu[2 * N + i];
-        const int m = cnt[i];
-        const int* row = nbr + (size_t)i * cap;
-        for (int k = sub; k < m; k += G) {
-            const int j = row[k];
+        const double4 ri = ld_rec(rec + i);
+        const BPair* Pi = pc + (int)__double_as_longlong(ri.w) * NT;
+        double mi0 = 0.0, mi1 = 0.0, mi2 = 0.0;
+        if (MODE == 2) {
+            const double4 mi = ld_rec(mrec + i);
+            mi0 = mi.x; mi1 = mi.y; mi2 = mi.z;
+        }
+        const CellP cell = C.cell;
+        const int geom = C.geom;
+        const double rc2 = C.rc2, alpha = C.alpha;
+        Row<G> nb(nbr + (size_t)i * cap, rec, cnt[i], i, sub);
+        while (nb.next()) {
+            double4 mj = make_double4(0.0, 0.0, 0.0, 0.0);
+            if (MODE == 2) mj = ld_rec(mrec + nb.j);
             double rx, ry, rz;
-            const double d2 = pairvec_exact(C.cell, si1, si2, si3, sx[j], sy[j], sz[j], rx, ry, rz);
-            if (d2 > C.rc2) continue;
-            const PairG g = ewald_radial(d2, C.alpha, fl.erfc_ref);
-            if (MODE == 1) {
-                const double mj0 = mu[j], mj1 = mu[N + j], mj2 = mu[2 * N + j];
-                const double rmj = rx * mj0 + ry * mj1 + rz * mj2;
-                V[0] += rx * rmj * g.B2 - mj0 * g.A1;
-                V[1] += ry * rmj * g.B2 - mj1 * g.A1;
-                V[2] += rz * rmj * g.B2 - mj2 * g.A1;
-                continue;
-            }
-            const int tj = type[j];
-            const double qj = q[j];
-            const BPair& P = pc[ti * NT + tj];
+            const double d2 = pairvec(geom, cell, ri.x, ri.y, ri.z, nb.r.x, nb.r.y, nb.r.z, rx, ry, rz);
+            if (d2 > rc2) continue;
+            const PairG g = ewald_radial(d2, alpha, fl.erfc_ref, s_erfcx);
+            const BPair& P = Pi[nb.type()];
+            const double qi = P.qi, qj = P.qj;
             double gi = 0.0, gdi = 0.0, gj = 0.0, gdj = 0.0;
             if (P.ldamp) {
                 double f1, f2;
                 tt_damp_d(P.db_i, P.dc_i, g.d, P.dk_i, f1, gdi);
-                tt_damp_d(P.db_j, P.dc_j, g.d, P.dk_j, f2, gdj);
                 gi = 1.0 - f1;
-                gj = 1.0 - f2;
+                if (MODE == 2) {
+                    tt_damp_d(P.db_j, P.dc_j, g.d, P.dk_j, f2, gdj);
+                    gj = 1.0 - f2;
+                }
             }
             if (MODE == 0) {
-                const double s = qj * (g.A1 - gi / (g.d * d2));
+                const double s = qj * (g.A1 - gi * g.dm3);
                 V[0] += s * rx; V[1] += s * ry; V[2] += s * rz;
                 continue;
             }
-            const double mj0 = mu[j], mj1 = mu[N + j], mj2 = mu[2 * N + j];
+            const double mj0 = mj.x, mj1 = mj.y, mj2 = mj.z;
             const double rmj = rx * mj0 + ry * mj1 + rz * mj2;
             const double rmi = rx * mi0 + ry * mi1 + rz * mi2;
             const double mimj = mi0 * mj0 + mi1 * mj1 + mi2 * mj2;
@@ -437,10 +487,10 @@ __global__ void __launch_bounds__(256) k_b_dir(int N, const int* __restrict__ cf
             fi[1] += ry * s - (qi * mj1 - qj * mi1) * g.A1;
             fi[2] += rz * s - (qi * mj2 - qj * mi2) * g.A1;
             if (P.ldamp) {
-                const double dm3 = 1.0 / (g.d * d2), dm5 = dm3 / d2;
+                const double dm3 = g.dm3, dm5 = g.dm5, d3 = g.d * (1.0 / 3.0);
                 u += 0.5 * (-qi * gj * dm3 * rmj + qj * gi * dm3 * rmi);
-                const double Bi = 3.0 * (gi + (g.d / 3.0) * gdi) * dm5, Ai = gi * dm3;
-                const double Bj = 3.0 * (gj + (g.d / 3.0) * gdj) * dm5, Aj = gj * dm3;
+                const double Bi = 3.0 * (gi + d3 * gdi) * dm5, Ai = gi * dm3;
+                const double Bj = 3.0 * (gj + d3 * gdj) * dm5, Aj = gj * dm3;
                 fi[0] += qj * (rx * rmi * Bi - mi0 * Ai) - qi * (rx * rmj * Bj - mj0 * Aj);
                 fi[1] += qj * (ry * rmi * Bi - mi1 * Ai) - qi * (ry * rmj * Bj - mj1 * Aj);
                 fi[2] += qj * (rz * rmi * Bi - mi2 * Ai) - qi * (rz * rmj * Bj - mj2 * Aj);
@@ -494,14 +544,14 @@ __device__ __forceinline__ void force_mu_grad(const double r[3], const double W[
 // damped charge-dipole force w.r.t. the damping b and c at fixed mu (slots
 // G_DI_*, G_DJ_* of the ordered pair (ti,tj)).
 template <int G>
-__global__ void __launch_bounds__(256) k_b_dir_adj(int N, const int* __restrict__ cfg_of, const BCfg* __restrict__ cf,
-                                                   const double* __restrict__ sx, const double* __restrict__ sy,
-                                                   const double* __restrict__ sz, const int* __restrict__ type,
-                                                   const double* __restrict__ q, const double* __restrict__ mu,
-                                                   const double* __restrict__ R, const double* __restrict__ Sres,
-                                                   const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
-                                                   const BPair* __restrict__ pc, BFlags fl, double* __restrict__ h,
-                                                   double* part) {
+__global__ void __launch_bounds__(256, 2)
+    k_b_dir_adj(int N, const int* __restrict__ cfg_of, const BCfg* __restrict__ cf, const double4* __restrict__ rec,
+                const double4* __restrict__ mrec, const double4* __restrict__ rrec, const double* __restrict__ Sres,
+                const int* __restrict__ nbr, const int* __restrict__ cnt, int cap, const BPair* __restrict__ pc, BFlags fl,
+                double* __restrict__ h, double* part) {
+    __shared__ double s_erfcx[ERFCX_LEN];
+    for (int k = threadIdx.x; k < ERFCX_LEN; k += blockDim.x) s_erfcx[k] = (&c_erfcx[0][0])[k];
+    __syncthreads();
     const int gid = (int)(((long)blockIdx.x * blockDim.x + threadIdx.x) / G);
     const int sub = threadIdx.x & (G - 1);
     const bool active = gid < N;
@@ -512,44 +562,47 @@ __global__ void __launch_bounds__(256) k_b_dir_adj(int N, const int* __restrict_
     double acc[NTYB][4];
 #pragma unroll
     for (int t = 0; t < NTYB; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.0;
-    const int ti = type[i];
+    const double4 ri = ld_rec(rec + i);
+    const int ti = (int)__double_as_longlong(ri.w);
     if (active) {
-        const double si1 = sx[i], si2 = sy[i], si3 = sz[i];
-        const double qi = q[i];
-        const double mi[3] = {mu[i], mu[N + i], mu[2 * N + i]};
-        const double Ri[3] = {R[i], R[N + i], R[2 * N + i]};
+        const double4 mi4 = ld_rec(mrec + i), Ri4 = ld_rec(rrec + i);
+        const double mi[3] = {mi4.x, mi4.y, mi4.z};
+        const double Ri[3] = {Ri4.x, Ri4.y, Ri4.z};
         double Sm[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) Sm[k] = Sres[c * 9 + k];
         const double sw = 0.5 * fl.cu / (C.cell.omega * fl.press);
-        const int m = cnt[i];
-        const int* row = nbr + (size_t)i * cap;
-        for (int k = sub; k < m; k += G) {
-            const int j = row[k];
+        const CellP cell = C.cell;
+        const int geom = C.geom;
+        const double rc2 = C.rc2, alpha = C.alpha;
+        Row<G> nb(nbr + (size_t)i * cap, rec, cnt[i], i, sub);
+        while (nb.next()) {
+            const double4 mj4 = ld_rec(mrec + nb.j), Rj4 = ld_rec(rrec + nb.j);
             double r[3];
-            const double d2 = pairvec_exact(C.cell, si1, si2, si3, sx[j], sy[j], sz[j], r[0], r[1], r[2]);
-            if (d2 > C.rc2) continue;
-            const PairG g = ewald_radial(d2, C.alpha, fl.erfc_ref);
-            const int tj = type[j];
-            const double qj = q[j];
-            const double mj[3] = {mu[j], mu[N + j], mu[2 * N + j]};
-            const double Rj[3] = {R[j], R[N + j], R[2 * N + j]};
+            const double d2 = pairvec(geom, cell, ri.x, ri.y, ri.z, nb.r.x, nb.r.y, nb.r.z, r[0], r[1], r[2]);
+            if (d2 > rc2) continue;
+            const PairG g = ewald_radial(d2, alpha, fl.erfc_ref, s_erfcx);
+            const int tj = nb.type();
+            const BPair& P = pc[ti * NT + tj];
+            const double qi = P.qi, qj = P.qj;
+            const double mj[3] = {mj4.x, mj4.y, mj4.z};
+            const double Rj[3] = {Rj4.x, Rj4.y, Rj4.z};
             double Sr[3];
 #pragma unroll
             for (int a = 0; a < 3; ++a) Sr[a] = Sm[a * 3] * r[0] + Sm[a * 3 + 1] * r[1] + Sm[a * 3 + 2] * r[2];
-            const double dm3 = 1.0 / (g.d * d2), dm5 = dm3 / d2;
+            const double dm3 = g.dm3, dm5 = g.dm5, d3 = g.d * (1.0 / 3.0);
             // evaluation (i,j): W_ij = cu R_i + sw S r
             double W[3], hf[3], hs[3];
 #pragma unroll
             for (int a = 0; a < 3; ++a) W[a] = fl.cu * Ri[a] + sw * Sr[a];
-            const BPair& P = pc[ti * NT + tj];
             double Bi = 0, Ai = 0, Bj = 0, Aj = 0;
             TTD Ti{}, Tj{};
             if (P.ldamp) {
                 Ti = tt_deriv(P.db_i, P.dc_i, g.d, P.dk_i);
-                Tj = tt_deriv(P.db_j, P.dc_j, g.d, P.dk_j);
-                Ai = Ti.g * dm3; Bi = 3.0 * (Ti.g + g.d / 3.0 * Ti.gd) * dm5;
-                Aj = Tj.g * dm3; Bj = 3.0 * (Tj.g + g.d / 3.0 * Tj.gd) * dm5;
+                // (identical constants at both atoms: identical values)
+                Tj = P.db_j == P.db_i && P.dc_j == P.dc_i && P.dk_j == P.dk_i ? Ti : tt_deriv(P.db_j, P.dc_j, g.d, P.dk_j);
+                Ai = Ti.g * dm3; Bi = 3.0 * (Ti.g + d3 * Ti.gd) * dm5;
+                Aj = Tj.g * dm3; Bj = 3.0 * (Tj.g + d3 * Tj.gd) * dm5;
             }
             force_mu_grad(r, W, qi, qj, mi, mj, g, Bi, Ai, Bj, Aj, hf, hs);
             H[0] += hf[0]; H[1] += hf[1]; H[2] += hf[2];
@@ -578,13 +631,16 @@ __global__ void __launch_bounds__(256) k_b_dir_adj(int N, const int* __restrict_
             for (int a = 0; a < 3; ++a) W[a] = fl.cu * Rj[a] - sw * Sr[a];
             const BPair& Q = pc[tj * NT + ti];
             double Bf = 0, Af = 0, Bs = 0, As = 0;
-            if (Q.ldamp) {
+            if (P.sym) {   // the factors of (i,j), swapped
+                Af = Aj; Bf = Bj;
+                As = Ai; Bs = Bi;
+            } else if (Q.ldamp) {
                 double f1, gd1, f2, gd2;
                 tt_damp_d(Q.db_i, Q.dc_i, g.d, Q.dk_i, f1, gd1);
                 tt_damp_d(Q.db_j, Q.dc_j, g.d, Q.dk_j, f2, gd2);
                 const double g1 = 1.0 - f1, g2 = 1.0 - f2;
-                Af = g1 * dm3; Bf = 3.0 * (g1 + g.d / 3.0 * gd1) * dm5;
-                As = g2 * dm3; Bs = 3.0 * (g2 + g.d / 3.0 * gd2) * dm5;
+                Af = g1 * dm3; Bf = 3.0 * (g1 + d3 * gd1) * dm5;
+                As = g2 * dm3; Bs = 3.0 * (g2 + d3 * gd2) * dm5;
             }
             force_mu_grad(rn, W, qj, qi, mj, mi, g, Bf, Af, Bs, As, hf, hs);
             H[0] += hs[0]; H[1] += hs[1]; H[2] += hs[2];
@@ -608,13 +664,12 @@ __global__ void __launch_bounds__(256) k_b_dir_adj(int N, const int* __restrict_
 // parameters (dw/dtheta [R_i.r + r.S.r/(2 omega press)] per ordered pair) and
 // the damping of the static field (-q_j lambda_i.r/d^3 dg_i/dtheta).
 template <int G>
-__global__ void __launch_bounds__(256) k_b_grad_rows(int N, const int* __restrict__ cfg_of, const BCfg* __restrict__ cf,
-                                                     const double* __restrict__ sx, const double* __restrict__ sy,
-                                                     const double* __restrict__ sz, const int* __restrict__ type,
-                                                     const double* __restrict__ q, const double* __restrict__ R,
-                                                     const double* __restrict__ Sres, const double* __restrict__ lam,
-                                                     const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
-                                                     const BPair* __restrict__ pc, BFlags fl, double* part) {
+__global__ void __launch_bounds__(256, 2)
+    k_b_grad_rows(int N, const int* __restrict__ cfg_of, const BCfg* __restrict__ cf, const double4* __restrict__ rec,
+                  const double* __restrict__ R, const double* __restrict__ Sres, const double* __restrict__ lam,
+                  const int* __restrict__ nbr, const int* __restrict__ cnt, int cap, const BPair* __restrict__ pc,
+                  BFlags fl, double* part) {
+    constexpr InvFact IF;
     const int gid = (int)(((long)blockIdx.x * blockDim.x + threadIdx.x) / G);
     const int sub = threadIdx.x & (G - 1);
     const bool active = gid < N;
@@ -627,67 +682,83 @@ __global__ void __launch_bounds__(256) k_b_grad_rows(int N, const int* __restric
     for (int t = 0; t < NTYB; ++t)
 #pragma unroll
         for (int s = 0; s < NS; ++s) acc[t][s] = 0.0;
-    const int ti = type[i];
+    const double4 ri = ld_rec(rec + i);
+    const int ti = (int)__double_as_longlong(ri.w);
     if (active) {
-        const double si1 = sx[i], si2 = sy[i], si3 = sz[i];
         const double Ri[3] = {R[i], R[N + i], R[2 * N + i]};
         const double li[3] = {lam[i], lam[N + i], lam[2 * N + i]};
         double Sm[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) Sm[k] = Sres[c * 9 + k];
         const double so2 = 0.5 / (C.cell.omega * fl.press);
-        const int m = cnt[i];
-        const int* row = nbr + (size_t)i * cap;
-        for (int k = sub; k < m; k += G) {
-            const int j = row[k];
+        const CellP cell = C.cell;
+        const int geom = C.geom;
+        const double rc2 = C.rc2;
+        Row<G> nb(nbr + (size_t)i * cap, rec, cnt[i], i, sub);
+        while (nb.next()) {
             double r[3];
-            const double d2 = pairvec_exact(C.cell, si1, si2, si3, sx[j], sy[j], sz[j], r[0], r[1], r[2]);
-            if (d2 > C.rc2) continue;
-            const int tj = type[j];
+            const double d2 = pairvec(geom, cell, ri.x, ri.y, ri.z, nb.r.x, nb.r.y, nb.r.z, r[0], r[1], r[2]);
+            if (d2 > rc2) continue;
+            const int tj = nb.type();
             const BPair& P = pc[ti * NT + tj];
-            const double d = sqrt(d2);
+            const double dm1 = rsqrt(d2), d = d2 * dm1;
             double v[NS];
 #pragma unroll
             for (int s = 0; s < NS; ++s) v[s] = 0.0;
-            if (d2 < C.rc2) {
+            if (d2 < rc2) {
                 double rSr = 0.0;
 #pragma unroll
                 for (int a = 0; a < 3; ++a) rSr += r[a] * (Sm[a * 3] * r[0] + Sm[a * 3 + 1] * r[1] + Sm[a * 3 + 2] * r[2]);
-                const double geo = Ri[0] * r[0] + Ri[1] * r[1] + Ri[2] * r[2] + so2 * rSr;
+                const double geo = (Ri[0] * r[0] + Ri[1] * r[1] + Ri[2] * r[2] + so2 * rSr) * dm1;
                 if ((fl.bmh || fl.bmhftd) && P.A != 0.0) {
-                    const double e1 = exp(-P.B * d), erh = P.A * e1;
-                    const double d6 = 1.0 / (d2 * d2 * d2), d8 = d6 / d2;
-                    double f6 = 1.0, f8 = 1.0, fd6 = 0.0, fd8 = 0.0, df6 = 0.0, df8 = 0.0, dfd6 = 0.0, dfd8 = 0.0;
-                    if (fl.bmhftd) {
-                        const TTD a6 = tt_deriv(P.BD, 1.0, d, 6), a8 = tt_deriv(P.BD, 1.0, d, 8);
-                        f6 = 1.0 - a6.g; fd6 = a6.gd; df6 = -a6.g_b; dfd6 = a6.gd_b;
-                        f8 = 1.0 - a8.g; fd8 = a8.gd; df8 = -a8.g_b; dfd8 = a8.gd_b;
+                    const double e1 = exp(-P.B * d), dm2 = dm1 * dm1;
+                    const double d6 = dm2 * dm2 * dm2, d8 = d6 * dm2;
+                    double f6 = 1.0, f8 = 1.0, fd6 = 0.0, fd8 = 0.0;
+                    if (fl.bmhftd) {   // Tang-Toennies of orders 6 and 8 (tt_deriv with c = 1), one series for both
+                        const double x = P.BD * d, e = exp(-x);
+                        double term = 1.0, sum = 1.0;
+#pragma unroll
+                        for (int m = 1; m <= 6; ++m) {
+                            term *= x;
+                            sum = fma(term, IF.v[m], sum);
+                        }
+                        f6 = 1.0 - e * sum;
+                        const double et6 = e * (term * IF.v[6]);
+                        term *= x;
+                        sum = fma(term, IF.v[7], sum);
+                        term *= x;
+                        sum = fma(term, IF.v[8], sum);
+                        f8 = 1.0 - e * sum;
+                        const double et8 = e * (term * IF.v[8]);
+                        fd6 = P.BD * et6;
+                        fd8 = P.BD * et8;
+                        // d f/d BD = d et, d f'/d BD = et (1 + k - x)
+                        v[4] = geo * (P.C * d6 * et6 * (1.0 - x) + P.D * d8 * et8 * (1.0 - x));
                     }
-                    v[0] = geo * P.B * e1 / d;
-                    v[1] = geo * erh * (1.0 - P.B * d) / d;
-                    v[2] = geo * (-6.0 * f6 * d6 / d + fd6 * d6) / d;
-                    v[3] = geo * (-8.0 * f8 * d8 / d + fd8 * d8) / d;
-                    if (fl.bmhftd)
-                        v[4] = geo * (-6.0 * P.C * d6 / d * df6 - 8.0 * P.D * d8 / d * df8 + P.C * d6 * dfd6 + P.D * d8 * dfd8) / d;
+                    v[0] = geo * P.B * e1;
+                    v[1] = geo * P.A * e1 * (1.0 - P.B * d);
+                    v[2] = geo * d6 * (fd6 - 6.0 * f6 * dm1);
+                    v[3] = geo * d8 * (fd8 - 8.0 * f8 * dm1);
                 }
                 if (fl.morse) {
                     const double e = exp(-d * P.rho) * P.rs;
-                    v[5] = geo * 2.0 * P.rho * e * (e - 1.0) / d;
-                    v[6] = geo * 2.0 * P.eps / d * (e * (e - 1.0) + P.rho * (P.sig - d) * e * (2.0 * e - 1.0));
-                    v[7] = geo * 2.0 * P.eps * P.rho / d * P.rho * e * (2.0 * e - 1.0);
+                    v[5] = geo * 2.0 * P.rho * e * (e - 1.0);
+                    v[6] = geo * 2.0 * P.eps * (e * (e - 1.0) + P.rho * (P.sig - d) * e * (2.0 * e - 1.0));
+                    v[7] = geo * 2.0 * P.eps * P.rho * P.rho * e * (2.0 * e - 1.0);
                 }
             }
             if (fl.coul && P.ldamp) {
                 const TTD Ti = tt_deriv(P.db_i, P.dc_i, d, P.dk_i);
-                const double lr = (li[0] * r[0] + li[1] * r[1] + li[2] * r[2]) / (d * d2);
-                v[8] = -q[j] * lr * Ti.g_b;
-                v[9] = -q[j] * lr * Ti.g_c;
+                const double lr = -P.qj * (li[0] * r[0] + li[1] * r[1] + li[2] * r[2]) * (dm1 * dm1 * dm1);
+                v[8] = lr * Ti.g_b;
+                v[9] = lr * Ti.g_c;
             }
 #pragma unroll
             for (int t = 0; t < NTYB; ++t)
                 if (t == tj)
 #pragma unroll
-                    for (int s = 0; s < NS; ++s) acc[t][s] += v[s];
+                    for (int s = 0; s < NS; ++s)
+                        if (s < 5 || s > 7 || fl.morse) acc[t][s] += v[s];
         }
     }
     double v[NTYB * NTYB * NS];
@@ -1480,6 +1551,7 @@ struct mdff_batch {
     int* cfg_of = nullptr;
     int* type = nullptr;
     double *x = nullptr, *y = nullptr, *z = nullptr, *sx = nullptr, *sy = nullptr, *sz = nullptr;
+    double4 *rec = nullptr, *mrec = nullptr, *rrec = nullptr;   // gather records: (fractional coordinates, type), dipoles, residuals
     double *q = nullptr, *alpha = nullptr, *inv_alpha = nullptr;
     int *nbr = nullptr, *cnt = nullptr, cap = 0;
     int* overflow = nullptr;
@@ -1641,6 +1713,14 @@ int upload_params(mdff_batch* b, const mdff_params& pin) {
             P.db_i = p.dip_pol_damp_b[it][it][jt]; P.dc_i = p.dip_pol_damp_c[it][it][jt]; P.dk_i = p.dip_pol_damp_k[it][it][jt];
             P.db_j = p.dip_pol_damp_b[jt][it][jt]; P.dc_j = p.dip_pol_damp_c[jt][it][jt]; P.dk_j = p.dip_pol_damp_k[jt][it][jt];
             P.ldamp = (p.lcoulomb && (p.ldip_damping[it][it][jt] || p.ldip_damping[jt][it][jt])) ? 1 : 0;
+            P.qi = p.qch[it];
+            P.qj = p.qch[jt];
+        }
+    for (int it = 0; it < p.ntype; ++it)
+        for (int jt = 0; jt < p.ntype; ++jt) {
+            BPair &P = tab[it * NT + jt], &Q = tab[jt * NT + it];
+            P.sym = P.ldamp == Q.ldamp && P.db_i == Q.db_j && P.dc_i == Q.dc_j && P.dk_i == Q.dk_j && P.db_j == Q.db_i &&
+                    P.dc_j == Q.dc_i && P.dk_j == Q.dk_i;
         }
     BCK(cudaMemcpyAsync(b->pc, tab.data(), sizeof(BPair) * NT * NT, cudaMemcpyHostToDevice, b->st));
     // per-atom polarisabilities and charges
@@ -1726,7 +1806,7 @@ int build_ddtab(mdff_batch* b) {
         BTRY(balloc(b, &b->dd_nbr, NC));
         BTRY(balloc(b, &b->dd_cnt, (size_t)N));
         if (mixed) BTRY(balloc(b, &b->dd32, 5 * NC));
-        else BTRY(balloc(b, &b->dd64, 5 * NC));
+        else BTRY(balloc(b, &b->dd64, 4 * NC));
     }
     const int er = b->fl.erfc_ref;
     if (mixed)
@@ -1835,9 +1915,8 @@ int forward_launches(mdff_batch* b, bool captured) {
     const int N = b->N;
     const mdff_params& p = b->p;
     if (p.lbmhft || p.lbmhftd || p.lmorse) {
-        k_b_pair<8><<<nblk((long)N * 8, 256), 256, 0, b->st>>>(N, b->cfg_of, b->cfg, b->sx, b->sy, b->sz, b->type,
-                                                             b->nbr, b->cnt, b->cap, b->pc, b->fl, b->fpair,
-                                                             b->e_pair, b->s_pair);
+        k_b_pair<8><<<nblk((long)N * 8, 256), 256, 0, b->st>>>(N, b->cfg_of, b->cfg, b->rec, b->nbr, b->cnt, b->cap,
+                                                             b->pc, b->fl, b->fpair, b->e_pair, b->s_pair);
         BTRY(blaunch(b, "pair"));
     } else {
         BCK(cudaMemsetAsync(b->fpair, 0, sizeof(double) * 3 * N, b->st));
@@ -1847,9 +1926,8 @@ int forward_launches(mdff_batch* b, bool captured) {
     if (!captured) b->fwd_iters = 0;
     if (p.lcoulomb) {
         // static field b: damped charges, real + reciprocal
-        k_b_dir<16, 0><<<dir_blocks(N, 16), 256, 0, b->st>>>(N, b->cfg_of, b->cfg, nullptr, b->sx, b->sy, b->sz, b->type,
-                                                             b->q, nullptr, b->nbr, b->cnt, b->cap, b->pc, b->fl,
-                                                             b->Estat, nullptr, nullptr);
+        k_b_dir<16, 0><<<dir_blocks(N, 16), 256, 0, b->st>>>(N, b->cfg_of, b->cfg, b->rec, nullptr, b->nbr, b->cnt,
+                                                             b->cap, b->pc, b->fl, b->Estat, nullptr, nullptr);
         BTRY(blaunch(b, "static field"));
         BTRY((structure_factor<0, 0>(b, nullptr, nullptr)));
         BTRY((kfield<0, 1, 1>(b, nullptr, b->Estat, nullptr)));
@@ -1860,9 +1938,9 @@ int forward_launches(mdff_batch* b, bool captured) {
             BCK(cudaMemsetAsync(b->mu, 0, sizeof(double) * 3 * N, b->st));
         }
         // final multipole Ewald: forces, energy, stress
-        k_b_dir<16, 2><<<dir_blocks(N, 16), 256, 0, b->st>>>(N, b->cfg_of, b->cfg, nullptr, b->sx, b->sy, b->sz, b->type,
-                                                             b->q, b->mu, b->nbr, b->cnt, b->cap, b->pc, b->fl, b->fdir,
-                                                             b->e_dir, b->s_dir);
+        k_b_records<<<nblk(N, 256), 256, 0, b->st>>>(N, b->mu, b->mrec);
+        k_b_dir<16, 2><<<dir_blocks(N, 16), 256, 0, b->st>>>(N, b->cfg_of, b->cfg, b->rec, b->mrec, b->nbr, b->cnt,
+                                                             b->cap, b->pc, b->fl, b->fdir, b->e_dir, b->s_dir);
         BTRY(blaunch(b, "final real space"));
         BTRY((structure_factor<2, 1>(b, nullptr, b->mu)));
         BTRY((kfield<1, 0, 1>(b, nullptr, b->Erec, b->G)));
@@ -2044,8 +2122,9 @@ int loss_grad_launches(mdff_batch* b, bool with_grad) {
     const int blk16 = dir_blocks(N, 16);
     if (p.lcoulomb && any_polarisable(b)) {
         // adjoint right-hand side h = dJ/dmu
-        k_b_dir_adj<16><<<blk16, 256, 0, b->st>>>(N, b->cfg_of, b->cfg, b->sx, b->sy, b->sz, b->type, b->q, b->mu, b->R,
-                                                  b->Sres, b->nbr, b->cnt, b->cap, b->pc, b->fl, b->h, b->gpart);
+        k_b_records<<<nblk(N, 256), 256, 0, b->st>>>(N, b->R, b->rrec);   // (mrec: the forward pass's final dipoles)
+        k_b_dir_adj<16><<<blk16, 256, 0, b->st>>>(N, b->cfg_of, b->cfg, b->rec, b->mrec, b->rrec, b->Sres, b->nbr,
+                                                  b->cnt, b->cap, b->pc, b->fl, b->h, b->gpart);
         k_b_reduce_cols<<<nblk(KA, 8), 256, 0, b->st>>>(b->gpart, blk16, KA, b->gsum);
         BTRY(blaunch(b, "adjoint real space"));
         BTRY((structure_factor<3, 2>(b, nullptr, b->mu)));
@@ -2060,8 +2139,8 @@ int loss_grad_launches(mdff_batch* b, bool with_grad) {
     } else {
         BCK(cudaMemsetAsync(b->lam, 0, sizeof(double) * 3 * N, b->st));
     }
-    k_b_grad_rows<16><<<blk16, 256, 0, b->st>>>(N, b->cfg_of, b->cfg, b->sx, b->sy, b->sz, b->type, b->q, b->R, b->Sres,
-                                                b->lam, b->nbr, b->cnt, b->cap, b->pc, b->fl, b->gpart);
+    k_b_grad_rows<16><<<blk16, 256, 0, b->st>>>(N, b->cfg_of, b->cfg, b->rec, b->R, b->Sres, b->lam, b->nbr, b->cnt,
+                                                b->cap, b->pc, b->fl, b->gpart);
     k_b_reduce_cols<<<nblk(KR, 8), 256, 0, b->st>>>(b->gpart, blk16, KR, b->gsum + KA);
     return blaunch(b, "row gradient");
 }
@@ -2209,6 +2288,12 @@ int mdff_batch_create(const mdff_params* p, int nconf, const int* natm, const in
         C.n = natm[c];
         off += natm[c];
         C.rc2 = rc[c] * rc[c];
+        // the short pair vectors where no pair inside the cutoff has two images
+        // equally far (rounding of the coordinates: 1e-15 of a width)
+        const double* A9 = C.cell.A;
+        C.geom = !(2.0 * rc[c] < std::min(W[0], std::min(W[1], W[2])) * (1.0 - 1e-12)) ? GEOM_EXACT
+                 : A9[1] == 0.0 && A9[2] == 0.0 && A9[3] == 0.0 && A9[5] == 0.0 && A9[6] == 0.0 && A9[7] == 0.0
+                     ? GEOM_DIAGONAL : GEOM_GENERAL;
         C.alpha = alpha[c];
         C.selfa = alpha[c] / std::sqrt(PI);
         C.selfa2 = 2.0 * C.selfa * alpha[c] * alpha[c] / 3.0;
@@ -2287,6 +2372,7 @@ int mdff_batch_create(const mdff_params* p, int nconf, const int* natm, const in
     for (double** v : {&b->f, &b->fpair, &b->fdir, &b->Erec, &b->Estat, &b->mu, &b->Eind, &b->cg_r, &b->cg_z, &b->cg_d,
                        &b->cg_Ad, &b->h, &b->lam, &b->R, &b->ft})
         A(v, 3 * N);
+    for (double4** v : {&b->rec, &b->mrec, &b->rrec}) A(v, N);
     A(&b->G, 6 * N);
     A(&b->s_pair, 6 * N);
     A(&b->s_dir, 6 * N);
@@ -2357,7 +2443,8 @@ int mdff_batch_create(const mdff_params* p, int nconf, const int* natm, const in
     b->tau_t.assign((size_t)9 * nconf, 0.0);
     b->tau.assign((size_t)9 * nconf, 0.0);
     if (int r2 = upload_params(b, *p)) return bad(r2);
-    k_b_wrap_frac<<<nblk(N, 256), 256, 0, b->st>>>(b->N, b->cfg_of, b->cfg, b->x, b->y, b->z, b->sx, b->sy, b->sz);
+    k_b_wrap_frac<<<nblk(N, 256), 256, 0, b->st>>>(b->N, b->cfg_of, b->cfg, b->x, b->y, b->z, b->type,
+                                                   b->sx, b->sy, b->sz, b->rec);
     if (int r2 = blaunch(b, "wrap")) return bad(r2);
     // neighbour rows (no skin: the positions of a batch do not move)
     int cap = p->nlist_capacity > 0 ? p->nlist_capacity : cap_est;

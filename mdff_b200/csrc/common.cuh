@@ -148,6 +148,41 @@ __device__ __forceinline__ void tt_damp_d(double b, double c, double r, int k, d
     fd = term * inv * e * b;
 }
 
+// A BMH pair at distance d = 1/dm1, ftd: with Tang-Toennies damping of orders 6 and
+// 8 (tt_damp_d with c = 1; one exponential and one series for both).  Returns
+// -(du/dr)/r; u: the pair's energy.
+__device__ __forceinline__ double bmh_pair(bool ftd, double A, double B, double C, double D, double BD, double d,
+                                           double dm1, double& u) {
+    constexpr InvFact IF;
+    const double ir2 = dm1 * dm1, erh = A * exp(-B * d);
+    double ir6 = ir2 * ir2 * ir2;
+    double ir8 = ir6 * ir2;
+    ir6 *= C;
+    ir8 *= D;
+    double w0 = B * erh;
+    if (ftd) {
+        const double br = BD * d, e = exp(-br), e1 = e * BD;
+        double term = 1.0, sum = 1.0;
+#pragma unroll
+        for (int q = 1; q <= 6; ++q) {
+            term *= br;
+            sum = fma(term, IF.v[q], sum);
+        }
+        const double f6 = 1.0 - sum * e;
+        w0 = fma(ir6, term * IF.v[6] * e1, w0);
+        term *= br;
+        sum = fma(term, IF.v[7], sum);
+        term *= br;
+        sum = fma(term, IF.v[8], sum);
+        const double f8 = 1.0 - sum * e;
+        w0 = fma(ir8, term * IF.v[8] * e1, w0);
+        ir6 *= f6;
+        ir8 *= f8;
+    }
+    u = erh - (ir6 + ir8);
+    return fma(-(6.0 * ir6 + 8.0 * ir8), dm1, w0) * dm1;
+}
+
 // Packed two-lane FP32 arithmetic of sm_100 (add / mul / fma .rn.f32x2): a
 // 64-bit register holds the pair (lo, hi).
 typedef unsigned long long f2p;

@@ -40,7 +40,6 @@ template <int G, int KIND>
 __global__ void __launch_bounds__(256, KIND == 0 ? 4 : 3)
     k_pair1(int n, const double4* __restrict__ rec, CellP c, const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
             const PairConst* __restrict__ pc, PairFlags fl, double* fx, double* fy, double* fz, double* part) {
-    constexpr InvFact IF;
     const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
     const int sub = threadIdx.x & (G - 1);
     const bool active = gid < n;
@@ -74,37 +73,10 @@ __global__ void __launch_bounds__(256, KIND == 0 ? 4 : 3)
                 ue += u;
             } else {
                 if (P.A == 0.0) continue;
-                const double dm1 = rsqrt(rsq), d = rsq * dm1, ir2 = dm1 * dm1;
-                const double erh = P.A * exp(-P.B * d);
-                double ir6 = ir2 * ir2 * ir2;
-                double ir8 = ir6 * ir2;
-                ir6 *= P.C;
-                ir8 *= P.D;
-                double w0 = P.B * erh, i68 = ir6 + ir8, i6d = 6.0 * ir6, i8d = 8.0 * ir8;
-                if (KIND == 2) {   // Tang-Toennies damping of orders 6 and 8 (tt_damp_d with c = 1)
-                    const double br = P.BD * d, e = exp(-br), e1 = e * P.BD;
-                    double term = 1.0, sum = 1.0;
-#pragma unroll
-                    for (int q = 1; q <= 6; ++q) {
-                        term *= br;
-                        sum = fma(term, IF.v[q], sum);
-                    }
-                    const double f6 = 1.0 - sum * e;
-                    w0 = fma(ir6, term * IF.v[6] * e1, w0);
-                    term *= br;
-                    sum = fma(term, IF.v[7], sum);
-                    term *= br;
-                    sum = fma(term, IF.v[8], sum);
-                    const double f8 = 1.0 - sum * e;
-                    w0 = fma(ir8, term * IF.v[8] * e1, w0);
-                    ir6 *= f6;
-                    ir8 *= f8;
-                    i68 = ir6 + ir8;
-                    i6d = 6.0 * ir6;
-                    i8d = 8.0 * ir8;
-                }
-                w = fma(-(i6d + i8d), dm1, w0) * dm1;
-                ue += erh - i68;
+                const double dm1 = rsqrt(rsq);
+                double ub;
+                w = bmh_pair(KIND == 2, P.A, P.B, P.C, P.D, P.BD, rsq * dm1, dm1, ub);
+                ue += ub;
             }
             f0 = fma(w, rx, f0);
             f1 = fma(w, ry, f1);
