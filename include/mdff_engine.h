@@ -353,6 +353,10 @@ int  mdff_set_positions(mdff_ctx* ctx, const double* rx, const double* ry, const
 /* Wrapped positions as the engine holds them. */
 int  mdff_get_positions(mdff_ctx* ctx, double* rx, double* ry, double* rz);
 
+/* Positions and forces as (n, 3) arrays, (x, y, z) of an atom in a row; either
+ * may be NULL. */
+int  mdff_get_state(mdff_ctx* ctx, double* pos, double* force);
+
 /* Current velocities (internal units). */
 int  mdff_get_velocities(mdff_ctx* ctx, double* vx, double* vy, double* vz);
 

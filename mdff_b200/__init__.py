@@ -58,6 +58,7 @@ def lib():
         L.mdff_rmc_efg.argtypes = [vp, C.POINTER(abi.RmcParams), C.POINTER(abi.RmcEfgParams), dp, dp, dp, dp, dp,
                                    C.c_longlong, C.c_ulonglong, dp, dp, dp, dp, C.POINTER(abi.RmcResult)]
         L.mdff_get_positions.argtypes = [vp, dp, dp, dp]
+        L.mdff_get_state.argtypes = [vp, dp, dp]
         L.mdff_engforce.argtypes = [vp, dp, dp, dp, C.POINTER(abi.Energies), dp, dp, dp, dp, dp]
         L.mdff_nlist_build.argtypes = [vp]
         L.mdff_nlist_get.argtypes = [vp, C.c_int, ip, ip, C.c_int, ip]
@@ -212,9 +213,9 @@ class Engine:
             pass
 
     def positions(self):
-        r = [np.empty(self.n) for _ in range(3)]
-        self._check(lib().mdff_get_positions(self._h, *(_dp(a) for a in r)))
-        return np.stack(r, axis=1)
+        pos = np.empty((self.n, 3))
+        self._check(lib().mdff_get_state(self._h, _dp(pos), None))
+        return pos
 
     def gr(self, cut, res):
         """g(r) of the current positions as rmc_gr forms it: [npairs+1][nbins]
@@ -488,19 +489,16 @@ class Engine:
     def step(self, nsteps, thermo=True):
         """Advance nsteps; return final positions, velocities, forces and the
         per-step thermodynamics."""
-        n = self.n
-        r = [np.empty(n) for _ in range(3)]
-        v = [np.empty(n) for _ in range(3)]
-        f = [np.empty(n) for _ in range(3)]
         th = (abi.Thermo * max(nsteps, 1))() if thermo else None
         # no upload (NULL position/velocity inputs would skip the download too),
         # so advance first, then read the state back
-        self._check(lib().mdff_step(self._h, nsteps, None, None, None, None, None, None, *(_dp(a) for a in f),
+        self._check(lib().mdff_step(self._h, nsteps, None, None, None, None, None, None, None, None, None,
                                     th if thermo else None))
-        pos = self.positions()
+        pos, f = np.empty((2, self.n, 3))   # (one block: fewer page faults)
+        self._check(lib().mdff_get_state(self._h, _dp(pos), _dp(f)))
         return {
             "pos": pos,
-            "f": np.stack(f, axis=1),
+            "f": f,
             "thermo": [th[i].as_dict() for i in range(nsteps)] if thermo else [],
         }
 

@@ -12,6 +12,16 @@ namespace mdff {
 
 constexpr int IB = 256;
 
+// (x, y, z) of each atom in a row
+__global__ void k_aos3(int n, const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
+                       double* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    out[3 * (size_t)i] = x[i];
+    out[3 * (size_t)i + 1] = y[i];
+    out[3 * (size_t)i + 2] = z[i];
+}
+
 // r += v dt + f dt^2/2 / m ; fold = f
 __global__ void k_vv_positions(int n, double* x, double* y, double* z, const double* vx, const double* vy,
                                const double* vz, const double* fx, const double* fy, const double* fz,
