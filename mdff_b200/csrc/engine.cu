@@ -230,14 +230,24 @@ int check_launch(mdff_ctx* ctx, const char* where) {
     return MDFF_OK;
 }
 
-int sync_scalars(mdff_ctx* ctx) {
+int copy_scalars(mdff_ctx* ctx) {
     CK(cudaMemcpyAsync(ctx->hsc, ctx->dsc, sizeof(DevScalars), cudaMemcpyDeviceToHost, ctx->st));
+    return MDFF_OK;
+}
+
+// after copy_scalars
+int wait_scalars(mdff_ctx* ctx) {
     CK(cudaStreamSynchronize(ctx->st));
     ctx->prof.harvest();
     if (ctx->hsc->tc_err)
         return fail(ctx, MDFF_E_CUDA, "tensor-core structure factor: a pipeline wait gave up (code " +
                                           std::to_string(ctx->hsc->tc_err) + ")");
     return MDFF_OK;
+}
+
+int sync_scalars(mdff_ctx* ctx) {
+    TRY(copy_scalars(ctx));
+    return wait_scalars(ctx);
 }
 
 // lattice (src/lattice.f90:60-175) on the host, for A given column-major.
@@ -1050,12 +1060,16 @@ int engforce_device(mdff_ctx* ctx) {
     const int n = ctx->n;
     const mdff_params& p = ctx->p;
     const bool efg = p.doefg && ctx->efg_due;
+    const bool built = !p.lvnlist || !ctx->have_list;
     if (!p.lvnlist) TRY(build_lists(ctx, 0.0));
     else if (!ctx->have_list) TRY(build_lists(ctx, p.skindiff));   // lists dropped (an interrupted RMC chain)
-    ctx->prof.begin(PK_OTHER);
-    k_frac_rec<<<nb(n), 256, 0, ctx->st>>>(n, ctx->x, ctx->y, ctx->z, ctx->type, ctx->cell, ctx->sx, ctx->sy, ctx->sz,
-                                           ctx->rec);
-    ctx->prof.end(1);
+    if (!(ctx->rec_fresh && p.lvnlist && !built)) {
+        ctx->prof.begin(PK_OTHER);
+        k_frac_rec<<<nb(n), 256, 0, ctx->st>>>(n, ctx->x, ctx->y, ctx->z, ctx->type, ctx->cell, ctx->sx, ctx->sy,
+                                               ctx->sz, ctx->rec);
+        ctx->prof.end(1);
+    }
+    ctx->rec_fresh = false;
     ctx->rs.want_epoch++;   // positions may have changed: rebuild the phase tables
     if (p.autotune && !ctx->tuned) TRY(autotune(ctx));
     std::memset(&ctx->en, 0, sizeof ctx->en);
@@ -1067,9 +1081,9 @@ int engforce_device(mdff_ctx* ctx) {
         PairFlags fl{p.lnmlj, p.lbmhft, p.lbmhftd, p.lmorse, p.trunc, ctx->ntype, lj126, geom_of(ctx),
                      p.precision == MDFF_PREC_FP64};
         ctx->prof.begin(PK_PAIR);
-        launch_pair(ctx->st, n, ctx->rec, ctx->cell, ctx->lv, ctx->pc, fl, ctx->fx, ctx->fy,
-                    ctx->fz, ctx->part, ctx->dsc);
-        ctx->prof.end(2);
+        ctx->pair_blocks = launch_pair(ctx->st, n, ctx->rec, ctx->cell, ctx->lv, ctx->pc, fl, ctx->fx, ctx->fy, ctx->fz,
+                                       ctx->part, ctx->dsc, !ctx->defer_pair);
+        ctx->prof.end(ctx->defer_pair ? 1 : 2);
     } else {
         CK(cudaMemsetAsync(ctx->fx, 0, sizeof(double) * n, ctx->st));
         CK(cudaMemsetAsync(ctx->fy, 0, sizeof(double) * n, ctx->st));
@@ -1077,8 +1091,8 @@ int engforce_device(mdff_ctx* ctx) {
         CK(cudaMemsetAsync(ctx->dsc->nonb, 0, sizeof(double) * 12, ctx->st));
     }
     TRY(check_launch(ctx, "pair"));
-    CK(cudaMemsetAsync(ctx->dsc->upol, 0, sizeof(double) * 2, ctx->st));
     if (p.lcoulomb) {
+        CK(cudaMemsetAsync(ctx->dsc->upol, 0, sizeof(double) * 2, ctx->st));
         const int n3 = 3 * n;
         if (ctx->npol > 0) {
             TRY(solve_dipoles(ctx));
@@ -1530,15 +1544,28 @@ int md_launches(mdff_ctx* ctx) {
     } else if (p.integrator == MDFF_NVE_VV) {
         ctx->prof.begin(PK_INTEGRATE);
         k_vv_positions<<<nb(n), 256, 0, ctx->st>>>(n, ctx->x, ctx->y, ctx->z, ctx->vx, ctx->vy, ctx->vz, ctx->fx, ctx->fy,
-                                                   ctx->fz, ctx->fox, ctx->foy, ctx->foz, ctx->mass, dt);
+                                                   ctx->fz, ctx->fox, ctx->foy, ctx->foz, ctx->mass, dt, ctx->type,
+                                                   ctx->cell, ctx->sx, ctx->sy, ctx->sz, ctx->rec);
         ctx->prof.end(1);
         TRY(check_launch(ctx, "vv_positions"));
-        TRY(engforce_device(ctx));
+        ctx->rec_fresh = true;
+        // in a captured step the host reads the pair sums after the step, and without
+        // Coulomb interactions nothing else uses the partials before its end
+        const bool nonb = p.lnmlj || p.lbmhft || p.lbmhftd || p.lmorse;
+        ctx->defer_pair = ctx->capturing && !p.lcoulomb && nonb;
+        const int rc = engforce_device(ctx);
+        const int npair = ctx->defer_pair ? ctx->pair_blocks : 0;
+        ctx->defer_pair = false;
+        TRY(rc);
+        double* kpart = ctx->part2;
+        double* spart = p.lvnlist ? ctx->part2 + nb(n) : nullptr;
         ctx->prof.begin(PK_INTEGRATE);
         k_vv_velocities<<<nb(n), 256, 0, ctx->st>>>(n, ctx->vx, ctx->vy, ctx->vz, ctx->fx, ctx->fy, ctx->fz, ctx->fox,
-                                                    ctx->foy, ctx->foz, ctx->mass, dt, ctx->part.buf);
-        launch_reduce_partials(ctx->st, ctx->part.buf, nb(n), 1, ctx->dsc->ke2, 0);
+                                                    ctx->foy, ctx->foz, ctx->mass, dt, ctx->sx, ctx->sy, ctx->sz,
+                                                    ctx->xs, ctx->ys, ctx->zs, ctx->cell, kpart, spart);
+        k_step_sums<<<1, 14 * 32, 0, ctx->st>>>(npair, ctx->part.buf, nb(n), kpart, spart, skin_allowance(ctx), ctx->dsc);
         ctx->prof.end(2);
+        return check_launch(ctx, "step");
     } else {
         // nhcn (src/integration.f90:476-558) or nhc2 (:205-254): chain half,
         // prop_pos_vel_verlet, chain half; only the chain kernel differs
@@ -1556,9 +1583,11 @@ int md_launches(mdff_ctx* ctx) {
         TRY(ke_reduce(ctx, 1));
         ctx->prof.begin(PK_INTEGRATE);
         k_kick_drift<<<nb(n), 256, 0, ctx->st>>>(n, ctx->x, ctx->y, ctx->z, ctx->vx, ctx->vy, ctx->vz, ctx->fx, ctx->fy,
-                                                 ctx->fz, ctx->mass, dt);
+                                                 ctx->fz, ctx->mass, dt, ctx->type, ctx->cell, ctx->sx, ctx->sy, ctx->sz,
+                                                 ctx->rec);
         ctx->prof.end(1);
         TRY(check_launch(ctx, "kick_drift"));
+        ctx->rec_fresh = true;
         TRY(engforce_device(ctx));
         ctx->prof.begin(PK_INTEGRATE);
         k_kick<<<nb(n), 256, 0, ctx->st>>>(n, ctx->vx, ctx->vy, ctx->vz, ctx->fx, ctx->fy, ctx->fz, ctx->mass, dt,
@@ -1670,6 +1699,7 @@ int capture_step(mdff_ctx* ctx, int slot, const StepKey& key) {
         rc = fail(ctx, MDFF_E_CUDA, std::string("capture of the MD step: ") + cudaGetErrorString(e));
     } else {
         rc = md_launches(ctx);
+        if (rc == MDFF_OK) rc = copy_scalars(ctx);
         cudaError_t e2 = cudaStreamEndCapture(ctx->st, &g);
         if (rc == MDFF_OK && e2 != cudaSuccess)
             rc = fail(ctx, MDFF_E_CUDA, std::string("capture of the MD step: ") + cudaGetErrorString(e2));
@@ -1711,7 +1741,7 @@ int md_step_graph(mdff_ctx* ctx) {
     }
     CK(cudaGraphLaunch(ctx->gexec[slot], ctx->st));
     ctx->nstep_graph++;
-    TRY(sync_scalars(ctx));
+    TRY(wait_scalars(ctx));   // (the step's last node copies the scalars)
     const bool pcg = ctx->gbody[slot] > 0;
     ctx->prof.launches += ctx->glaunch[slot] + (pcg ? ctx->gbody[slot] * (long)ctx->hsc->iter : 0);
     if (pcg) {
@@ -3162,6 +3192,8 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
     TRY(dalloc(ctx, &ctx->coef, PLAN_LEN));
     TRY(dalloc(ctx, &ctx->type, n));
     TRY(dalloc(ctx, &ctx->rec, n));
+    TRY(dalloc(ctx, &ctx->aos, 6 * (size_t)n));
+    TRY(dalloc(ctx, &ctx->part2, 3 * (size_t)nb(n)));
     TRY(dalloc(ctx, &ctx->mrec, n));
     TRY(dalloc(ctx, &ctx->pc, NT * NT));
     TRY(dalloc(ctx, &ctx->dsc, 1));
@@ -3192,8 +3224,6 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
     if (p.lcoulomb) {
         KGrid& kg = ctx->kg;
         for (int d = 0; d < 3; ++d) kg.kmax[d] = ctx->kES[d];
-    TRY(dalloc(ctx, &ctx->aos, 6 * (size_t)n));
-    TRY(dalloc(ctx, &ctx->part2, 3 * (size_t)nb(n)));
         kg.ncol = (kg.kmax[0] + 1) * (2 * kg.kmax[1] + 1);
         kg.nzl = 2 * kg.kmax[2] + 1;
         kg.nrect = kg.ncol * kg.nzl;
@@ -3583,6 +3613,25 @@ int mdff_get_positions(mdff_ctx* ctx, double* rx, double* ry, double* rz) {
     return MDFF_OK;
 }
 
+// (x, y, z) per atom, as the caller's (n, 3) arrays hold them: transposed on the
+// device and copied whole (in one piece where force follows pos), where a copy of
+// each component and a transposition on the host took 1.2 ms
+// more (108 000 atoms, both: 0.33 ms).
+int mdff_get_state(mdff_ctx* ctx, double* pos, double* force) {
+    if (!ctx || !ctx->have_system) return ctx ? fail(ctx, MDFF_E_STATE, "set_system first") : MDFF_E_STATE;
+    cudaSetDevice(ctx->p.device);
+    const size_t n3 = 3 * (size_t)ctx->n;
+    if (pos) k_aos3<<<nb(ctx->n), 256, 0, ctx->st>>>(ctx->n, ctx->x, ctx->y, ctx->z, ctx->aos);
+    if (force) k_aos3<<<nb(ctx->n), 256, 0, ctx->st>>>(ctx->n, ctx->fx, ctx->fy, ctx->fz, ctx->aos + n3);
+    TRY(check_launch(ctx, "get_state"));
+    const bool whole = pos && force == pos + n3;
+    if (pos) CK(cudaMemcpyAsync(pos, ctx->aos, sizeof(double) * (whole ? 2 * n3 : n3), cudaMemcpyDeviceToHost, ctx->st));
+    if (force && !whole)
+        CK(cudaMemcpyAsync(force, ctx->aos + n3, sizeof(double) * n3, cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaStreamSynchronize(ctx->st));
+    return MDFF_OK;
+}
+
 int mdff_nlist_build(mdff_ctx* ctx) {
     if (!ctx || !ctx->have_system) return ctx ? fail(ctx, MDFF_E_STATE, "set_system first") : MDFF_E_STATE;
     cudaSetDevice(ctx->p.device);
@@ -3613,25 +3662,6 @@ int mdff_nlist_get(mdff_ctx* ctx, int which, int* point, int* list, int cap, int
     int total = 0;
     std::vector<int> row;
     for (int i = 0; i < n; ++i) {
-// (x, y, z) per atom, as the caller's (n, 3) arrays hold them: transposed on the
-// device and copied whole (in one piece where force follows pos), where a copy of
-// each component and a transposition on the host took 1.2 ms
-// more (108 000 atoms, both: 0.33 ms).
-int mdff_get_state(mdff_ctx* ctx, double* pos, double* force) {
-    if (!ctx || !ctx->have_system) return ctx ? fail(ctx, MDFF_E_STATE, "set_system first") : MDFF_E_STATE;
-    cudaSetDevice(ctx->p.device);
-    const size_t n3 = 3 * (size_t)ctx->n;
-    if (pos) k_aos3<<<nb(ctx->n), 256, 0, ctx->st>>>(ctx->n, ctx->x, ctx->y, ctx->z, ctx->aos);
-    if (force) k_aos3<<<nb(ctx->n), 256, 0, ctx->st>>>(ctx->n, ctx->fx, ctx->fy, ctx->fz, ctx->aos + n3);
-    TRY(check_launch(ctx, "get_state"));
-    const bool whole = pos && force == pos + n3;
-    if (pos) CK(cudaMemcpyAsync(pos, ctx->aos, sizeof(double) * (whole ? 2 * n3 : n3), cudaMemcpyDeviceToHost, ctx->st));
-    if (force && !whole)
-        CK(cudaMemcpyAsync(force, ctx->aos + n3, sizeof(double) * n3, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    return MDFF_OK;
-}
-
         point[i] = total + 1;
         row.clear();
         const int I = i + 1;

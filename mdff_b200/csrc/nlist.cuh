@@ -29,17 +29,21 @@ void launch_frac(cudaStream_t st, int n, const double* x, const double* y, const
 
 // The same with the record (fractional coordinates, type as bits) that the pair
 // kernels gather.
+__device__ __forceinline__ void frac_record(int i, double X, double Y, double Z, int type, const CellP& c, double* sx,
+                                            double* sy, double* sz, double4* rec) {
+    const double a = __dadd_rn(__dadd_rn(__dmul_rn(X, c.B[0]), __dmul_rn(Y, c.B[3])), __dmul_rn(Z, c.B[6]));
+    const double b = __dadd_rn(__dadd_rn(__dmul_rn(X, c.B[1]), __dmul_rn(Y, c.B[4])), __dmul_rn(Z, c.B[7]));
+    const double d = __dadd_rn(__dadd_rn(__dmul_rn(X, c.B[2]), __dmul_rn(Y, c.B[5])), __dmul_rn(Z, c.B[8]));
+    sx[i] = a; sy[i] = b; sz[i] = d;
+    rec[i] = make_double4(a, b, d, __longlong_as_double((long long)type));
+}
+
 __global__ void k_frac_rec(int n, const double* __restrict__ x, const double* __restrict__ y,
                            const double* __restrict__ z, const int* __restrict__ type, CellP c, double* sx, double* sy,
                            double* sz, double4* rec) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    double X = x[i], Y = y[i], Z = z[i];
-    const double a = __dadd_rn(__dadd_rn(__dmul_rn(X, c.B[0]), __dmul_rn(Y, c.B[3])), __dmul_rn(Z, c.B[6]));
-    const double b = __dadd_rn(__dadd_rn(__dmul_rn(X, c.B[1]), __dmul_rn(Y, c.B[4])), __dmul_rn(Z, c.B[7]));
-    const double d = __dadd_rn(__dadd_rn(__dmul_rn(X, c.B[2]), __dmul_rn(Y, c.B[5])), __dmul_rn(Z, c.B[8]));
-    sx[i] = a; sy[i] = b; sz[i] = d;
-    rec[i] = make_double4(a, b, d, __longlong_as_double((long long)type[i]));
+    frac_record(i, x[i], y[i], z[i], type[i], c, sx, sy, sz, rec);
 }
 
 // read_pos.f90:148-150: kardir, periodicbc (x - NINT(x)), dirkar, in place.
@@ -345,16 +349,14 @@ __device__ __forceinline__ void top2_merge(double& a1, double& a2, double b1, do
     else a2 = fmax(a2, b1);
 }
 
-__global__ void k_skin_partial(int n, const double* sx, const double* sy, const double* sz, const double* xs,
-                               const double* ys, const double* zs, CellP c, double* part) {
-    double m1 = 0.0, m2 = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double rx, ry, rz;
-        double d2 = pairvec_exact(c, sx[i], sy[i], sz[i], xs[i], ys[i], zs[i], rx, ry, rz);
-        double d = sqrt(d2);
-        if (d > m1) { m2 = m1; m1 = d; }
-        else if (d > m2) m2 = d;
-    }
+__device__ __forceinline__ double skin_distance(const CellP& c, double s1, double s2, double s3, double x1, double x2,
+                                                double x3) {
+    double rx, ry, rz;
+    return sqrt(pairvec_exact(c, s1, s2, s3, x1, x2, x3, rx, ry, rz));
+}
+
+// the block's two largest of its threads' (m1 >= m2) into part[2 block]
+__device__ __forceinline__ void skin_block(double m1, double m2, double* part) {
     for (int o = 16; o > 0; o >>= 1) {
         double b1 = __shfl_xor_sync(0xffffffffu, m1, o), b2 = __shfl_xor_sync(0xffffffffu, m2, o);
         top2_merge(m1, m2, b1, b2);
@@ -375,18 +377,36 @@ __global__ void k_skin_partial(int n, const double* sx, const double* sy, const 
     }
 }
 
-__global__ void k_skin_final(int nblocks, const double* part, double skindiff, DevScalars* d) {
+__global__ void k_skin_partial(int n, const double* sx, const double* sy, const double* sz, const double* xs,
+                               const double* ys, const double* zs, CellP c, double* part) {
     double m1 = 0.0, m2 = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += 32) top2_merge(m1, m2, part[2 * b], part[2 * b + 1]);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double d = skin_distance(c, sx[i], sy[i], sz[i], xs[i], ys[i], zs[i]);
+        if (d > m1) { m2 = m1; m1 = d; }
+        else if (d > m2) m2 = d;
+    }
+    skin_block(m1, m2, part);
+}
+
+// one warp
+__device__ __forceinline__ void skin_finish(int nblocks, const double* __restrict__ part, double skindiff, DevScalars* d) {
+    const int lane = threadIdx.x & 31;
+    double m1 = 0.0, m2 = 0.0;
+#pragma unroll 4
+    for (int b = lane; b < nblocks; b += 32) top2_merge(m1, m2, part[2 * b], part[2 * b + 1]);
     for (int o = 16; o > 0; o >>= 1) {
         double b1 = __shfl_xor_sync(0xffffffffu, m1, o), b2 = __shfl_xor_sync(0xffffffffu, m2, o);
         top2_merge(m1, m2, b1, b2);
     }
-    if (threadIdx.x == 0) {
+    if (lane == 0) {
         d->dmax1 = m1;
         d->dmax2 = m2;
         d->rebuild = (m1 + m2 > skindiff) ? 1 : 0;
     }
+}
+
+__global__ void k_skin_final(int nblocks, const double* part, double skindiff, DevScalars* d) {
+    skin_finish(nblocks, part, skindiff, d);
 }
 
 void launch_skin_check(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz,

@@ -200,8 +200,8 @@ __global__ void __launch_bounds__(256) k_pair(int n, const double4* __restrict__
     block_partials<12>(v, part);
 }
 
-void launch_pair(cudaStream_t st, int n, const double4* rec, CellP c, const NList& l, const PairConst* pc, PairFlags fl, double* fx, double* fy, double* fz,
-                 Partials& part, DevScalars* d) {
+int launch_pair(cudaStream_t st, int n, const double4* rec, CellP c, const NList& l, const PairConst* pc, PairFlags fl,
+                double* fx, double* fy, double* fz, Partials& part, DevScalars* d, bool sum) {
     const int threads = 256;
     auto grid = [&](int g) { return (int)(((size_t)n * g + threads - 1) / threads); };
     int blocks;
@@ -222,7 +222,8 @@ void launch_pair(cudaStream_t st, int n, const double4* rec, CellP c, const NLis
     }
 #undef PAIR1
     // u_lj vir_lj u_bmh vir_bmh u_mor vir_mor, then the stress sums
-    launch_reduce_partials(st, part.buf, blocks, 12, d->nonb, 0);
+    if (sum) launch_reduce_partials(st, part.buf, blocks, 12, d->nonb, 0);
+    return blocks;
 }
 
 }  // namespace mdff

@@ -18,6 +18,7 @@ __global__ void k_reduce_partials(const double* __restrict__ buf, int nblocks, i
     const int lane = threadIdx.x & 31;
     if (k >= K) return;
     double s = 0.0;
+#pragma unroll 8   // the loads together, the additions in order
     for (int b = lane; b < nblocks; b += 32) s += buf[(size_t)b * K + k];
     s = warp_sum(s);
     if (lane == 0) out[k] = accumulate ? out[k] + s : s;
@@ -62,6 +63,7 @@ __global__ void k_cg_init(int n, const double* __restrict__ b, const double* __r
 __device__ __forceinline__ double warp_reduce_partials(const double* __restrict__ buf, int nblocks, int K, int k) {
     const int lane = threadIdx.x & 31;
     double s = 0.0;
+#pragma unroll 8   // the loads together, the additions in order
     for (int b = lane; b < nblocks; b += 32) s += buf[(size_t)b * K + k];
     return warp_sum(s);
 }

@@ -1,4 +1,7 @@
-"""Reading a state back.  Exact: the same bytes through either entry point."""
+"""Reading a state back, and the captured step's kernels against the plain ones.
+
+Exact: a copied state is the same bytes through either entry point; a captured step does
+the arithmetic of the plain one, in the same order."""
 import ctypes as C
 
 import numpy as np
@@ -40,3 +43,15 @@ def test_state(n):
     assert np.array_equal(r["pos"], np.stack(xyz, axis=1)) and np.array_equal(r["f"], np.stack(f, axis=1))
     assert np.array_equal(e.positions(), r["pos"])
     assert r["pos"].flags.c_contiguous and r["f"].flags.c_contiguous
+
+
+@pytest.mark.parametrize("integrator", [abi.NVE_VV, abi.NVT_NHCN])
+@pytest.mark.parametrize("n", [200, 500, 30000])
+def test_captured_step_is_the_plain_one(n, integrator):
+    s = argon(n, integrator)
+    a, b = engine(s), engine(s)
+    b.enable_profile(True)   # profiled steps run as plain launches
+    ra, rb = a.step(12), b.step(12)
+    assert np.array_equal(ra["pos"], rb["pos"]) and np.array_equal(ra["f"], rb["f"])
+    assert ra["thermo"] == rb["thermo"]
+    assert any(t["nlist_rebuilt"] for t in a.step(40)["thermo"])
