@@ -1,8 +1,7 @@
 // EFG post-processing on the device: efg_stat (src/efg.f90:2057-2440) with
 // nmr_convention (:2546-2650) over a batch of configurations in one pass.
 // Per site: the Czjzek components U of the tensor and S = |U|, the principal
-// values from a cyclic Jacobi iteration in FP64 (ascending, as DSYEV returns
-// them), ordered by the NMR convention |Vzz| >= |Vyy| >= |Vxx| with
+// values in FP64 (sym3_eigvals; ascending, as DSYEV returns them), ordered by the NMR convention |Vzz| >= |Vyy| >= |Vxx| with
 // eta = (Vxx - Vyy) / Vzz; then, in the same kernel, the site's bins of the
 // Vzz, eta, U and S distributions (block-private shared-memory counts flushed
 // with integer atomics: exact and order-free) and its contribution to the
@@ -13,8 +12,9 @@
 
 namespace mdff {
 
-// principal values of the symmetric 3x3 (a00 a11 a22 a01 a02 a12), ascending
-__device__ __forceinline__ void sym3_eigvals(double a00, double a11, double a22, double a01, double a02, double a12,
+// principal values of the symmetric 3x3 (a00 a11 a22 a01 a02 a12), ascending, by
+// cyclic Jacobi rotations
+__device__ __noinline__ void sym3_jacobi(double a00, double a11, double a22, double a01, double a02, double a12,
                                              double w[3]) {
     double d0 = a00, d1 = a11, d2 = a22, o01 = a01, o02 = a02, o12 = a12;
     const double nrm = fabs(a00) + fabs(a11) + fabs(a22) + fabs(a01) + fabs(a02) + fabs(a12);
@@ -49,6 +49,76 @@ __device__ __forceinline__ void sym3_eigvals(double a00, double a11, double a22,
     if (y > z) { t = y; y = z; z = t; }
     if (x > y) { t = x; x = y; y = t; }
     w[0] = x; w[1] = y; w[2] = z;
+}
+
+// 2 cos(acos(r) / 3), r in [0, 1]: the largest root of x^3 - 3x - 2r, to 2e-12 (the
+// Chebyshev expansion on [0, 1] cut at degree 12; analytic down to r = -1).
+static __device__ const double c_root3[13] = {
+    1.7320508075704548, 0.3333333327844548, -0.09622501304407653, 0.04938198588801779, -0.031175250877004023,
+    0.021884006780256562, -0.01621223481643358, 0.012009045565307437, -0.008238552609840997, 0.004744084587962769,
+    -0.002043769071151769, 0.000565319565323375, -7.376232442871896e-05};
+
+// The same without iteration (the construction of Eberly, A Robust Eigensolver for
+// 3 x 3 Symmetric Matrices): the deviator over p = sqrt(tr B^2 / 6) has the roots of
+// x^3 - 3x - 2r, and one of them, x, is at least 1.7 from the others, so that the
+// adjugate of B/p - x gives its vector w; the Rayleigh quotient of w and the 2 x 2
+// block of B across w hold all three values, with the square of the vector's error
+// (1e-12).  A quotient is divided by its vector's norm to first order.  Error of the
+// values against extended precision, per |A|: rms 1.0e-16, the Jacobi iteration's.
+// 230 FP64 instructions, no division and no loop, where Jacobi takes about 1 100.
+__device__ __forceinline__ void sym3_eigvals(double a00, double a11, double a22, double a01, double a02, double a12,
+                                             double w[3]) {
+    const double nrm = fabs(a00) + fabs(a11) + fabs(a22) + fabs(a01) + fabs(a02) + fabs(a12);
+    const double q = (a00 + a11 + a22) * (1.0 / 3.0);
+    const double b0 = a00 - q, b1 = a11 - q, b2 = a22 - q;
+    const double p2 = fma(b0, b0, fma(b1, b1, fma(b2, b2, 2.0 * fma(a01, a01, fma(a02, a02, a12 * a12))))) * (1.0 / 6.0);
+    // diagonal (exact there), a multiple of the identity, not finite, or squares out
+    // of range
+    if (!(nrm > 1e-100 && nrm < 1e100 && p2 > 1e-210) || (a01 == 0.0 && a02 == 0.0 && a12 == 0.0)) {
+        sym3_jacobi(a00, a11, a22, a01, a02, a12, w);
+        return;
+    }
+    const double ip = rsqrt(p2);
+    const double c0 = b0 * ip, c1 = b1 * ip, c2 = b2 * ip, e01 = a01 * ip, e02 = a02 * ip, e12 = a12 * ip;
+    const double det = c0 * fma(c1, c2, -e12 * e12) - e01 * fma(e01, c2, -e12 * e02) + e02 * fma(e01, e12, -c1 * e02);
+    const double r = fmin(0.5 * fabs(det), 1.0);
+    double x = c_root3[12];
+#pragma unroll
+    for (int k = 11; k >= 0; --k) x = fma(x, r, c_root3[k]);
+    x = copysign(x, det);
+    const double m0 = c0 - x, m1 = c1 - x, m2 = c2 - x;
+    const double g0 = fma(m1, m2, -e12 * e12), g1 = fma(m0, m2, -e02 * e02), g2 = fma(m0, m1, -e01 * e01);
+    const double g01 = fma(e02, e12, -e01 * m2), g02 = fma(e01, e12, -e02 * m1), g12 = fma(e01, e02, -e12 * m0);
+    // the row of the largest diagonal element
+    const double f0 = fabs(g0), f1 = fabs(g1), f2 = fabs(g2);
+    const bool k0 = f0 >= f1 && f0 >= f2, k1 = !k0 && f1 >= f2;
+    double w0 = k0 ? g0 : (k1 ? g01 : g02), w1 = k0 ? g01 : (k1 ? g1 : g12), w2 = k0 ? g02 : (k1 ? g12 : g2);
+    double n = rsqrt(fma(w0, w0, fma(w1, w1, w2 * w2)));
+    w0 *= n; w1 *= n; w2 *= n;
+    // u, v across w
+    const bool big = fabs(w0) > fabs(w1);
+    const double t = big ? w0 : w1;
+    n = rsqrt(fma(t, t, w2 * w2));
+    const double tn = t * n, wn = w2 * n;
+    const double u0 = big ? -wn : 0.0, u1 = big ? 0.0 : wn, u2 = big ? tn : -tn;
+    const double v0 = fma(w1, u2, -w2 * u1), v1 = fma(w2, u0, -w0 * u2), v2 = fma(w0, u1, -w1 * u0);
+    auto row = [](double a, double b, double c, double x0, double x1, double x2) { return fma(a, x0, fma(b, x1, c * x2)); };
+    auto norm1 = [&](double x0, double x1, double x2) {   // 1 - |x|^2
+        return fma(-x0, x0, fma(-x1, x1, fma(-x2, x2, 1.0)));
+    };
+    const double Bu0 = row(b0, a01, a02, u0, u1, u2), Bu1 = row(a01, b1, a12, u0, u1, u2), Bu2 = row(a02, a12, b2, u0, u1, u2);
+    const double Bv0 = row(b0, a01, a02, v0, v1, v2), Bv1 = row(a01, b1, a12, v0, v1, v2), Bv2 = row(a02, a12, b2, v0, v1, v2);
+    const double Bw0 = row(b0, a01, a02, w0, w1, w2), Bw1 = row(a01, b1, a12, w0, w1, w2), Bw2 = row(a02, a12, b2, w0, w1, w2);
+    double lw = row(w0, w1, w2, Bw0, Bw1, Bw2), lu = row(u0, u1, u2, Bu0, Bu1, Bu2), lv = row(v0, v1, v2, Bv0, Bv1, Bv2);
+    lw = fma(lw, norm1(w0, w1, w2), lw);
+    lu = fma(lu, norm1(u0, u1, u2), lu);
+    lv = fma(lv, norm1(v0, v1, v2), lv);
+    const double uv = row(v0, v1, v2, Bu0, Bu1, Bu2);
+    const double h = 0.5 * (lu - lv), mm = 0.5 * (lu + lv), rt = sqrt(fma(h, h, uv * uv));
+    double y0 = q + lw, y1 = q + (mm - rt), y2 = q + (mm + rt), z;
+    if (y0 > y1) { z = y0; y0 = y1; y1 = z; }
+    if (y1 > y2) { z = y1; y1 = y2; y2 = z; }
+    w[0] = y0; w[1] = y1; w[2] = y2;
 }
 
 // nmr_convention (src/efg.f90:2546-2650): nmr = (Vxx, Vyy, Vzz, eta)
