@@ -969,6 +969,29 @@ float time_launch(mdff_ctx* ctx, const std::function<void()>& fn) {
     return ms / 3.f;
 }
 
+// Lanes per atom of k_ewald_dir on the mixed path, where a sum in another order
+// changes the forces by 1e-9 a step later: by a rule, so that two contexts of the
+// same system agree.  A block of 256 threads takes 256 / g atoms and two blocks fit
+// an SM; g lanes need the time of ceil(blocks / resident) / g of a row.  Equal
+// times: the fewest lanes (the least work beside the pairs), unless the last wave
+// of more lanes is less than a quarter full, where it runs faster than a whole one.
+// Where the times tie, a choice by timing went either way from one context to the
+// next (45 systems of 940 to 15 366 ions, three contexts each: 14 of them; the rule
+// agrees with 120 of the 135 choices).
+int dir_lanes(int n, const int* cand, int nc) {
+    int sms = 148, dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int best = cand[0];
+    double tbest = 1e300;
+    for (int k = 0; k < nc; ++k) {
+        const double waves = std::ceil((double)n * cand[k] / 256.0) / (2.0 * sms);
+        const double t = std::ceil(waves) / cand[k];
+        const bool thin = waves > 1.0 && waves - std::floor(waves) < 0.25 && waves > std::floor(waves);
+        if (t < tbest || (t == tbest && thin)) { best = cand[k]; tbest = t; }
+    }
+    return best;
+}
+
 int autotune(mdff_ctx* ctx) {
     ctx->tuned = true;
     if (!ctx->p.lcoulomb) return MDFF_OK;
@@ -997,10 +1020,12 @@ int autotune(mdff_ctx* ctx) {
     f.damp = 1;
     f.field = 1;
     f.forces = 1;
-    ctx->g_dir = pick([&](int g) {
-        launch_ewald_dir(ctx->st, n, ctx->rec, ctx->mrec, ctx->q, ctx->mu, ctx->cell, coul_list(ctx),
-                         ctx->pc, f, ctx->ef, nullptr, ctx->fcoul, ctx->part, ctx->dsc, g);
-    }, gs, 3);
+    if (ctx->p.precision == MDFF_PREC_MIXED) ctx->g_dir = dir_lanes(n, gs, 3);
+    else
+        ctx->g_dir = pick([&](int g) {
+            launch_ewald_dir(ctx->st, n, ctx->rec, ctx->mrec, ctx->q, ctx->mu, ctx->cell, coul_list(ctx),
+                             ctx->pc, f, ctx->ef, nullptr, ctx->fcoul, ctx->part, ctx->dsc, g);
+        }, gs, 3);
     if (ctx->p.precision == MDFF_PREC_MIXED) {
         ensure_phase_tables(ctx->st, n, ctx->sx, ctx->sy, ctx->sz, ctx->rs);
         // the pair table of this step, then the lanes per atom of its operator
