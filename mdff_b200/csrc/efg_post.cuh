@@ -341,26 +341,29 @@ __global__ void __launch_bounds__(EFG_THREADS, 3) k_efg_sites(int n, int nblk, i
     if (flag) atomicOr(bad, flag);
     if (SMEM) __syncthreads();
     if (SMEM) {
-        // flush: global bin k of the full layout from the block's type rows
-        const int nt = b.ntype, nt1 = nt + 1;
-        for (int k = threadIdx.x; k < b.nbins; k += EFG_THREADS) {
-            int base, w, row, hsel = 0;
-            if (k < b.oe) { w = b.PANvzz + 1; row = k / w; base = b.cv; }
-            else if (k < b.ou) { w = b.PANeta + 1; row = (k - b.oe) / w; base = b.ce; }
-            else if (k < b.os) { w = b.PANU + 1; const int q = (k - b.ou) / w; hsel = q / nt1; row = q % nt1; base = b.cu; }
-            else { w = b.PANS + 1; row = (k - b.os) / w; base = b.cs; }
-            const int bin = (k < b.oe ? k : k < b.ou ? k - b.oe : k < b.os ? k - b.ou : k - b.os) % w;
-            int v = 0;
-            const int u0 = hsel < 5 ? hsel : 1, u1 = hsel < 5 ? hsel : 4;   // U2..U5 together: histograms 1..4
-            for (int uh = u0; uh <= u1; ++uh) {
-                const int hb = base + uh * nt * w;   // uh = 0 for the three single histograms
-                if (row == 0)
-                    for (int t = 0; t < nt; ++t) v += efg_sh[hb + t * w + bin];
-                else
-                    v += efg_sh[hb + (row - 1) * w + bin];
+        // flush: the type rows and the all-sites row of one histogram, a bin a thread,
+        // without the four integer divisions a bin of the flat layout (97 us -> 79 at
+        // 32 440 sites, 32 configurations)
+        // (nh > 1: nh counted histograms into one)
+        const int nt = b.ntype;
+        auto flush = [&](int out, int in, int w, int nh) {
+            for (int bin = threadIdx.x; bin < w; bin += EFG_THREADS) {
+                int all = 0;
+                for (int t = 0; t < nt; ++t) {
+                    int v = 0;
+                    for (int h = 0; h < nh; ++h) v += efg_sh[in + (h * nt + t) * w + bin];
+                    if (v) atomicAdd(&hist[out + (t + 1) * w + bin], v);
+                    all += v;
+                }
+                if (all) atomicAdd(&hist[out + bin], all);
             }
-            if (v) atomicAdd(&hist[k], v);
-        }
+        };
+        const int wu = b.PANU + 1;
+        flush(b.ov, b.cv, b.PANvzz + 1, 1);
+        flush(b.oe, b.ce, b.PANeta + 1, 1);
+        for (int h = 0; h < 5; ++h) flush(b.ou + h * (nt + 1) * wu, b.cu + h * nt * wu, wu, 1);
+        flush(b.ou + 5 * (nt + 1) * wu, b.cu + nt * wu, wu, 4);   // U2..U5 together
+        flush(b.os, b.cs, b.PANS + 1, 1);
     }
 }
 
