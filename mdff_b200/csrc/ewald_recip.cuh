@@ -285,27 +285,50 @@ struct FieldParts {
 
 // Sum the field parts and scale by 2 (half mesh) * 4 pi / V.  ef (3n) += E_rec;
 // efg (6n: xx yy zz xy xz yz) += G_rec; fo (3n) += q E_rec + G_rec mu.  flow: nlow
-// more parts, with room for nine components each.  Block = 32 atoms x 8 runs:
-// eight parts at a time are read together and added in their order (the order
-// decides the last bit, and the mixed path's results with it).  A thread per
-// atom, its parts one after another, took 9.3 us at 4 056 ions and 85 at 1 536.
-template <int NV>
+// more parts, with room for nine components each.  Block = 256 / RUNS atoms x RUNS.
+// ORDERED (the mixed path): eight parts at a time are read together and added in
+// their order (the order decides the last bit, and the mixed path's results with
+// it).  Else run r adds the parts r, r + RUNS, ... and the runs are added at the
+// end, with 32 runs where few tiles share all CTAs: 512 ions, 148 parts an atom,
+// 10.6 us in order, 7.3 with 8 runs, 5.5 with 32 (the gradient 30, 17, 7.3).
+// A thread per atom, its parts one after another, took 9.3 us at 4 056 ions and
+// 85 at 1 536.
+template <int NV, bool ORDERED, int RUNS = 8>
 __global__ void __launch_bounds__(256)
     k_kfield_reduce(int n, FieldParts fp, const double* __restrict__ fpart, double scale, const double* __restrict__ q,
                     const double* __restrict__ mu, double* ef, double* efg, double* fo,
                     const double* __restrict__ flow, int nlow) {
-    __shared__ double s[8][NV][32];
-    const int lane = threadIdx.x & 31, run = threadIdx.x >> 5;
-    const int i = blockIdx.x * 32 + lane;
+    static_assert(!ORDERED || RUNS == 8, "the order of eight");
+    constexpr int A = 256 / RUNS;
+    __shared__ double s[RUNS][NV][A];
+    const int lane = threadIdx.x % A, run = threadIdx.x / A;
+    const int i = blockIdx.x * A + lane;
     double v[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) v[k] = 0.0;
     int np = fp.np;
-    if (fp.grid > 0) {   // (32 atoms are of one 128-atom tile)
-        const long units = (long)fp.ntile * fp.ncb, t0 = (long)(blockIdx.x * 32 / 128) * fp.ncb;
+    if (fp.grid > 0) {   // (a block's atoms are of one 128-atom tile)
+        const long units = (long)fp.ntile * fp.ncb, t0 = (long)(blockIdx.x * A / 128) * fp.ncb;
         np = (umma::range_of(t0 + fp.ncb - 1, units, fp.grid) - umma::range_of(t0, units, fp.grid) + 1) * fp.nq;
     }
-    for (int base = 0; base < np + nlow; base += 8) {
+    if (!ORDERED) {
+        if (i < n) {
+#pragma unroll 4
+            for (int p = run; p < np; p += RUNS) {
+                const double* o = fpart + (size_t)p * NV * n;
+#pragma unroll
+                for (int k = 0; k < NV; ++k) v[k] += o[(size_t)k * n + i];
+            }
+#pragma unroll
+            for (int k = 0; k < NV; ++k) s[run][k][lane] = v[k];
+        }
+        __syncthreads();
+        if (run == 0)
+            for (int w = 1; w < RUNS; ++w)
+#pragma unroll
+                for (int k = 0; k < NV; ++k) v[k] += s[w][k][lane];
+    }
+    for (int base = 0; ORDERED && base < np + nlow; base += 8) {
         const int p = base + run;
         if (p < np + nlow && i < n) {
             const double* o = p < np ? fpart + (size_t)p * NV * n : flow + (size_t)(p - np) * 9 * n;
@@ -1133,7 +1156,10 @@ int launch_t7_field(cudaStream_t st, int n, CellP c, const KGrid& kg, RecScratch
     tc7::k_kfield_t7<NMOM><<<grid, tc7::FTHREADS, NMOM == 3 ? t.smem_f3 : t.smem_f2, st>>>(
         n, t.ntile_f, t.ncol, ncb, t.aimg, t.xy, t.fimg, t.kx, t.ky, t.KZ, c, rs.fpart, &d->tc_err);
     const FieldParts fp{0, t.ntile_f, ncb, grid, tc7::NQ};
-    k_kfield_reduce<NV><<<(n + 31) / 32, 256, 0, st>>>(n, fp, rs.fpart, scale, q, mu, ef, efg, fo, nullptr, 0);
+    if (grid * tc7::NQ > 32 * t.ntile_f)   // parts an atom
+        k_kfield_reduce<NV, false, 32><<<(n + 7) / 8, 256, 0, st>>>(n, fp, rs.fpart, scale, q, mu, ef, efg, fo, nullptr, 0);
+    else
+        k_kfield_reduce<NV, false><<<(n + 31) / 32, 256, 0, st>>>(n, fp, rs.fpart, scale, q, mu, ef, efg, fo, nullptr, 0);
     return 3;
 }
 
@@ -1334,9 +1360,9 @@ void launch_ewald_rec(cudaStream_t st, int n, const double* sx, const double* sy
     double *oe = fl.field ? ef : nullptr, *of = fl.forces ? fo : nullptr;
     const int nlow = low ? (rs.low.tc ? tc4::NQ : LK_SPLIT) : 0;
     if (grad)
-        k_kfield_reduce<9><<<(n + 31) / 32, 256, 0, st>>>(n, fparts, rs.fpart, scale, fq, fm, oe, efg, of, fl_low, nlow);
+        k_kfield_reduce<9, true><<<(n + 31) / 32, 256, 0, st>>>(n, fparts, rs.fpart, scale, fq, fm, oe, efg, of, fl_low, nlow);
     else
-        k_kfield_reduce<3><<<(n + 31) / 32, 256, 0, st>>>(n, fparts, rs.fpart, scale, fq, fm, oe, efg, of, fl_low, nlow);
+        k_kfield_reduce<3, true><<<(n + 31) / 32, 256, 0, st>>>(n, fparts, rs.fpart, scale, fq, fm, oe, efg, of, fl_low, nlow);
     prof->end(nk);
 }
 
