@@ -1139,7 +1139,7 @@ int launch_t7_sfac(cudaStream_t st, int n, const double* sx, const double* sy, c
         t.nblk, t.bps, t.nin, t.bimg, t.xy, t.prm, t.bmax, t.pairs, t.trange, t.npair, t.kx, t.ky, t.kz, t.N, t.entmax,
         rs.part, t.pstride, &d->tc_err);
     const dim3 g(t.ntile, t.kz + 1);
-    tc7::k_t7_sreduce<<<g, 256, 0, st>>>(t.nsplit, t.N, t.npair, t.pstride, t.pairs, t.ky, t.kz, t.nzl, rs.part, kg.Ak,
+    tc7::k_t7_sreduce<<<g, t.nsplit >= 16 ? 1024 : 256, 0, st>>>(t.nsplit, t.N, t.npair, t.pstride, t.pairs, t.ky, t.kz, t.nzl, rs.part, kg.Ak,
                                          kg.kcoe, c, rs.aks, kg.nrect, fl.energy, part.buf);
     if (fl.energy) launch_reduce_partials(st, part.buf, t.ntile * (t.kz + 1), 7, d->rec, 0);
     return nk + 3 + (fl.energy ? 1 : 0);

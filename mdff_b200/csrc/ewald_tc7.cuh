@@ -429,13 +429,16 @@ __global__ void __launch_bounds__(THREADS, 1)
 
 // The splits summed in order, the four vectors (+-ny, +-m) of each (pair, m),
 // A_k S(k) and, with `energy`, the energy and stress sums (src/field.f90:
-// 2742-2745, 2803-2815).  grid (tiles of 32 pairs, kz + 1), 256 threads.
-__global__ void __launch_bounds__(256)
+// 2742-2745, 2803-2815).  grid (tiles of 32 pairs, kz + 1), 256 H threads: H
+// threads a sum, each taking every H-th split (H = 4 from 16 splits on, where one
+// thread's chain of reads is the kernel's time: 3 000 ions, 37 splits 6.5 -> 4.6 us).
+__global__ void __launch_bounds__(1024)
     k_t7_sreduce(int nsplit, int N, int npair, int pstride, const int* __restrict__ pairs, int ky, int kz, int nzl,
                  const double* __restrict__ part, const double* __restrict__ Ak, const double* __restrict__ kcoe,
                  CellP c, double* __restrict__ aks, int nrect, int energy, double* partials) {
-    __shared__ double s[8][32];
-    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;   // q = (row kind, U/V)
+    __shared__ double s[8][32], sh[3][8][32];
+    const int lane = threadIdx.x & 31, q = (threadIdx.x >> 5) & 7;   // q = (row kind, U/V)
+    const int h = threadIdx.x >> 8, H = blockDim.x >> 8;
     const int pi = blockIdx.x * 32 + lane, m = blockIdx.y;
     double v[7] = {0, 0, 0, 0, 0, 0, 0};
     double sum = 0.0;
@@ -443,12 +446,17 @@ __global__ void __launch_bounds__(256)
         const double* p = part + ((size_t)(q >> 1) * N + 2 * m + (q & 1)) * pstride + pi;
         const size_t step = (size_t)4 * N * pstride;
 #pragma unroll 8
-        for (int k = 0; k < nsplit; ++k) sum += p[k * step];
+        for (int k = h; k < nsplit; k += H) sum += p[k * step];
     }
-    s[q][lane] = sum;
+    if (h > 0) sh[h - 1][q][lane] = sum;
+    if (H > 1) __syncthreads();
+    if (h == 0) {
+        for (int w = 1; w < H; ++w) sum += sh[w - 1][q][lane];
+        s[q][lane] = sum;
+    }
     __syncthreads();
     const int sy = q & 1, sm = (q >> 1) & 1;   // sign of ny, of nz
-    if (q < 4 && pi < npair) {
+    if (threadIdx.x < 128 && pi < npair) {   // q < 4 of the first group
         const int nx = pairs[2 * pi], ny = sy ? -pairs[2 * pi + 1] : pairs[2 * pi + 1], nz = sm ? -m : m;
         const double Ur = s[4 * sy][lane], Vr = s[4 * sy + 1][lane], Ui = s[4 * sy + 2][lane], Vi = s[4 * sy + 3][lane];
         const double sr = sm ? Ur + Vi : Ur - Vi, si = sm ? Ui - Vr : Ui + Vr;
