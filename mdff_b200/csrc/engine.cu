@@ -579,8 +579,8 @@ void dd_field_real(mdff_ctx* ctx, const double* m, double* out) {
     }
     const NList& L = coul_list(ctx);
     if (ctx->ddtab64 && ctx->ddtab_epoch == ctx->rs.want_epoch && ctx->ddtab_lcap == L.cap) {
-        launch_ewald_ddtab64(ctx->st, n, ctx->rec, ctx->mrec, m, ctx->cell, ctx->ddnbr, ctx->ddcnt, L.cap, ctx->ddtab64,
-                             out, ctx->g_dd);
+        launch_ewald_ddtab64(ctx->st, n, ctx->rec, ctx->mrec, m, ctx->cell, geom_of(ctx), ctx->ddnbr, ctx->ddcnt, L.cap,
+                             ctx->ddtab64, out, ctx->g_dd);
         ctx->prof.end(2);
         return;
     }
@@ -1064,8 +1064,8 @@ int autotune(mdff_ctx* ctx) {
             launch_ewald_dir(ctx->st, n, ctx->rec, ctx->mrec, ctx->q, ctx->mu, ctx->cell, coul_list(ctx),
                              ctx->pc, fs, ctx->Estat, nullptr, nullptr, ctx->part, ctx->dsc, ctx->g_dir);
             ctx->g_dd = pick([&](int g) {
-                launch_ewald_ddtab64(ctx->st, n, ctx->rec, ctx->mrec, ctx->mu, ctx->cell, ctx->ddnbr, ctx->ddcnt,
-                                     coul_list(ctx).cap, ctx->ddtab64, ctx->Eind, g);
+                launch_ewald_ddtab64(ctx->st, n, ctx->rec, ctx->mrec, ctx->mu, ctx->cell, geom_of(ctx), ctx->ddnbr,
+                                     ctx->ddcnt, coul_list(ctx).cap, ctx->ddtab64, ctx->Eind, g);
             }, gs, 3);
         }
     }

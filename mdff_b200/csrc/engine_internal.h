@@ -361,7 +361,7 @@ void launch_ewald_ddtab(cudaStream_t st, int n, const uint32_t* fx, const double
 
 // The FP64 path's form: FP64 pair table and k_ewald_dir's records.
 void launch_ewald_ddtab64(cudaStream_t st, int n, const double4* rec, double4* mrec, const double* mu, CellP c,
-                          const int* nbr, const int* cnt, int cap, const double2* tab, double* ef, int g = 16);
+                          int geom, const int* nbr, const int* cnt, int cap, const double2* tab, double* ef, int g = 16);
 
 // Solver vector kernels.
 

@@ -390,14 +390,16 @@ __global__ void k_dir_records(int n, const double* __restrict__ mu, const double
 
 // FP64 path: the operator from an FP64 pair table, so that a solver iteration
 // evaluates no square root, exponential or erfc: 20 bytes of table and ~31 FP64
-// instructions per ordered pair, the image from the fractional coordinates
-// (d - rint(d); where the two images of a pair are equally far, T2 is the same
-// for both).  A1 and B2 are the charge pass's own doubles, so the operator is
+// instructions per ordered pair, the image from the fractional coordinates as
+// d - rint(d).  EXACT: the reference's expression instead (pairvec_exact), for a
+// cell narrower than twice the cutoff, where a pair inside it can have d = +-1/2,
+// rint and the reference's NINT take different images of it, and the two images'
+// r r^T differ.  A1 and B2 are the charge pass's own doubles, so the operator is
 // MODE 1's to rounding and symmetric to the last bit.  Bound: the gathers of
 // two 32-byte records a pair through L2 (930 MB at 32 440 ions, rc 10 A) beside the table's
 // 290 MB from HBM: 117 us per application against 279 of MODE 1, 14 against 33
 // at 3 000 ions; the charge pass takes 64 us longer once a step.
-template <int G>
+template <int G, bool EXACT>
 __global__ void __launch_bounds__(256) k_ewald_ddtab64(int n, const double4* __restrict__ rec,
                                                        const double4* __restrict__ mrec, CellP c,
                                                        const int* __restrict__ nbr, const int* __restrict__ cnt,
@@ -407,7 +409,6 @@ __global__ void __launch_bounds__(256) k_ewald_ddtab64(int n, const double4* __r
     const int sub = threadIdx.x & (G - 1);
     const bool active = gid < n;
     const int i = active ? gid : 0;
-    constexpr double M = 6755399441055744.0;   // 1.5 2^52: (d + M) - M = rint(d)
     double E0 = 0.0, E1 = 0.0, E2 = 0.0;
     if (active) {
         const double4 ri = ld_rec(rec + i);
@@ -417,13 +418,8 @@ __global__ void __launch_bounds__(256) k_ewald_ddtab64(int n, const double4* __r
         auto term = [&](int j, double2 t) {
             const double4 p = ld_rec(rec + j), mj = ld_rec(mrec + j);
             const double m0 = mj.x, m1 = mj.y, m2 = mj.z;
-            double d0 = ri.x - p.x, d1 = ri.y - p.y, d2 = ri.z - p.z;
-            d0 -= (d0 + M) - M;
-            d1 -= (d1 + M) - M;
-            d2 -= (d2 + M) - M;
-            const double rx = fma(d2, c.A[2], fma(d1, c.A[1], d0 * c.A[0]));
-            const double ry = fma(d2, c.A[5], fma(d1, c.A[4], d0 * c.A[3]));
-            const double rz = fma(d2, c.A[8], fma(d1, c.A[7], d0 * c.A[6]));
+            double rx, ry, rz;
+            pairvec(EXACT ? GEOM_EXACT : GEOM_GENERAL, c, ri.x, ri.y, ri.z, p.x, p.y, p.z, rx, ry, rz);
             const double rb = fma(rz, m2, fma(ry, m1, rx * m0)) * t.y;
             E0 = fma(rx, rb, fma(-m0, t.x, E0));
             E1 = fma(ry, rb, fma(-m1, t.x, E1));
@@ -445,13 +441,15 @@ __global__ void __launch_bounds__(256) k_ewald_ddtab64(int n, const double4* __r
 }
 
 void launch_ewald_ddtab64(cudaStream_t st, int n, const double4* rec, double4* mrec, const double* mu, CellP c,
-                          const int* nbr, const int* cnt, int cap, const double2* tab, double* ef, int g) {
+                          int geom, const int* nbr, const int* cnt, int cap, const double2* tab, double* ef, int g) {
     k_dir_records<<<(n + 255) / 256, 256, 0, st>>>(n, mu, nullptr, mrec);
     const int blocks = (int)(((size_t)n * g + 255) / 256);
-#define DDT(G) k_ewald_ddtab64<G><<<blocks, 256, 0, st>>>(n, rec, mrec, c, nbr, cnt, cap, tab, ef)
+#define DDTX(G, X) k_ewald_ddtab64<G, X><<<blocks, 256, 0, st>>>(n, rec, mrec, c, nbr, cnt, cap, tab, ef)
+#define DDT(G) do { if (geom == GEOM_EXACT) DDTX(G, true); else DDTX(G, false); } while (0)
     if (g == 8) DDT(8);
     else if (g == 32) DDT(32);
     else DDT(16);
+#undef DDTX
 #undef DDT
 }
 
