@@ -4432,7 +4432,10 @@ int rmc_cap(const mdff_ctx* ctx, double rl) {
 
 // Full neighbour rows within rl of the fractional coordinates s by the cell
 // grid of the Verlet lists (its buffers are scratch between builds); nbr grows,
-// with cap, until the rows fit.
+// with cap, until the rows fit.  The rows are in no order, which the integer
+// counts do not show: a cutoff near half the cell leaves eight cells, and one
+// thread sorts a cell of more than 4 096 atoms (RMC of 46 656 ions, cut 36 A, 500
+// moves: 440 ms with the cells sorted, 112 without).
 int rmc_lists(mdff_ctx* ctx, const double* s, double rl, int& cap, int** nbr, int* cnt) {
     const int n = ctx->n;
     CellGrid& g = ctx->grid;
@@ -4445,7 +4448,7 @@ int rmc_lists(mdff_ctx* ctx, const double* s, double rl, int& cap, int** nbr, in
         TRY(dalloc(ctx, &g.cell_cursor, g.ncell));
         g.ncell_alloc = g.ncell;
     }
-    launch_bin(ctx->st, n, s, s + n, s + 2 * (size_t)n, g);
+    launch_bin(ctx->st, n, s, s + n, s + 2 * (size_t)n, g, false);
     for (int attempt = 0;; ++attempt) {
         if (!*nbr) CK(cudaMallocAsync((void**)nbr, sizeof(int) * (size_t)n * cap, ctx->st));
         CK(cudaMemsetAsync(ctx->d_overflow, 0, sizeof(int), ctx->st));

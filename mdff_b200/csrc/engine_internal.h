@@ -181,7 +181,8 @@ struct CellGrid {
     float4* cell_w = nullptr;   // [n] cell order: FP32 wrapped fractional coordinates, atom index as bits
     int ncell_alloc = 0;
 };
-void launch_bin(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz, CellGrid& g);
+void launch_bin(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz, CellGrid& g,
+                bool sorted = true);
 void launch_nlist(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz, CellP c,
                   const CellGrid& g, double rskinsq_a, NList& la, double rskinsq_b, NList* lb, int* overflow);
 void launch_skin_check(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz,

@@ -171,12 +171,13 @@ __global__ void k_cell_coords(int n, const double* __restrict__ sx, const double
     cw[k] = make_float4((float)(a - floor(a)), (float)(b - floor(b)), (float)(c - floor(c)), __int_as_float(j));
 }
 
-void launch_bin(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz, CellGrid& g) {
+// sorted: the cells' atoms by index (the order of the rows).
+void launch_bin(cudaStream_t st, int n, const double* sx, const double* sy, const double* sz, CellGrid& g, bool sorted) {
     cudaMemsetAsync(g.cell_count, 0, sizeof(int) * g.ncell, st);
     k_bin_count<<<(n + 255) / 256, 256, 0, st>>>(n, sx, sy, sz, g.nc[0], g.nc[1], g.nc[2], g.cell_of, g.cell_count);
     k_scan<<<1, 1024, 0, st>>>(g.ncell, g.cell_count, g.cell_start, g.cell_cursor);
     k_bin_fill<<<(n + 255) / 256, 256, 0, st>>>(n, g.cell_of, g.cell_cursor, g.cell_atoms);
-    k_sort_cells<<<g.ncell, 128, 0, st>>>(g.ncell, g.cell_start, g.cell_atoms);
+    if (sorted) k_sort_cells<<<g.ncell, 128, 0, st>>>(g.ncell, g.cell_start, g.cell_atoms);
     k_cell_coords<<<(n + 255) / 256, 256, 0, st>>>(n, sx, sy, sz, g.cell_atoms, g.cell_w);
 }
 

@@ -1,0 +1,39 @@
+"""RMC and g(r) with cutoffs near half the cell's width: the eight cells of the
+neighbour rows then hold thousands of atoms each, and the rows most of all pairs.
+
+Times are compared with the same call just past half the width, which counts all
+pairs without rows; the counts are integers and have to be equal."""
+import time
+
+import numpy as np
+import pytest
+
+import mdff_b200
+from mdff_b200 import systems
+
+from test_gpu_rmc import rmc_params
+
+pytestmark = pytest.mark.gpu
+
+
+def best(f, k=3):
+    t = []
+    for _ in range(k):
+        a = time.perf_counter()
+        f()
+        t.append(time.perf_counter() - a)
+    return min(t)
+
+
+def test_chain():
+    s = systems.mgo_pim(grid=(34, 34, 34), rc=8.0, alpha=0.4, kmax=3, seed=2)   # 4 913 ions a cell
+    half = 0.5 * s["cell"][0, 0]
+    e = mdff_b200.Engine(s["params"], s["itype"], s["pos"], s["cell"])
+    t = {}
+    for cut in (half - 1.3, half + 0.2):
+        gexp = e.gr(cut, 0.05) * 1.01
+        rp = rmc_params(10 ** 9, 40, cut, 0.05)
+        _, g = e.rmc(rp, gexp, seed=1)
+        assert np.array_equal(g, e.gr(cut, 0.05))
+        t[cut > half] = best(lambda: e.rmc(rp, gexp, seed=1))
+    assert t[False] < 2.0 * t[True], t
