@@ -4487,16 +4487,35 @@ int rmc_counts(mdff_ctx* ctx, const double* s, const RmcConst& k, const int* nbr
     return check_launch(ctx, "gr");
 }
 
-// The same with rows built for it where the cell has room for a list.
+// The same with rows built for it where they pay: with five cells along each edge
+// 32 768 and 64 000 ions take 3.7 and 11.3 ms from rows; with four, where the cells
+// around an atom hold 27 / 64 of the others, 5.9 and 21.2 from rows and 4.6 and 15.7
+// over all pairs.  So rows when that share is below 0.3 and, past 256 MB of them,
+// when a quarter of the free memory holds them (they grow as n^2 cut^3); without
+// memory for them all pairs as well.
 int rmc_counts_of(mdff_ctx* ctx, const double* s, const RmcConst& k, double cut, int* hist) {
-    if (rmc_all_pairs(ctx, cut) || ctx->n < 2) return rmc_counts(ctx, s, k, nullptr, nullptr, 0, hist);
+    double share = 1.0;
+    for (int d = 0; d < 3; ++d) {
+        const double nc = std::floor(ctx->W[d] / cut);
+        if (nc > 3.0) share *= 3.0 / nc;
+    }
     int cap = std::max(1, rmc_cap(ctx, cut));
+    const size_t bytes = sizeof(int) * (size_t)ctx->n * cap;
+    bool rows = !rmc_all_pairs(ctx, cut) && ctx->n > 1 && share < 0.3;
+    if (rows && bytes > ((size_t)256 << 20)) {
+        size_t fr = 0, tot = 0;
+        CK(cudaMemGetInfo(&fr, &tot));
+        rows = bytes <= fr / 4;
+    }
     int *nbr = nullptr, *cnt = nullptr;
-    CK(cudaMallocAsync((void**)&cnt, sizeof(int) * (size_t)ctx->n, ctx->st));
-    int rc = rmc_lists(ctx, s, cut, cap, &nbr, cnt);
-    if (rc == MDFF_OK) rc = rmc_counts(ctx, s, k, nbr, cnt, cap, hist);
+    if (rows) {
+        rows = cudaMallocAsync((void**)&cnt, sizeof(int) * (size_t)ctx->n, ctx->st) == cudaSuccess &&
+               rmc_lists(ctx, s, cut, cap, &nbr, cnt) == MDFF_OK;
+        if (!rows) cudaGetLastError();
+    }
+    const int rc = rows ? rmc_counts(ctx, s, k, nbr, cnt, cap, hist) : rmc_counts(ctx, s, k, nullptr, nullptr, 0, hist);
     if (nbr) cudaFreeAsync(nbr, ctx->st);
-    cudaFreeAsync(cnt, ctx->st);
+    if (cnt) cudaFreeAsync(cnt, ctx->st);
     return rc;
 }
 
@@ -4514,15 +4533,20 @@ int mdff_gr(mdff_ctx* ctx, double cut, double res, double* grr, int* nbins) {
     const int n = ctx->n;
     double* s = nullptr;
     int* h = nullptr;
-    CK(cudaMallocAsync((void**)&s, sizeof(double) * 3 * (size_t)n, ctx->st));
-    CK(cudaMallocAsync((void**)&h, sizeof(int) * (size_t)k.nrow * k.nbins, ctx->st));
-    CK(cudaMemsetAsync(h, 0, sizeof(int) * (size_t)k.nrow * k.nbins, ctx->st));
-    TRY(rmc_frac(ctx, s));
-    TRY(rmc_counts_of(ctx, s, k, cut, h));
     std::vector<int> hh((size_t)k.nrow * k.nbins);
-    CK(cudaMemcpyAsync(hh.data(), h, sizeof(int) * hh.size(), cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaFreeAsync(s, ctx->st));
-    CK(cudaFreeAsync(h, ctx->st));
+    auto counts = [&]() -> int {
+        CK(cudaMallocAsync((void**)&s, sizeof(double) * 3 * (size_t)n, ctx->st));
+        CK(cudaMallocAsync((void**)&h, sizeof(int) * hh.size(), ctx->st));
+        CK(cudaMemsetAsync(h, 0, sizeof(int) * hh.size(), ctx->st));
+        TRY(rmc_frac(ctx, s));
+        TRY(rmc_counts_of(ctx, s, k, cut, h));
+        CK(cudaMemcpyAsync(hh.data(), h, sizeof(int) * hh.size(), cudaMemcpyDeviceToHost, ctx->st));
+        return MDFF_OK;
+    };
+    const int rc = counts();
+    if (s) cudaFreeAsync(s, ctx->st);
+    if (h) cudaFreeAsync(h, ctx->st);
+    TRY(rc);
     CK(cudaStreamSynchronize(ctx->st));
     rmc_normalise(k, hh, grr);
     return MDFF_OK;

@@ -2,7 +2,8 @@
 neighbour rows then hold thousands of atoms each, and the rows most of all pairs.
 
 Times are compared with the same call just past half the width, which counts all
-pairs without rows; the counts are integers and have to be equal."""
+pairs without rows; the counts are integers and have to be equal.  The same counts
+without memory for the rows."""
 import time
 
 import numpy as np
@@ -11,6 +12,7 @@ import pytest
 import mdff_b200
 from mdff_b200 import systems
 
+from gpu_memory import memory_left
 from test_gpu_rmc import rmc_params
 
 pytestmark = pytest.mark.gpu
@@ -37,3 +39,24 @@ def test_chain():
         assert np.array_equal(g, e.gr(cut, 0.05))
         t[cut > half] = best(lambda: e.rmc(rp, gexp, seed=1))
     assert t[False] < 2.0 * t[True], t
+
+
+def liquid(m):
+    s = systems.mgo_pim(grid=(m, m, m), rc=8.0, alpha=0.4, kmax=3, seed=2, jitter=0.1)
+    return mdff_b200.Engine(s["params"], s["itype"], s["pos"], s["cell"]), s["cell"][0, 0]
+
+
+def test_gr_time():
+    e, edge = liquid(32)
+    t = {f: best(lambda: e.gr(f * edge, 0.05)) for f in (0.24, 0.49, 0.51)}
+    assert max(t[0.24], t[0.49]) < 2.0 * t[0.51], t
+
+
+@pytest.mark.parametrize("m,left", [(32, 100), (40, 1000)])
+def test_gr_without_memory(m, left):
+    """Rows of 161 MB in 100 MB, and of 630 MB where they are more than a quarter of what is free."""
+    e, edge = liquid(m)
+    g = e.gr(0.19 * edge, 0.05)
+    with memory_left(left << 20):
+        assert np.array_equal(g, e.gr(0.19 * edge, 0.05))
+    assert np.array_equal(g, e.gr(0.19 * edge, 0.05))
