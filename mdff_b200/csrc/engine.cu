@@ -118,6 +118,7 @@ struct mdff_ctx {
     PairConst* pc = nullptr;
     NList lv, lc;
     bool shared_list = false;
+    int list_cap = 32;                   // row capacity the lists start with
     CellGrid grid;
     KGrid kg;
     RecScratch rs;
@@ -183,8 +184,10 @@ int fail(mdff_ctx* c, int code, const std::string& msg) {
 #define CK(call)                                                                                  \
     do {                                                                                          \
         cudaError_t e_ = (call);                                                                  \
-        if (e_ != cudaSuccess)                                                                    \
+        if (e_ != cudaSuccess) {                                                                  \
+            cudaGetLastError(); /* reported here, not by the next launch */                       \
             return fail(ctx, MDFF_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));   \
+        }                                                                                         \
     } while (0)
 
 #define TRY(expr)                  \
@@ -198,7 +201,10 @@ int dalloc(mdff_ctx* ctx, T** ptr, size_t count) {
     if (count == 0) count = 1;
     void* p = nullptr;
     cudaError_t e = cudaMalloc(&p, sizeof(T) * count);
-    if (e != cudaSuccess) return fail(ctx, MDFF_E_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();   // reported here, not by the next launch
+        return fail(ctx, MDFF_E_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
     ctx->allocs.push_back(p);
     *ptr = (T*)p;
     return MDFF_OK;
@@ -422,7 +428,7 @@ int ensure_lists(mdff_ctx* ctx, int cap) {
     ctx->shared_list = !(nonb && ctx->p.lcoulomb) || (ctx->cut_vdw == ctx->cut_coul);
     auto alloc_list = [&](NList& L) -> int {
         if (L.cap >= cap && L.nbr) return MDFF_OK;
-        if (L.nbr) { cudaFree(L.nbr); ctx->allocs.erase(std::find(ctx->allocs.begin(), ctx->allocs.end(), (void*)L.nbr)); L.nbr = nullptr; }
+        if (L.nbr) { cudaFree(L.nbr); ctx->allocs.erase(std::find(ctx->allocs.begin(), ctx->allocs.end(), (void*)L.nbr)); L.nbr = nullptr; L.cap = 0; }
         TRY(dalloc(ctx, &L.nbr, (size_t)ctx->n * cap));
         if (!L.cnt) TRY(dalloc(ctx, &L.cnt, (size_t)ctx->n));
         L.cap = cap;
@@ -439,6 +445,8 @@ int build_lists(mdff_ctx* ctx, double skin, bool from_frac = false) {
     const int n = ctx->n;
     double rl = rlist_max(ctx, skin);
     if (rl <= 0.0) return MDFF_OK;
+    ctx->have_list = false;   // until this build is done: one that fails leaves no list behind
+    if (!ctx->lv.nbr || (!ctx->shared_list && !ctx->lc.nbr)) TRY(ensure_lists(ctx, ctx->list_cap));
     CellGrid& g = ctx->grid;
     for (int d = 0; d < 3; ++d) {
         int nc = (int)std::floor(ctx->W[d] / (rl * (1.0 + 1e-12)));
@@ -3594,6 +3602,7 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
         cap = (int)std::min<double>((double)n, est * 1.4 + 32.0);
         cap = std::max(cap, 32);
     }
+    ctx->list_cap = cap;
     TRY(ensure_lists(ctx, cap));
     ctx->itime = 0;
     ctx->have_system = true;
