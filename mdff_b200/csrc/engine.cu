@@ -1093,16 +1093,17 @@ int engforce_device(mdff_ctx* ctx) {
     const int n = ctx->n;
     const mdff_params& p = ctx->p;
     const bool efg = p.doefg && ctx->efg_due;
+    const bool fresh = ctx->rec_fresh;   // of this evaluation alone, also when it fails below
+    ctx->rec_fresh = false;
     const bool built = !p.lvnlist || !ctx->have_list;
     if (!p.lvnlist) TRY(build_lists(ctx, 0.0));
     else if (!ctx->have_list) TRY(build_lists(ctx, p.skindiff));   // lists dropped (an interrupted RMC chain)
-    if (!(ctx->rec_fresh && p.lvnlist && !built)) {
+    if (!(fresh && p.lvnlist && !built)) {
         ctx->prof.begin(PK_OTHER);
         k_frac_rec<<<nb(n), 256, 0, ctx->st>>>(n, ctx->x, ctx->y, ctx->z, ctx->type, ctx->cell, ctx->sx, ctx->sy,
                                                ctx->sz, ctx->rec);
         ctx->prof.end(1);
     }
-    ctx->rec_fresh = false;
     ctx->rs.want_epoch++;   // positions may have changed: rebuild the phase tables
     if (p.autotune && !ctx->tuned) TRY(autotune(ctx));
     std::memset(&ctx->en, 0, sizeof ctx->en);

@@ -39,3 +39,13 @@ def test_next_evaluation():
     e.set_positions(s["pos"])
     g = e.engforce()
     assert np.array_equal(f["f"], g["f"]) and f["e"] == g["e"]
+
+
+def test_positions_after_a_failed_step():
+    """The evaluation is one of the positions set last, not of the failed step's."""
+    s, f = liquid()
+    e = failed_step(s)
+    e.set_positions(s["pos"])
+    e.nlist_build()
+    g = e.engforce()
+    assert np.array_equal(f["f"], g["f"]) and f["e"] == g["e"]
