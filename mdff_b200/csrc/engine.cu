@@ -225,6 +225,15 @@ int dgrow(mdff_ctx* ctx, T** ptr, size_t* cap, size_t need) {
     return MDFF_OK;
 }
 
+// Whether a table that a call can do without may be made: it leaves room for what
+// cannot be done without, here (list growth, per-call buffers) and in the other
+// libraries of the process.
+bool table_fits(size_t bytes) {
+    if (bytes <= ((size_t)256 << 20)) return true;   // (or its allocation fails)
+    size_t fr = 0, tot = 0;
+    return cudaMemGetInfo(&fr, &tot) == cudaSuccess && bytes <= fr / 4;
+}
+
 void free_all(mdff_ctx* ctx) {
     for (void* p : ctx->allocs) cudaFree(p);
     ctx->allocs.clear();
@@ -618,8 +627,8 @@ int induced_field(mdff_ctx* ctx, const double* m, double* out, bool self = true)
 
 // Let this charge pass also write the dipole-dipole pair table for the solver's
 // operator (allocated for the current list capacity), in FP32 on the mixed
-// path and in FP64 on the FP64 path.  Where the FP64 table does not fit in
-// device memory the operator goes on without it.
+// path and in FP64 on the FP64 path.  Where the FP64 table (20 bytes per list slot,
+// 16 kB an atom at rc 10 A) does not fit the operator goes on without it.
 int arm_ddtab(mdff_ctx* ctx, DirFlags& f) {
     const bool mixed = ctx->p.precision == MDFF_PREC_MIXED;
     if (!mixed && ctx->ddtab_off) return MDFF_OK;
@@ -633,11 +642,12 @@ int arm_ddtab(mdff_ctx* ctx, DirFlags& f) {
         ctx->ddtab64 = nullptr;
         ctx->ddnbr = nullptr;
         ctx->ddtab_cap = 0;
-        cudaError_t e = mixed ? cudaMalloc(&ctx->ddtab, sizeof(float2) * need)
-                              : cudaMalloc(&ctx->ddtab64, sizeof(double2) * need);
+        cudaError_t e = cudaErrorMemoryAllocation;
+        if (mixed) e = cudaMalloc(&ctx->ddtab, sizeof(float2) * need);
+        else if (table_fits((sizeof(double2) + sizeof(int)) * need)) e = cudaMalloc(&ctx->ddtab64, sizeof(double2) * need);
         if (e == cudaSuccess) e = cudaMalloc(&ctx->ddnbr, sizeof(int) * need);
+        if (e != cudaSuccess) cudaGetLastError();
         if (e != cudaSuccess && !mixed) {
-            cudaGetLastError();
             cudaFree(ctx->ddtab64);
             ctx->ddtab64 = nullptr;
             ctx->ddtab_off = true;
@@ -4500,9 +4510,8 @@ int rmc_counts(mdff_ctx* ctx, const double* s, const RmcConst& k, const int* nbr
 // The same with rows built for it where they pay: with five cells along each edge
 // 32 768 and 64 000 ions take 3.7 and 11.3 ms from rows; with four, where the cells
 // around an atom hold 27 / 64 of the others, 5.9 and 21.2 from rows and 4.6 and 15.7
-// over all pairs.  So rows when that share is below 0.3 and, past 256 MB of them,
-// when a quarter of the free memory holds them (they grow as n^2 cut^3); without
-// memory for them all pairs as well.
+// over all pairs.  So rows when that share is below 0.3 and they fit (they grow as
+// n^2 cut^3).
 int rmc_counts_of(mdff_ctx* ctx, const double* s, const RmcConst& k, double cut, int* hist) {
     double share = 1.0;
     for (int d = 0; d < 3; ++d) {
@@ -4511,12 +4520,7 @@ int rmc_counts_of(mdff_ctx* ctx, const double* s, const RmcConst& k, double cut,
     }
     int cap = std::max(1, rmc_cap(ctx, cut));
     const size_t bytes = sizeof(int) * (size_t)ctx->n * cap;
-    bool rows = !rmc_all_pairs(ctx, cut) && ctx->n > 1 && share < 0.3;
-    if (rows && bytes > ((size_t)256 << 20)) {
-        size_t fr = 0, tot = 0;
-        CK(cudaMemGetInfo(&fr, &tot));
-        rows = bytes <= fr / 4;
-    }
+    bool rows = !rmc_all_pairs(ctx, cut) && ctx->n > 1 && share < 0.3 && table_fits(bytes);
     int *nbr = nullptr, *cnt = nullptr;
     if (rows) {
         rows = cudaMallocAsync((void**)&cnt, sizeof(int) * (size_t)ctx->n, ctx->st) == cudaSuccess &&
