@@ -142,6 +142,8 @@ struct mdff_ctx {
     // Coulomb list entry), written by the charge pass of each force evaluation
     float2* ddtab = nullptr;
     double2* ddtab64 = nullptr;          // FP64 path
+    bool rec_ready = false;              // the FP64 path's reciprocal space is planned and allocated (ensure_rec)
+    std::vector<char> kcol;              // which columns of the k rectangle hold wave vectors
     bool ddtab_off = false;              // FP64 path: no memory for the table, the operator is evaluated per pair
     int* ddnbr = nullptr;
     int* ddcnt = nullptr;
@@ -1092,6 +1094,124 @@ int autotune(mdff_ctx* ctx) {
     return check_launch(ctx, "autotune");
 }
 
+// The most CTAs that share a 128-atom tile when ntile x ncb units are cut into
+// `grid` ranges.
+size_t tile_slots(int ntile, int ncb, int grid) {
+    const long U = (long)ntile * ncb;
+    int m = 1;
+    for (int b = 0; b < ntile; ++b)
+        m = std::max(m, umma::range_of((long)b * ncb + ncb - 1, U, grid) - umma::range_of((long)b * ncb, U, grid) + 1);
+    return (size_t)m;
+}
+
+// Plan and buffers of the FP64 path's tensor-core reciprocal space for the columns
+// that hold wave vectors; off (the CUDA-core kernels run) when kz > 31, where the
+// seven digit levels of one tile no longer fit tensor memory, or when a tile's
+// tables do not fit shared memory.
+int plan_t7(mdff_ctx* ctx) {
+    const KGrid& kg = ctx->kg;
+    T7K& t = ctx->rs.t7;
+    const int n = ctx->n;
+    t.kx = kg.kmax[0]; t.ky = kg.kmax[1]; t.kz = kg.kmax[2]; t.nzl = kg.nzl;
+    t.N = ((2 * (t.kz + 1) + 15) / 16) * 16;
+    t.KZ = ((2 * (t.kz + 1) + 31) / 32) * 32;
+    if (t.N > tc7::NLEV_MAX || t.KZ > tc7::FK_MAX) return MDFF_OK;
+    const int nyn = 2 * t.ky + 1;
+    const std::vector<char>& has = ctx->kcol;
+    std::vector<int> cols, pairs, tr;
+    for (int col = 0; col < kg.ncol; ++col)
+        if (has[col]) cols.push_back(col);
+    for (int nx = 0; nx <= t.kx; ++nx)
+        for (int ny = 0; ny <= t.ky; ++ny)
+            if (has[nx * nyn + t.ky + ny] || has[nx * nyn + t.ky - ny]) { pairs.push_back(nx); pairs.push_back(ny); }
+    if (cols.empty()) return MDFF_OK;
+    t.ncol = (int)cols.size();
+    t.npair = (int)(pairs.size() / 2);
+    t.ntile = (t.npair + tc7::TP - 1) / tc7::TP;
+    t.pstride = t.ntile * tc7::TP;
+    for (int b = 0; b < t.ntile; ++b) {
+        int x0 = t.kx, x1 = 0, y0 = t.ky, y1 = 0;
+        for (int q = b * tc7::TP; q < std::min(t.npair, (b + 1) * tc7::TP); ++q) {
+            x0 = std::min(x0, pairs[2 * q]); x1 = std::max(x1, pairs[2 * q]);
+            y0 = std::min(y0, pairs[2 * q + 1]); y1 = std::max(y1, pairs[2 * q + 1]);
+        }
+        tr.insert(tr.end(), {x0, x1 - x0 + 1, y0, y1 - y0 + 1});
+        t.entmax = std::max(t.entmax, x1 - x0 + 1 + y1 - y0 + 1);
+    }
+    const size_t smax = 227 * 1024 - 2048;   // static shared memory aside
+    t.nin = tc7::Layout::depth(t.N, t.entmax, smax);
+    if (t.nin < 2) return MDFF_OK;
+    const tc7::Layout lay(t.N, t.entmax, t.nin);
+    t.smem = lay.smem_bytes();
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->p.device);
+    // atoms split so that the grid covers the SMs about once
+    t.nblk = (n + tc7::SA - 1) / tc7::SA;
+    t.npad = t.nblk * tc7::SA;
+    const int S = std::max(1, sms / t.ntile);
+    t.bps = std::min(std::max(1, (t.nblk + S - 1) / S), tc7::MAX_BLOCKS_PER_CTA);
+    t.nsplit = (t.nblk + t.bps - 1) / t.bps;
+    t.ntile_f = (n + 127) / 128;
+    t.ncb2 = (t.ncol + tc7::Cfg<2>::CB - 1) / tc7::Cfg<2>::CB;
+    t.ncb3 = (t.ncol + tc7::Cfg<3>::CB - 1) / tc7::Cfg<3>::CB;
+    t.grid2 = (int)std::min<long>((long)t.ntile_f * t.ncb2, sms);
+    t.grid3 = (int)std::min<long>((long)t.ntile_f * t.ncb3, sms);
+    const tc7::FLayout f2(t.KZ, tc7::Cfg<2>::CB), f3(t.KZ, tc7::Cfg<3>::CB);
+    t.smem_f2 = f2.smem_bytes();
+    t.smem_f3 = f3.smem_bytes();
+    // one allocation
+    const int ent = t.kx + t.ky + 2;
+    size_t at = 0;
+    auto place = [&](auto** q, size_t count) {   // at the base once it is known
+        if (ctx->rs.t7_buf) *q = reinterpret_cast<std::remove_pointer_t<decltype(q)>>(ctx->rs.t7_buf + at);
+        at = (at + sizeof(**q) * count + 255) & ~(size_t)255;
+    };
+    auto carve = [&]() {
+        at = 0;
+        place(&t.pairs, pairs.size());
+        place(&t.trange, tr.size());
+        place(&t.cols, cols.size());
+        place(&t.xy, (size_t)t.nblk * ent * tc7::AP);
+        place(&t.bimg, (size_t)t.nblk * lay.b_bytes());
+        place(&t.aimg, (size_t)t.ntile_f * f2.a_bytes);
+        place(&t.prm, (size_t)t.npad);
+        place(&t.bmax, (size_t)t.nblk);
+        place(&t.fimg, std::max((size_t)t.ncb2 * f2.stage_bytes, (size_t)t.ncb3 * f3.stage_bytes));
+        place(&ctx->rs.part, (size_t)t.nsplit * 4 * t.N * t.pstride);
+        place(&ctx->rs.fpart, (size_t)n * tc7::NQ *
+                                  std::max(3 * tile_slots(t.ntile_f, t.ncb2, t.grid2), 9 * tile_slots(t.ntile_f, t.ncb3, t.grid3)));
+    };
+    ctx->rs.t7_buf = nullptr;
+    carve();
+    TRY(dalloc(ctx, &ctx->rs.t7_buf, at));
+    carve();
+    CK(cudaMemcpyAsync(t.pairs, pairs.data(), sizeof(int) * pairs.size(), cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaMemcpyAsync(t.trange, tr.data(), sizeof(int) * tr.size(), cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaMemcpyAsync(t.cols, cols.data(), sizeof(int) * cols.size(), cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaStreamSynchronize(ctx->st));   // the host vectors go out of scope
+    // one limit for every context of the process, whatever its sizes
+    CK(cudaFuncSetAttribute(tc7::k_sfac_t7, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax));
+    CK(cudaFuncSetAttribute(tc7::k_kfield_t7<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax));
+    CK(cudaFuncSetAttribute(tc7::k_kfield_t7<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax));
+    t.on = 1;
+    return MDFF_OK;
+}
+
+// The FP64 path's reciprocal space, made by the first evaluation that needs it: an
+// engine for g(r), Monte Carlo or statistics alone is not charged for it.
+int ensure_rec(mdff_ctx* ctx) {
+    if (ctx->rec_ready) return MDFF_OK;
+    TRY(plan_t7(ctx));
+    if (!ctx->rs.t7.on) {
+        size_t fp = 0;
+        const size_t pc = rec_scratch_doubles(ctx->n, ctx->kg, &fp, 0);
+        TRY(dalloc(ctx, &ctx->rs.part, pc));
+        TRY(dalloc(ctx, &ctx->rs.fpart, fp));
+    }
+    ctx->rec_ready = true;
+    return MDFF_OK;
+}
+
 int engforce_finish(mdff_ctx* ctx);
 
 // engforce_driver (src/field.f90:1111-1166) on the device; results stay in
@@ -1103,6 +1223,7 @@ int engforce_device(mdff_ctx* ctx) {
     const int n = ctx->n;
     const mdff_params& p = ctx->p;
     const bool efg = p.doefg && ctx->efg_due;
+    if (p.lcoulomb && p.precision == MDFF_PREC_FP64) TRY(ensure_rec(ctx));
     const bool fresh = ctx->rec_fresh;   // of this evaluation alone, also when it fails below
     ctx->rec_fresh = false;
     const bool built = !p.lvnlist || !ctx->have_list;
@@ -1246,97 +1367,6 @@ int engforce_finish(mdff_ctx* ctx) {
     double usum = ctx->en.u_lj + ctx->en.u_bmhft + ctx->en.u_morse + ctx->en.u_coul;
     if (!std::isfinite(usum)) return fail(ctx, MDFF_E_NONFINITE, "non-finite energy");
     ctx->forces_valid = true;
-    return MDFF_OK;
-}
-
-// The most CTAs that share a 128-atom tile when ntile x ncb units are cut into
-// `grid` ranges.
-size_t tile_slots(int ntile, int ncb, int grid) {
-    const long U = (long)ntile * ncb;
-    int m = 1;
-    for (int b = 0; b < ntile; ++b)
-        m = std::max(m, umma::range_of((long)b * ncb + ncb - 1, U, grid) - umma::range_of((long)b * ncb, U, grid) + 1);
-    return (size_t)m;
-}
-
-// Plan and buffers of the FP64 path's tensor-core reciprocal space for the
-// vectors with ak != 0; off (the CUDA-core kernels run) when kz > 31, where the
-// seven digit levels of one tile no longer fit tensor memory, or when a tile's
-// tables do not fit shared memory.
-int plan_t7(mdff_ctx* ctx, const std::vector<double>& ak, size_t* part, size_t* fpart) {
-    const KGrid& kg = ctx->kg;
-    T7K& t = ctx->rs.t7;
-    const int n = ctx->n;
-    t.kx = kg.kmax[0]; t.ky = kg.kmax[1]; t.kz = kg.kmax[2]; t.nzl = kg.nzl;
-    t.N = ((2 * (t.kz + 1) + 15) / 16) * 16;
-    t.KZ = ((2 * (t.kz + 1) + 31) / 32) * 32;
-    if (t.N > tc7::NLEV_MAX || t.KZ > tc7::FK_MAX) return MDFF_OK;
-    const int nyn = 2 * t.ky + 1;
-    std::vector<int> cols, pairs, tr;
-    std::vector<char> has(kg.ncol, 0);
-    for (int col = 0; col < kg.ncol; ++col) {
-        for (int m = 0; m < kg.nzl; ++m) has[col] |= ak[(size_t)col * kg.nzl + m] != 0.0;
-        if (has[col]) cols.push_back(col);
-    }
-    for (int nx = 0; nx <= t.kx; ++nx)
-        for (int ny = 0; ny <= t.ky; ++ny)
-            if (has[nx * nyn + t.ky + ny] || has[nx * nyn + t.ky - ny]) { pairs.push_back(nx); pairs.push_back(ny); }
-    if (cols.empty()) return MDFF_OK;
-    t.ncol = (int)cols.size();
-    t.npair = (int)(pairs.size() / 2);
-    t.ntile = (t.npair + tc7::TP - 1) / tc7::TP;
-    t.pstride = t.ntile * tc7::TP;
-    for (int b = 0; b < t.ntile; ++b) {
-        int x0 = t.kx, x1 = 0, y0 = t.ky, y1 = 0;
-        for (int q = b * tc7::TP; q < std::min(t.npair, (b + 1) * tc7::TP); ++q) {
-            x0 = std::min(x0, pairs[2 * q]); x1 = std::max(x1, pairs[2 * q]);
-            y0 = std::min(y0, pairs[2 * q + 1]); y1 = std::max(y1, pairs[2 * q + 1]);
-        }
-        tr.insert(tr.end(), {x0, x1 - x0 + 1, y0, y1 - y0 + 1});
-        t.entmax = std::max(t.entmax, x1 - x0 + 1 + y1 - y0 + 1);
-    }
-    const size_t smax = 227 * 1024 - 2048;   // static shared memory aside
-    t.nin = tc7::Layout::depth(t.N, t.entmax, smax);
-    if (t.nin < 2) return MDFF_OK;
-    const tc7::Layout lay(t.N, t.entmax, t.nin);
-    t.smem = lay.smem_bytes();
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->p.device);
-    // atoms split so that the grid covers the SMs about once
-    t.nblk = (n + tc7::SA - 1) / tc7::SA;
-    t.npad = t.nblk * tc7::SA;
-    const int S = std::max(1, sms / t.ntile);
-    t.bps = std::min(std::max(1, (t.nblk + S - 1) / S), tc7::MAX_BLOCKS_PER_CTA);
-    t.nsplit = (t.nblk + t.bps - 1) / t.bps;
-    t.ntile_f = (n + 127) / 128;
-    t.ncb2 = (t.ncol + tc7::Cfg<2>::CB - 1) / tc7::Cfg<2>::CB;
-    t.ncb3 = (t.ncol + tc7::Cfg<3>::CB - 1) / tc7::Cfg<3>::CB;
-    t.grid2 = (int)std::min<long>((long)t.ntile_f * t.ncb2, sms);
-    t.grid3 = (int)std::min<long>((long)t.ntile_f * t.ncb3, sms);
-    const tc7::FLayout f2(t.KZ, tc7::Cfg<2>::CB), f3(t.KZ, tc7::Cfg<3>::CB);
-    t.smem_f2 = f2.smem_bytes();
-    t.smem_f3 = f3.smem_bytes();
-    *part = (size_t)t.nsplit * 4 * t.N * t.pstride;
-    *fpart = (size_t)n * tc7::NQ * std::max(3 * tile_slots(t.ntile_f, t.ncb2, t.grid2), 9 * tile_slots(t.ntile_f, t.ncb3, t.grid3));
-    const int ent = t.kx + t.ky + 2;
-    TRY(dalloc(ctx, &t.pairs, pairs.size()));
-    TRY(dalloc(ctx, &t.trange, tr.size()));
-    TRY(dalloc(ctx, &t.cols, cols.size()));
-    TRY(dalloc(ctx, &t.xy, (size_t)t.nblk * ent * tc7::AP));
-    TRY(dalloc(ctx, &t.bimg, (size_t)t.nblk * lay.b_bytes()));
-    TRY(dalloc(ctx, &t.aimg, (size_t)t.ntile_f * f2.a_bytes));
-    TRY(dalloc(ctx, &t.prm, (size_t)t.npad));
-    TRY(dalloc(ctx, &t.bmax, (size_t)t.nblk));
-    TRY(dalloc(ctx, &t.fimg, std::max((size_t)t.ncb2 * f2.stage_bytes, (size_t)t.ncb3 * f3.stage_bytes)));
-    CK(cudaMemcpyAsync(t.pairs, pairs.data(), sizeof(int) * pairs.size(), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(t.trange, tr.data(), sizeof(int) * tr.size(), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(t.cols, cols.data(), sizeof(int) * cols.size(), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));   // the host vectors go out of scope
-    // one limit for every context of the process, whatever its sizes
-    CK(cudaFuncSetAttribute(tc7::k_sfac_t7, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax));
-    CK(cudaFuncSetAttribute(tc7::k_kfield_t7<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax));
-    CK(cudaFuncSetAttribute(tc7::k_kfield_t7<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax));
-    t.on = 1;
     return MDFF_OK;
 }
 
@@ -1695,6 +1725,7 @@ bool graph_eligible(const mdff_ctx* ctx) {
     if (p.lcoulomb && p.precision == MDFF_PREC_MIXED &&
         (!ctx->ddcnt || !ctx->ddrec || (size_t)ctx->n * coul_list(ctx).cap > ctx->ddtab_cap))
         return false;
+    if (p.lcoulomb && p.precision == MDFF_PREC_FP64 && !ctx->rec_ready) return false;
     if (p.lcoulomb && p.precision == MDFF_PREC_FP64 && ctx->npol > 0 && !ctx->ddtab_off &&
         (!ctx->ddcnt || (size_t)ctx->n * coul_list(ctx).cap > ctx->ddtab_cap))
         return false;
@@ -3235,10 +3266,11 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
     TRY(dalloc(ctx, &ctx->hist, (size_t)ctx->nhist * 3 * n));
     TRY(dalloc(ctx, &ctx->coef, PLAN_LEN));
     TRY(dalloc(ctx, &ctx->type, n));
-    TRY(dalloc(ctx, &ctx->rec, n));
-    TRY(dalloc(ctx, &ctx->aos, 6 * (size_t)n));
-    TRY(dalloc(ctx, &ctx->part2, 3 * (size_t)nb(n)));
-    TRY(dalloc(ctx, &ctx->mrec, n));
+    // (one allocation: each costs an engine's creation about as much as a small system)
+    TRY(dalloc(ctx, &ctx->rec, 2 * (size_t)n + (6 * (size_t)n + 3 * (size_t)nb(n) + 3) / 4));
+    ctx->mrec = ctx->rec + n;
+    ctx->aos = reinterpret_cast<double*>(ctx->mrec + n);
+    ctx->part2 = ctx->aos + 6 * (size_t)n;
     TRY(dalloc(ctx, &ctx->pc, NT * NT));
     TRY(dalloc(ctx, &ctx->dsc, 1));
     TRY(dalloc(ctx, &ctx->d_overflow, 1));
@@ -3580,28 +3612,30 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
             CK(cudaMemcpyAsync(kg.mask, mk.data(), kg.nrect, cudaMemcpyHostToDevice, ctx->st));
             CK(cudaStreamSynchronize(ctx->st));
         }
-        size_t fp = 0, pc = 0;
         ctx->rs.t7 = T7K();
-        if (p.precision == MDFF_PREC_FP64) TRY(plan_t7(ctx, ak, &pc, &fp));
-        if (!ctx->rs.t7.on) {
-            pc = std::max(tc_part, rec_scratch_doubles(n, kg, &fp, p.precision == MDFF_PREC_MIXED));
+        ctx->rec_ready = false;
+        ctx->kcol.assign(kg.ncol, 0);
+        for (int r = 0; r < kg.nrect; ++r) ctx->kcol[r / kg.nzl] |= ak[r] != 0.0;
+        if (p.precision == MDFF_PREC_MIXED) {
+            size_t fp = 0;
+            const size_t pc = std::max(tc_part, rec_scratch_doubles(n, kg, &fp, 1));
+            fp = std::max(fp, (size_t)2 * tcf::NQ * 9 * n);   // tensor-core field pass: NQ column parts x 2 column slots
+            TRY(dalloc(ctx, &ctx->rs.part, pc));
+            TRY(dalloc(ctx, &ctx->rs.fpart, fp));
         }
-        if (p.precision == MDFF_PREC_MIXED)   // tensor-core field pass: NQ column parts x 2 column slots
-            fp = std::max(fp, (size_t)2 * tcf::NQ * 9 * n);
-        TRY(dalloc(ctx, &ctx->rs.part, pc));
-        TRY(dalloc(ctx, &ctx->rs.fpart, fp));
         TRY(dalloc(ctx, &ctx->rs.aks, 2 * (size_t)kg.nrect));
         TRY(dalloc(ctx, &ctx->rs.aks_acc, 2 * (size_t)kg.nrect));
         CK(cudaMemsetAsync(ctx->rs.aks, 0, sizeof(double) * 2 * kg.nrect, ctx->st));   // vectors no pass writes
         TRY(dalloc(ctx, &ctx->rs.fixed, 3 * (size_t)n));
         TRY(dalloc(ctx, &ctx->rs.tab, (size_t)n * 16));
         TRY(dalloc(ctx, &ctx->rs.aks2, (size_t)kg.ncol * (((kg.nzl + 15) / 16) * 16)));
-        ctx->rs.part_cap = pc;
-        ctx->rs.fpart_cap = fp;
     }
     int parts = std::max(16 * 1024, 12 * (int)(((size_t)n * 32 + 255) / 256));
-    if (p.lcoulomb)   // energy and stress sums of the structure factor's reductions
-        parts = std::max(parts, 7 * std::max(ctx->rs.t7.ntile * (ctx->rs.t7.kz + 1), (ctx->kg.nrect + 31) / 32));
+    if (p.lcoulomb) {   // energy and stress sums of the structure factor's reductions
+        const int* km = ctx->kg.kmax;
+        const int tiles7 = ((km[0] + 1) * (km[1] + 1) + tc7::TP - 1) / tc7::TP;   // at most
+        parts = std::max(parts, 7 * std::max(tiles7 * (km[2] + 1), (ctx->kg.nrect + 31) / 32));
+    }
     TRY(dalloc(ctx, &ctx->part.buf, parts));
     ctx->part.capacity = parts;
     // neighbour lists

@@ -322,11 +322,9 @@ struct T7K {
 
 struct RecScratch {
     double* part = nullptr;    // structure-factor partials
-    size_t part_cap = 0;       // doubles
     double* aks = nullptr;     // [2][nrect] Ak*S (re, im)
     double* aks_acc = nullptr; // [2][nrect] solver accumulator of Ak*S (reuse of structure factors)
     double* fpart = nullptr;   // per-atom field partials [split][9][n]
-    size_t fpart_cap = 0;
     uint32_t* fixed = nullptr;  // [3][n] fractional coordinates as 32-bit fixed point
     float2* tab = nullptr;      // [n][16] e^{2 pi i m s_z}
     float4* aks2 = nullptr;     // [ncol][nzp] A_k S(k) padded, FP32 pairs (re, re, im, im)
@@ -336,6 +334,7 @@ struct RecScratch {
     LowK low;
     TcK tc;
     T7K t7;
+    uint8_t* t7_buf = nullptr;  // its buffers, part and fpart
 };
 struct RecFlags {
     int with_q, with_mu;

@@ -48,3 +48,17 @@ def test_pair_table(m, left):
         free = torch.cuda.mem_get_info()[0]
     compare(got, want)
     assert left < 256 or free > 0.8 * (left << 20)
+
+
+def test_creation():
+    """The reciprocal space's buffers are the first evaluation's: a context that evaluates no
+    force does without them."""
+    s = systems.mgo_pim(grid=(48, 48, 48), rc=5.0, alpha=0.6, kmax=8, seed=4)
+    args = [s[k] for k in ("params", "itype", "pos", "cell")]
+    free = torch.cuda.mem_get_info()[0]
+    eng = mdff_b200.Engine(*args)
+    made = torch.cuda.mem_get_info()[0]
+    eng.gr(4.0, 0.1)
+    torch.cuda.synchronize()
+    eng.engforce()
+    assert free - made < 240 << 20 and made - torch.cuda.mem_get_info()[0] > 100 << 20
