@@ -1106,8 +1106,8 @@ size_t tile_slots(int ntile, int ncb, int grid) {
 
 // Plan and buffers of the FP64 path's tensor-core reciprocal space for the columns
 // that hold wave vectors; off (the CUDA-core kernels run) when kz > 31, where the
-// seven digit levels of one tile no longer fit tensor memory, or when a tile's
-// tables do not fit shared memory.
+// seven digit levels of one tile no longer fit tensor memory, when a tile's
+// tables do not fit shared memory, or when there is no memory for the buffers.
 int plan_t7(mdff_ctx* ctx) {
     const KGrid& kg = ctx->kg;
     T7K& t = ctx->rs.t7;
@@ -1159,7 +1159,7 @@ int plan_t7(mdff_ctx* ctx) {
     const tc7::FLayout f2(t.KZ, tc7::Cfg<2>::CB), f3(t.KZ, tc7::Cfg<3>::CB);
     t.smem_f2 = f2.smem_bytes();
     t.smem_f3 = f3.smem_bytes();
-    // one allocation
+    // one allocation, all of it or nothing
     const int ent = t.kx + t.ky + 2;
     size_t at = 0;
     auto place = [&](auto** q, size_t count) {   // at the base once it is known
@@ -1183,7 +1183,7 @@ int plan_t7(mdff_ctx* ctx) {
     };
     ctx->rs.t7_buf = nullptr;
     carve();
-    TRY(dalloc(ctx, &ctx->rs.t7_buf, at));
+    if (dalloc(ctx, &ctx->rs.t7_buf, at) != MDFF_OK) return MDFF_OK;
     carve();
     CK(cudaMemcpyAsync(t.pairs, pairs.data(), sizeof(int) * pairs.size(), cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(t.trange, tr.data(), sizeof(int) * tr.size(), cudaMemcpyHostToDevice, ctx->st));
