@@ -350,6 +350,9 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
         }
     }
+    // every MMA has completed before the tensor memory is released, also when the
+    // pipeline was abandoned on an error (bounded, whatever the stop flag)
+    if (warp == 0 && nst > 0 && !umma::mbar_wait_ns(&done, 0, WAIT_NS)) atomicOr(err, 16);
     umma::fence_before_sync();
     __syncthreads();
     if (warp == 0) {
@@ -795,8 +798,9 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
         }
     }
-    // every MMA has completed before the tensor memory is released
-    if (warp == 0) f_wait(&fin, 0, err, 64, &abort_);
+    // every MMA has completed before the tensor memory is released, also when the
+    // pipeline was abandoned on an error (bounded, whatever the abort flag)
+    if (warp == 0 && !umma::mbar_wait_ns(&fin, 0, WAIT_NS)) atomicOr(err, 64);
     umma::fence_before_sync();
     __syncthreads();
     if (warp == 0) {

@@ -419,6 +419,9 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
         }
     }
+    // every MMA has completed before the tensor memory is released, also when the
+    // pipeline was abandoned on an error (bounded, whatever the stop flag)
+    if (warp == 0 && !umma::mbar_wait_ns(&done, 0, WAIT_NS)) atomicOr(err, 1 << 13);
     umma::fence_before_sync();
     __syncthreads();
     if (warp == 0) {
@@ -870,8 +873,9 @@ __global__ void __launch_bounds__(FTHREADS, 1)
             if (++q == ncb) { q = 0; ++tile; }
         }
     }
-    // every MMA has completed before the tensor memory is released
-    if (warp == 0) wait(&fin, 0, err, 1 << 21, &stop);
+    // every MMA has completed before the tensor memory is released, also when the
+    // pipeline was abandoned on an error (bounded, whatever the stop flag)
+    if (warp == 0 && !umma::mbar_wait_ns(&fin, 0, WAIT_NS)) atomicOr(err, 1 << 21);
     umma::fence_before_sync();
     __syncthreads();
     if (warp == 0) {
