@@ -142,8 +142,6 @@ struct mdff_ctx {
     // Coulomb list entry), written by the charge pass of each force evaluation
     float2* ddtab = nullptr;
     double2* ddtab64 = nullptr;          // FP64 path
-    bool rec_ready = false;              // the FP64 path's reciprocal space is planned and allocated (ensure_rec)
-    std::vector<char> kcol;              // which columns of the k rectangle hold wave vectors
     bool ddtab_off = false;              // FP64 path: no memory for the table, the operator is evaluated per pair
     int* ddnbr = nullptr;
     int* ddcnt = nullptr;
@@ -1104,11 +1102,11 @@ size_t tile_slots(int ntile, int ncb, int grid) {
     return (size_t)m;
 }
 
-// Plan and buffers of the FP64 path's tensor-core reciprocal space for the columns
-// that hold wave vectors; off (the CUDA-core kernels run) when kz > 31, where the
+// Plan and buffers of the FP64 path's tensor-core reciprocal space for the
+// vectors with ak != 0; off (the CUDA-core kernels run) when kz > 31, where the
 // seven digit levels of one tile no longer fit tensor memory, when a tile's
 // tables do not fit shared memory, or when there is no memory for the buffers.
-int plan_t7(mdff_ctx* ctx) {
+int plan_t7(mdff_ctx* ctx, const std::vector<double>& ak) {
     const KGrid& kg = ctx->kg;
     T7K& t = ctx->rs.t7;
     const int n = ctx->n;
@@ -1117,10 +1115,12 @@ int plan_t7(mdff_ctx* ctx) {
     t.KZ = ((2 * (t.kz + 1) + 31) / 32) * 32;
     if (t.N > tc7::NLEV_MAX || t.KZ > tc7::FK_MAX) return MDFF_OK;
     const int nyn = 2 * t.ky + 1;
-    const std::vector<char>& has = ctx->kcol;
     std::vector<int> cols, pairs, tr;
-    for (int col = 0; col < kg.ncol; ++col)
+    std::vector<char> has(kg.ncol, 0);
+    for (int col = 0; col < kg.ncol; ++col) {
+        for (int m = 0; m < kg.nzl; ++m) has[col] |= ak[(size_t)col * kg.nzl + m] != 0.0;
         if (has[col]) cols.push_back(col);
+    }
     for (int nx = 0; nx <= t.kx; ++nx)
         for (int ny = 0; ny <= t.ky; ++ny)
             if (has[nx * nyn + t.ky + ny] || has[nx * nyn + t.ky - ny]) { pairs.push_back(nx); pairs.push_back(ny); }
@@ -1159,7 +1159,7 @@ int plan_t7(mdff_ctx* ctx) {
     const tc7::FLayout f2(t.KZ, tc7::Cfg<2>::CB), f3(t.KZ, tc7::Cfg<3>::CB);
     t.smem_f2 = f2.smem_bytes();
     t.smem_f3 = f3.smem_bytes();
-    // one allocation, all of it or nothing
+    // one allocation (eleven took 2.5 ms of a context's creation): all of it or nothing
     const int ent = t.kx + t.ky + 2;
     size_t at = 0;
     auto place = [&](auto** q, size_t count) {   // at the base once it is known
@@ -1197,21 +1197,6 @@ int plan_t7(mdff_ctx* ctx) {
     return MDFF_OK;
 }
 
-// The FP64 path's reciprocal space, made by the first evaluation that needs it: an
-// engine for g(r), Monte Carlo or statistics alone is not charged for it.
-int ensure_rec(mdff_ctx* ctx) {
-    if (ctx->rec_ready) return MDFF_OK;
-    TRY(plan_t7(ctx));
-    if (!ctx->rs.t7.on) {
-        size_t fp = 0;
-        const size_t pc = rec_scratch_doubles(ctx->n, ctx->kg, &fp, 0);
-        TRY(dalloc(ctx, &ctx->rs.part, pc));
-        TRY(dalloc(ctx, &ctx->rs.fpart, fp));
-    }
-    ctx->rec_ready = true;
-    return MDFF_OK;
-}
-
 int engforce_finish(mdff_ctx* ctx);
 
 // engforce_driver (src/field.f90:1111-1166) on the device; results stay in
@@ -1223,7 +1208,6 @@ int engforce_device(mdff_ctx* ctx) {
     const int n = ctx->n;
     const mdff_params& p = ctx->p;
     const bool efg = p.doefg && ctx->efg_due;
-    if (p.lcoulomb && p.precision == MDFF_PREC_FP64) TRY(ensure_rec(ctx));
     const bool fresh = ctx->rec_fresh;   // of this evaluation alone, also when it fails below
     ctx->rec_fresh = false;
     const bool built = !p.lvnlist || !ctx->have_list;
@@ -1725,7 +1709,6 @@ bool graph_eligible(const mdff_ctx* ctx) {
     if (p.lcoulomb && p.precision == MDFF_PREC_MIXED &&
         (!ctx->ddcnt || !ctx->ddrec || (size_t)ctx->n * coul_list(ctx).cap > ctx->ddtab_cap))
         return false;
-    if (p.lcoulomb && p.precision == MDFF_PREC_FP64 && !ctx->rec_ready) return false;
     if (p.lcoulomb && p.precision == MDFF_PREC_FP64 && ctx->npol > 0 && !ctx->ddtab_off &&
         (!ctx->ddcnt || (size_t)ctx->n * coul_list(ctx).cap > ctx->ddtab_cap))
         return false;
@@ -3613,13 +3596,12 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
             CK(cudaStreamSynchronize(ctx->st));
         }
         ctx->rs.t7 = T7K();
-        ctx->rec_ready = false;
-        ctx->kcol.assign(kg.ncol, 0);
-        for (int r = 0; r < kg.nrect; ++r) ctx->kcol[r / kg.nzl] |= ak[r] != 0.0;
-        if (p.precision == MDFF_PREC_MIXED) {
+        if (p.precision == MDFF_PREC_FP64) TRY(plan_t7(ctx, ak));
+        if (!ctx->rs.t7.on) {
+            const bool mixed = p.precision == MDFF_PREC_MIXED;
             size_t fp = 0;
-            const size_t pc = std::max(tc_part, rec_scratch_doubles(n, kg, &fp, 1));
-            fp = std::max(fp, (size_t)2 * tcf::NQ * 9 * n);   // tensor-core field pass: NQ column parts x 2 column slots
+            const size_t pc = std::max(tc_part, rec_scratch_doubles(n, kg, &fp, mixed));
+            if (mixed) fp = std::max(fp, (size_t)2 * tcf::NQ * 9 * n);   // tensor-core field pass: NQ column parts x 2 column slots
             TRY(dalloc(ctx, &ctx->rs.part, pc));
             TRY(dalloc(ctx, &ctx->rs.fpart, fp));
         }

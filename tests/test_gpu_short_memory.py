@@ -65,17 +65,3 @@ def test_reciprocal_space():
         if k == "ef":   # (another order of summation: the other kernels ran)
             assert not np.array_equal(got[k], want[k])
     assert abs(got["e"]["u_rec"] - want["e"]["u_rec"]) <= 1e-11 * abs(want["e"]["u_rec"])
-
-
-def test_creation():
-    """The reciprocal space's buffers are the first evaluation's: a context that evaluates no
-    force does without them."""
-    s = systems.mgo_pim(grid=(48, 48, 48), rc=5.0, alpha=0.6, kmax=8, seed=4)
-    args = [s[k] for k in ("params", "itype", "pos", "cell")]
-    free = torch.cuda.mem_get_info()[0]
-    eng = mdff_b200.Engine(*args)
-    made = torch.cuda.mem_get_info()[0]
-    eng.gr(4.0, 0.1)
-    torch.cuda.synchronize()
-    eng.engforce()
-    assert free - made < 240 << 20 and made - torch.cuda.mem_get_info()[0] > 100 << 20
