@@ -1102,11 +1102,11 @@ size_t tile_slots(int ntile, int ncb, int grid) {
     return (size_t)m;
 }
 
-// Plan and buffers of the FP64 path's tensor-core reciprocal space for the
-// vectors with ak != 0; off (the CUDA-core kernels run) when kz > 31, where the
+// Plan and buffers of the FP64 path's tensor-core reciprocal space for the columns
+// that hold wave vectors (has); off (the CUDA-core kernels run) when kz > 31, where the
 // seven digit levels of one tile no longer fit tensor memory, when a tile's
-// tables do not fit shared memory, or when there is no memory for the buffers.
-int plan_t7(mdff_ctx* ctx, const std::vector<double>& ak) {
+// tables do not fit shared memory, or when the buffers do not fit device memory.
+int plan_t7(mdff_ctx* ctx, const std::vector<char>& has) {
     const KGrid& kg = ctx->kg;
     T7K& t = ctx->rs.t7;
     const int n = ctx->n;
@@ -1116,11 +1116,8 @@ int plan_t7(mdff_ctx* ctx, const std::vector<double>& ak) {
     if (t.N > tc7::NLEV_MAX || t.KZ > tc7::FK_MAX) return MDFF_OK;
     const int nyn = 2 * t.ky + 1;
     std::vector<int> cols, pairs, tr;
-    std::vector<char> has(kg.ncol, 0);
-    for (int col = 0; col < kg.ncol; ++col) {
-        for (int m = 0; m < kg.nzl; ++m) has[col] |= ak[(size_t)col * kg.nzl + m] != 0.0;
+    for (int col = 0; col < kg.ncol; ++col)
         if (has[col]) cols.push_back(col);
-    }
     for (int nx = 0; nx <= t.kx; ++nx)
         for (int ny = 0; ny <= t.ky; ++ny)
             if (has[nx * nyn + t.ky + ny] || has[nx * nyn + t.ky - ny]) { pairs.push_back(nx); pairs.push_back(ny); }
@@ -1183,7 +1180,7 @@ int plan_t7(mdff_ctx* ctx, const std::vector<double>& ak) {
     };
     ctx->rs.t7_buf = nullptr;
     carve();
-    if (dalloc(ctx, &ctx->rs.t7_buf, at) != MDFF_OK) return MDFF_OK;
+    if (!table_fits(at) || dalloc(ctx, &ctx->rs.t7_buf, at) != MDFF_OK) return MDFF_OK;
     carve();
     CK(cudaMemcpyAsync(t.pairs, pairs.data(), sizeof(int) * pairs.size(), cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(t.trange, tr.data(), sizeof(int) * tr.size(), cudaMemcpyHostToDevice, ctx->st));
@@ -3280,6 +3277,7 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
     TRY(upload(ctx, ctx->z, rz, n));
     launch_wrap_positions(ctx->st, n, ctx->x, ctx->y, ctx->z, ctx->cell);
     // Ewald k grid (kpoint_sum_init, src/kspace.f90:142-207) as a full rectangle
+    std::vector<char> kcol;   // which of its columns hold wave vectors
     if (p.lcoulomb) {
         KGrid& kg = ctx->kg;
         for (int d = 0; d < 3; ++d) kg.kmax[d] = ctx->kES[d];
@@ -3596,12 +3594,12 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
             CK(cudaStreamSynchronize(ctx->st));
         }
         ctx->rs.t7 = T7K();
-        if (p.precision == MDFF_PREC_FP64) TRY(plan_t7(ctx, ak));
-        if (!ctx->rs.t7.on) {
-            const bool mixed = p.precision == MDFF_PREC_MIXED;
+        kcol.assign(kg.ncol, 0);
+        for (int r = 0; r < kg.nrect; ++r) kcol[r / kg.nzl] |= ak[r] != 0.0;
+        if (p.precision == MDFF_PREC_MIXED) {
             size_t fp = 0;
-            const size_t pc = std::max(tc_part, rec_scratch_doubles(n, kg, &fp, mixed));
-            if (mixed) fp = std::max(fp, (size_t)2 * tcf::NQ * 9 * n);   // tensor-core field pass: NQ column parts x 2 column slots
+            const size_t pc = std::max(tc_part, rec_scratch_doubles(n, kg, &fp, 1));
+            fp = std::max(fp, (size_t)2 * tcf::NQ * 9 * n);   // tensor-core field pass: NQ column parts x 2 column slots
             TRY(dalloc(ctx, &ctx->rs.part, pc));
             TRY(dalloc(ctx, &ctx->rs.fpart, fp));
         }
@@ -3631,6 +3629,15 @@ int mdff_set_system(mdff_ctx* ctx, int natm, const int* itype, const double* rx,
     }
     ctx->list_cap = cap;
     TRY(ensure_lists(ctx, cap));
+    if (p.lcoulomb && p.precision == MDFF_PREC_FP64) {   // last: the tensor-core kernels where the rest leaves room for them
+        TRY(plan_t7(ctx, kcol));
+        if (!ctx->rs.t7.on) {
+            size_t fp = 0;
+            const size_t pc = rec_scratch_doubles(n, ctx->kg, &fp, 0);
+            TRY(dalloc(ctx, &ctx->rs.part, pc));
+            TRY(dalloc(ctx, &ctx->rs.fpart, fp));
+        }
+    }
     ctx->itime = 0;
     ctx->have_system = true;
     if (p.lvnlist) TRY(build_lists(ctx, p.skindiff));
