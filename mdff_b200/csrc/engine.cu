@@ -1010,6 +1010,18 @@ int dir_lanes(int n, const int* cand, int nc) {
     return best;
 }
 
+// Lanes per atom of k_ewald_ddtab64.  A warp an atom hides the latency of the
+// gathers best, unless the last of two waves is then mostly empty: four blocks of
+// eight atoms fit an SM.  Us at 16 and 32 lanes: 3 000 ions 20.1 and 18.1, 5 832 27.0
+// and 33.1, 9 600 47.5 and 45.4, 32 768 121 and 114.  (Timing the shapes at the first
+// evaluation took 36 launches, longer than the table saves there.)
+int table_lanes(int n) {
+    int sms = 148, dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const double waves = (double)n / 8.0 / (4.0 * sms);
+    return waves > 1.0 && waves < 2.0 ? 16 : 32;
+}
+
 int autotune(mdff_ctx* ctx) {
     ctx->tuned = true;
     if (!ctx->p.lcoulomb) return MDFF_OK;
@@ -1072,21 +1084,7 @@ int autotune(mdff_ctx* ctx) {
                              ctx->ef, nullptr, nullptr, ctx->part, ctx->dsc, &ctx->prof);
         }, muls, 3);
     }
-    if (ctx->p.precision == MDFF_PREC_FP64 && ctx->npol > 0) {
-        DirFlags fs = dir_flags(ctx);
-        fs.qq = 1;
-        fs.damp = 1;
-        fs.field = 1;
-        TRY(arm_ddtab(ctx, fs));
-        if (fs.ddtab64) {
-            launch_ewald_dir(ctx->st, n, ctx->rec, ctx->mrec, ctx->q, ctx->mu, ctx->cell, coul_list(ctx),
-                             ctx->pc, fs, ctx->Estat, nullptr, nullptr, ctx->part, ctx->dsc, ctx->g_dir);
-            ctx->g_dd = pick([&](int g) {
-                launch_ewald_ddtab64(ctx->st, n, ctx->rec, ctx->mrec, ctx->mu, ctx->cell, geom_of(ctx), ctx->ddnbr,
-                                     ctx->ddcnt, coul_list(ctx).cap, ctx->ddtab64, ctx->Eind, g);
-            }, gs, 3);
-        }
-    }
+    if (ctx->p.precision == MDFF_PREC_FP64 && ctx->npol > 0) ctx->g_dd = table_lanes(n);
     ctx->prof.on = prof_on;
     ctx->prof.launches = launches;
     return check_launch(ctx, "autotune");
