@@ -561,6 +561,13 @@ int geom_of(const mdff_ctx* ctx) {
     return diag ? GEOM_DIAGONAL : GEOM_GENERAL;
 }
 
+// Whether the short-range kernels take a warp an atom (launch_pair): by the cell the
+// system was set with, so that a restarted run sums as the one it goes on from.
+bool wide_rows(const mdff_ctx* ctx) {
+    const double rl = ctx->cut_vdw + (ctx->p.lvnlist ? ctx->p.skindiff : 0.0);
+    return ctx->omega0 < 150.0 * rl * rl * rl;
+}
+
 DirFlags dir_flags(const mdff_ctx* ctx) {
     DirFlags f;
     std::memset(&f, 0, sizeof f);
@@ -1223,7 +1230,7 @@ int engforce_device(mdff_ctx* ctx) {
         for (int a = 0; a < ctx->ntype; ++a)
             for (int b = 0; b < ctx->ntype; ++b) lj126 &= p.plj[a][b] == 6.0 && p.qlj[a][b] == 12.0;
         PairFlags fl{p.lnmlj, p.lbmhft, p.lbmhftd, p.lmorse, p.trunc, ctx->ntype, lj126, geom_of(ctx),
-                     p.precision == MDFF_PREC_FP64};
+                     p.precision == MDFF_PREC_FP64, wide_rows(ctx)};
         ctx->prof.begin(PK_PAIR);
         ctx->pair_blocks = launch_pair(ctx->st, n, ctx->rec, ctx->cell, ctx->lv, ctx->pc, fl, ctx->fx, ctx->fy, ctx->fz,
                                        ctx->part, ctx->dsc, !ctx->defer_pair);

@@ -192,7 +192,8 @@ void launch_skin_check(cudaStream_t st, int n, const double* sx, const double* s
 // Short-range pair loop: LJ / BMH(FTD) / Morse, forces written (not added).
 // lj126: every type pair has the exponents 6 and 12; geom: GEOM_* (common.cuh)
 // fast: the short forms of the pair arithmetic (FP64 path)
-struct PairFlags { int lj, bmh, bmhftd, morse, trunc, ntype, lj126, geom, fast; };
+// wide: 32 lanes an atom instead of 8
+struct PairFlags { int lj, bmh, bmhftd, morse, trunc, ntype, lj126, geom, fast, wide; };
 // rec: (fractional coordinates, type) of k_frac_rec.  sum: energies, virials and
 // stress into d->nonb; else the caller sums part (12 per block).  Returns the blocks.
 int launch_pair(cudaStream_t st, int n, const double4* rec, CellP c, const NList& l, const PairConst* pc, PairFlags fl,

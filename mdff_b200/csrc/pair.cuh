@@ -208,8 +208,13 @@ int launch_pair(cudaStream_t st, int n, const double4* rec, CellP c, const NList
     const bool bm = fl.bmh || fl.bmhftd;
     const int kind = !fl.fast ? -1 : fl.lj && !bm && !fl.morse && fl.lj126 ? 0 : (bm && !fl.lj && !fl.morse ? (fl.bmhftd ? 2 : 1) : -1);
 #define PAIR1(G, K) k_pair1<G, K><<<blocks, threads, 0, st>>>(n, rec, c, l.nbr, l.cnt, l.cap, pc, fl, fx, fy, fz, part.buf)
-    // lanes per atom: a warp each until the atoms alone fill the SMs
-    const bool wide = n < 24000;
+    // lanes per atom: 32 until the atoms fill the SMs with 8.  Where they cross depends on
+    // the length of the rows too: at 35 to 39 times as many atoms as list neighbours, that
+    // is a cell of about 150 cubes of the list radius (wide_rows).  Us at 8 and 32 lanes,
+    // Lennard-Jones rc 2.5: 2 048 atoms 17.5 and 14.5, 16 384 25.7 and 36.7; rc 4.5: 6 912 45.0
+    // and 36.0, 32 000 107 and 116; BMHFTD rc 6: 1 728 20.3 and 17.5, 13 824 29.9 and 38.7; rc 10:
+    // 4 096 52.1 and 39.2, 32 768 181 and 194.
+    const bool wide = fl.wide;
     if (kind >= 0) {
         blocks = grid(wide ? 32 : 8);
         if (kind == 0) { if (wide) PAIR1(32, 0); else PAIR1(8, 0); }
