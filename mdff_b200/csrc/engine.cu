@@ -4525,7 +4525,9 @@ int rmc_counts(mdff_ctx* ctx, const double* s, const RmcConst& k, const int* nbr
     const int n = ctx->n;
     const size_t smem = sizeof(int) * (size_t)k.ntype * k.ntype * k.nbins;
     const int in_smem = smem <= 48 * 1024 ? 1 : 0;
-    const int blocks = std::min((n + 7) / 8, 4 * 148);
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->p.device);
+    const int blocks = std::min((n + 7) / 8, 4 * sms);
     if (nbr)
         k_gr_rows<true><<<blocks, 256, in_smem ? smem : 0, ctx->st>>>(n, s, ctx->type, ctx->cell, k.bin, nbr, cnt, cap,
                                                                      in_smem, hist);
