@@ -1020,7 +1020,8 @@ int dir_lanes(int n, const int* cand, int nc) {
 // Lanes per atom of k_ewald_ddtab64.  A warp an atom hides the latency of the
 // gathers best, unless the last of two waves is then mostly empty: four blocks of
 // eight atoms fit an SM.  Us at 16 and 32 lanes: 3 000 ions 20.1 and 18.1, 5 832 27.0
-// and 33.1, 9 600 47.5 and 45.4, 32 768 121 and 114.  (Timing the shapes at the first
+// and 33.1, 9 600 47.5 and 45.4, 32 768 121 and 114; the worst case found, 4 096 ions at a
+// cutoff of 8 A, 17.3 and 19.5.  (Timing the shapes at the first
 // evaluation took 36 launches, longer than the table saves there.)
 int table_lanes(int n) {
     int sms = 148, dev = 0;

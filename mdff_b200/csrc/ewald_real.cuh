@@ -464,7 +464,7 @@ void launch_ewald_dd32(cudaStream_t st, int n, const uint32_t* fx, const double*
 #undef DD32
 }
 
-// g: lanes per atom (8, 16 or 32; the autotuner's choice).
+// g: lanes per atom (8, 16 or 32; the autotuner's choice, on the mixed path a rule).
 void launch_ewald_dir(cudaStream_t st, int n, const double4* rec, double4* mrec, const double* q, const double* mu,
                       CellP c, const NList& l, const PairConst* pc, DirFlags fl, double* ef, double* efg, double* f,
                       Partials& part, DevScalars* d, int g) {

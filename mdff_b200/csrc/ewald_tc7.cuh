@@ -20,11 +20,14 @@
 // seven digits, balanced ones in [-128, 127], and for the structure factor's A
 // operand, which is made anew for every evaluation, the plain bytes of V (the
 // first signed, the others unsigned: nothing to carry); the 28 digit products of weight >= 2^48 (of 2^96) add
-// up exactly in seven S32 levels of tensor memory and are joined in FP64.  What
-// is lost per term: the rounding of V (2^-56 of the scale) and the dropped
-// products (rms 2^-55.3 or less), below one FP64 rounding; there is no error of a phase
-// recurrence along nz and none of the summation over atoms.  Scales are per
-// row (structure factor) and per (column, moment) (field).
+// up exactly in seven S32 levels of tensor memory and are joined in FP64.  Scales
+// are per row (structure factor: a bound over the CTA's atoms and over nz) and per
+// (column, moment) (field).  What is lost per term: the rounding of V, 2^-56 of the
+// scale, and the dropped products, rms 2^-55.3 of it or less.  That is below one FP64
+// rounding of the largest term and more of a small one: in a pass of dipoles alone
+// the scale is at least kz times the largest m3, so a term at |nz| = 1 loses up to about
+// kz 2^-56 of its own size (2^-51 at kz = 31), as much as a phase recurrence along nz
+// does, which this form does not have.  The summation over atoms loses nothing.
 //
 // The MMAs of one K step: A digit i times B digits 0..6-i, which lie side by
 // side along N, into levels i..6, N columns apart in tensor memory, as one MMA
